@@ -141,7 +141,8 @@ int fem_ctx_info(void* ctx, int64_t* out6);
 /* counters since creation: out[0] kernel launches that did work (library
  * kernels only), out[1] CG iterations, out[2] residual evaluations,
  * out[3] CG graph launches; matvec variant selection: out[4] variant in use
- * (0 fused node-block, 1 two-phase, 2 element-block), out[5] / out[6] timed
+ * (0 fused node-block, 1 two-phase, 2 element-block, 5 assembled in the
+ * persistent PCG kernel), out[5] / out[6] timed
  * ns per launch of the fused / two-phase variant (0 if not timed), out[7] 1
  * if the choice was made by timing; out[8] PCG solves run as one whole-solve
  * graph launch (conditional WHILE node), out[9] 1 if such graphs are
@@ -155,7 +156,9 @@ int fem_ctx_stats(void* ctx, int64_t* out18);
 /* Option keys of fem_set_option (no reference counterpart: the reference has
  * one matvec formulation, backend/fea/fem/material/nonlinear/base.py:110-145). */
 enum {
-  /* -1 (default): time the tangent-matvec variants on the first PCG solve
+  /* not set (default): plain TET4 solves run as one persistent kernel on the
+   * assembled tangent (stats variant 5) where the mesh fits it, everything
+   * else with variant 4; -1: time the element variants on the first PCG solve
    * and keep the fastest; 0: fused node-block kernel; 1: element pass writing
    * slot vectors in node order plus a node gather; 2 (TET4): element-block
    * kernel that sums each block's slot vectors in shared memory, nodes
@@ -189,7 +192,7 @@ enum {
    * chain of kernels.  Jacobi and two-level; batched solves use the chain. */
   FEM_OPT_FUSED_STEP = 6,
   /* 1 (default): a PCG solve runs as one graph launch (a conditional WHILE
-   * node); 0: as launches of fixed 12- or 32-iteration graphs with a host
+   * node) where it does not run as the persistent kernel; 0: as launches of fixed 12- or 32-iteration graphs with a host
    * check between them (kernel profilers cannot attribute kernels inside
    * conditional graphs) */
   FEM_OPT_WHOLE_SOLVE_GRAPH = 7,

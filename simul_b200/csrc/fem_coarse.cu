@@ -220,22 +220,48 @@ __device__ __forceinline__ void tile_ij(int t, int& I, int& J) {
   J = t - i * (i + 1) / 2;
 }
 
-// Packed BF16 copy: the lower block triangle of 64 x 64 tiles.
-__global__ void coarse_pack16_kernel(const __grid_constant__ CoarseDev c) {
+// Packed copy (BF16 or FP32): the lower block triangle of 64 x 64 tiles.  In
+// BF16 the 16-byte chunks of a tile row are swizzled (chunk c of row r at
+// c ^ (r % 8)), so that ldmatrix reads eight rows' chunks without bank
+// conflicts (fem_pcg.cu).
+template <bool F32>
+__global__ void coarse_pack_kernel(const __grid_constant__ CoarseDev c) {
   const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int nt = c.nb16 * (c.nb16 + 1) / 2;
   if (q >= (int64_t)nt * kTileElems) return;
   const int t = (int)(q / kTileElems), e = (int)(q % kTileElems);
   int I, J;
   tile_ij(t, I, J);
-  const int row = I * kTile + e / kTile, col = J * kTile + e % kTile;
+  const int r = e / kTile, ec = F32 ? e % kTile : (e % kTile) ^ (8 * (r & 7));
+  const int row = I * kTile + r, col = J * kTile + ec;
   const int n = c.n_dof;
   float v = 0.f;
   if (row < n && col < n) {
     const int lo = max(row, col), hi = min(row, col);
     v = c.Ac32 ? c.Ac32[(size_t)hi * n + lo] : (float)c.Ac[(size_t)hi * n + lo];
   }
-  c.Ainv16[q] = __float2bfloat16_rn(v);
+  if (F32)
+    c.Ainv32t[q] = v;
+  else
+    c.Ainv16[q] = __float2bfloat16_rn(v);
+}
+
+// Full rows of full_ld words (zero beyond n_dof) for the persistent solve.
+template <bool F32>
+__global__ void coarse_full_kernel(const __grid_constant__ CoarseDev c) {
+  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int n = c.n_dof, ld = c.full_ld;
+  if (q >= (int64_t)n * ld) return;
+  const int row = (int)(q / ld), col = (int)(q % ld);
+  float v = 0.f;
+  if (col < n) {
+    const int lo = max(row, col), hi = min(row, col);
+    v = c.Ac32 ? c.Ac32[(size_t)hi * n + lo] : (float)c.Ac[(size_t)hi * n + lo];
+  }
+  if (F32)
+    c.Afull32[q] = v;
+  else
+    c.Afull16[q] = __float2bfloat16_rn(v);
 }
 
 // ───────────────────────── per-iteration application ─────────────────────────
@@ -436,7 +462,7 @@ __global__ void __launch_bounds__(kTileWarps * 32, 3) coarse_tile_mv_kernel(
       const int row = 4 * k + q;
       float a[8];
       // streamed once per product (evict-first), so the matvec's working set keeps the L2
-      bf16x8_to_f32(__ldcs(tile + row * (kTile / 8) + cg8), a);
+      bf16x8_to_f32(__ldcs(tile + row * (kTile / 8) + (cg8 ^ (row & 7))), a);
       float s = 0.f;
 #pragma unroll
       for (int e = 0; e < 8; ++e) s += a[e] * xj[e];
@@ -858,11 +884,14 @@ void launch_coarse_assemble(const CoarseArgs& a, int model, cudaStream_t s) {
 }
 
 void launch_coarse_symmetrize(const CoarseDev& c, cudaStream_t s) {
+  const int64_t ne = (int64_t)c.nb16 * (c.nb16 + 1) / 2 * kTileElems, nf = (int64_t)c.n_dof * c.full_ld;
+  if (c.Afull16) coarse_full_kernel<false><<<nblk(nf, 256), 256, 0, s>>>(c);
+  if (c.Afull32) coarse_full_kernel<true><<<nblk(nf, 256), 256, 0, s>>>(c);
   if (c.Ainv16) {
-    const int64_t ne = (int64_t)c.nb16 * (c.nb16 + 1) / 2 * kTileElems;
-    coarse_pack16_kernel<<<nblk(ne, 256), 256, 0, s>>>(c);
+    coarse_pack_kernel<false><<<nblk(ne, 256), 256, 0, s>>>(c);
     return;
   }
+  if (c.Ainv32t) coarse_pack_kernel<true><<<nblk(ne, 256), 256, 0, s>>>(c);
   const int64_t nn = (int64_t)c.n_dof * c.n_dof;
   coarse_sym_kernel<<<nblk(nn, 256), 256, 0, s>>>(c);
 }

@@ -14,12 +14,15 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <numeric>
 #include <string>
 #include <vector>
 
 #include "../../include/femb200.h"
+#include "fem_asm.h"
 #include "fem_internal.h"
+#include "fem_pcg.h"
 
 using namespace femb200;
 
@@ -38,6 +41,8 @@ constexpr int kCGBatch = 32;
 constexpr int kCGBatchShort = 12;
 inline int cg_batch(int kind) { return kind == 0 ? kCGBatch : kCGBatchShort; }
 inline int step_chunks(int n_nodes) { return (n_nodes + kStepThreads - 1) / kStepThreads; }
+
+constexpr int kMvRule = -2;
 
 struct FemCtx {
   int device = 0;
@@ -204,9 +209,10 @@ struct FemCtx {
   DenseSched dense_sched;       // streams and events of the dense inverse
   std::vector<int> coarse_row_first;  // Ac's row envelope (lowest coupled DOF per row)
   int* h_info = nullptr;
-  // matvec variant: forced by fem_set_option (>= 0) or chosen by timing all
-  int mv_forced = -1;
-  int mv_variant = MV_FUSED;
+  // matvec variant: forced by fem_set_option (>= 0), chosen by timing all
+  // (-1, on request) or by the rule of choose_matvec_variant (kMvRule)
+  int mv_forced = kMvRule;
+  int mv_variant = MV_PERSIST;
   bool mv_tuned = false;
   int mv_tuned_model = -2;
   double mv_ns[MV_N_VARIANTS] = {0.0, 0.0, 0.0, 0.0, 0.0};
@@ -218,6 +224,25 @@ struct FemCtx {
   // warp-aggregated two-phase matvec tables (TET4; built when selected or timed)
   WaggDev wadev{};
   std::vector<void*> wa_bufs;
+  // assembled tangent: tables built on the first PCG solve that uses it
+  AsmDev asmdev{};
+  std::vector<void*> asm_bufs;
+  bool asm_built = false;
+  bool asm_refused = false;   // the mesh does not fit the format
+  bool asm_valid = false;     // the values belong to the current tangent state
+  // persistent PCG kernel (fem_pcg.cu): tables per matrix and per coarse
+  // lattice; chain_forced: an option of the kernel chain was set, so the
+  // solves run as that chain
+  PcgDev pcgdev{};
+  std::vector<int> asm_cta_row;        // first row of each CTA
+  std::vector<int> asm_prefix;         // steps of the first slices (shared-memory plan)
+  bool pcg_coarse_built = false;
+  bool chain_forced = false;
+  bool pcg_ok = true;         // a refused plan or launch turns it off
+  std::vector<void*> pcg_coarse_bufs;
+  double* pcg_part = nullptr;
+  unsigned int* pcg_bar = nullptr;
+  float* pcg_p2 = nullptr;    // second buffer of the direction
   int eb_size = 0;
   int eb_forced = 0;
   double eb_ns[4] = {0.0, 0.0, 0.0, 0.0};
@@ -345,6 +370,10 @@ void free_ctx(FemCtx* c) {
   for (void* p : c->eb_bufs)
     if (p) cudaFree(p);
   for (void* p : c->wa_bufs)
+    if (p) cudaFree(p);
+  for (void* p : c->asm_bufs)
+    if (p) cudaFree(p);
+  for (void* p : c->pcg_coarse_bufs)
     if (p) cudaFree(p);
   if (c->h_err) cudaFreeHost(c->h_err);
   if (c->dense_work) cudaFree(c->dense_work);
@@ -879,11 +908,105 @@ MvArgs make_mv(const FemCtx* c) {
   MvArgs mv;
   std::memset(&mv, 0, sizeof(mv));
   mv.m = c->mesh();
-  mv.variant = c->mv_variant;
+  // the assembled product runs in the persistent PCG kernel only: a single
+  // product with a new tangent is cheaper by elements than with an assembly
+  mv.variant = c->mv_variant == MV_ASSEMBLED ? MV_PERSIST : c->mv_variant;
   mv.stage = c->stage;
   mv.eb = c->ebdev;
   mv.wa = c->wadev;
   return mv;
+}
+
+AsmArgs asm_args(const FemCtx* c) {
+  AsmArgs a;
+  a.m = c->mesh();
+  a.s = c->asmdev;
+  a.matF = c->matF;
+  a.payload = c->payload;
+  return a;
+}
+
+template <typename T>
+int asm_upload(FemCtx* c, T** dst, const T* src, size_t n) {
+  int st;
+  if ((st = dalloc(c, dst, n))) return st;
+  c->asm_bufs.push_back(*dst);
+  if (src && n) CK(cudaMemcpyAsync(*dst, src, n * sizeof(T), cudaMemcpyHostToDevice, c->stream));
+  return FEM_OK;
+}
+
+// Tables of the assembled tangent; asm_refused where the mesh does not fit.
+int ensure_asm_tables(FemCtx* c) {
+  if (c->asm_built || c->asm_refused) return FEM_OK;
+  const size_t cw = (size_t)c->npe / 4;
+  std::vector<int4> conn(cw * c->Ne);
+  CK(cudaMemcpyAsync(conn.data(), c->conn, conn.size() * sizeof(int4), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  AsmHost h;
+  int sms = 0;
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+  if (!build_asm_host(conn.data(), c->Nn, c->Ne, c->npe, sms, &h)) {
+    c->asm_refused = true;
+    return FEM_OK;
+  }
+  int st;
+  AsmDev& S = c->asmdev;
+  uint32_t* words = nullptr;
+  auto up = [&](auto** dst, const auto& v) { return asm_upload(c, dst, v.data(), v.size()); };
+  int *cta_row = nullptr, *cta_slice = nullptr, *slice_step = nullptr, *slice_rows = nullptr, *halo_ptr = nullptr,
+      *halo = nullptr;
+  uint2* edges = nullptr;
+  uint32_t *eptr = nullptr, *list = nullptr;
+  if ((st = up(&cta_row, h.cta_row)) || (st = up(&cta_slice, h.cta_slice)) || (st = up(&slice_step, h.slice_step)) ||
+      (st = up(&slice_rows, h.slice_rows)) || (st = up(&halo_ptr, h.halo_ptr)) || (st = up(&halo, h.halo)) ||
+      (st = up(&edges, h.edges)) || (st = up(&eptr, h.eptr)) || (st = up(&list, h.list)))
+    return st;
+  if ((st = asm_upload(c, &words, (const uint32_t*)nullptr, (size_t)h.slice_step.back() * kAsmStepWords))) return st;
+  if ((st = asm_upload(c, &c->pcg_part, (const double*)nullptr, 3 * (size_t)h.grid))) return st;
+  if ((st = asm_upload(c, &c->pcg_bar, (const unsigned int*)nullptr, (size_t)1))) return st;
+  if ((st = asm_upload(c, &c->pcg_p2, (const float*)nullptr, 4 * (size_t)c->Nn))) return st;
+  S.grid = h.grid;
+  S.n_slices = (int)h.slice_step.size() - 1;
+  S.n_edges = (int)h.edges.size();
+  S.max_slices = h.max_slices;
+  S.max_halo = h.max_halo;
+  S.max_cols = h.max_cols;
+  S.max_pieces = h.max_pieces;
+  S.cta_row = cta_row;
+  S.cta_slice = cta_slice;
+  S.slice_step = slice_step;
+  S.slice_rows = slice_rows;
+  S.words = words;
+  S.edges = edges;
+  S.eptr = eptr;
+  S.list = list;
+  S.halo_ptr = halo_ptr;
+  S.halo = halo;
+  c->asm_cta_row = h.cta_row;
+  c->asm_prefix = h.prefix;
+  int2* entry = nullptr;
+  CK(cudaMalloc(reinterpret_cast<void**>(&entry), std::max<size_t>(h.entry.size(), 1) * sizeof(int2)));
+  cudaError_t e = cudaMemcpyAsync(entry, h.entry.data(), h.entry.size() * sizeof(int2), cudaMemcpyHostToDevice, c->stream);
+  if (e == cudaSuccess) {
+    launch_asm_fill(S, entry, c->stream);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);  // the host tables go out of scope
+  cudaFree(entry);
+  CK(e);
+  c->asm_built = true;
+  c->asm_valid = false;
+  return FEM_OK;
+}
+
+// The assembled blocks at the current tangent state.
+int ensure_assembled(FemCtx* c) {
+  if (c->asm_valid) return FEM_OK;
+  launch_asm(asm_args(c), c->model_kind, c->stream);
+  ++c->n_launches;
+  CKL();
+  c->asm_valid = true;
+  return FEM_OK;
 }
 
 int eval_residual(FemCtx* c, double* fneg_out_int, double* rnorm2) {
@@ -909,6 +1032,8 @@ int eval_residual(FemCtx* c, double* fneg_out_int, double* rnorm2) {
   CK(cudaMemcpyAsync(c->h_scalars, c->scalars, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   c->tangent_valid = true;
+  // linear models have no tangent payload: their blocks stay those of the materials
+  if (c->model_kind != M_LE && c->model_kind != M_TI) c->asm_valid = false;
   if (rnorm2) *rnorm2 = c->h_scalars[0];
   return FEM_OK;
 }
@@ -916,7 +1041,10 @@ int eval_residual(FemCtx* c, double* fneg_out_int, double* rnorm2) {
 // Jacobi scaling for the PCG solve: 1 / diag(K_T), or with `block` the
 // nodal 3 x 3 block inverse (diagonal in dinv, off-diagonals in boff).
 int compute_dinv(FemCtx* c, int precond, bool block = false) {
-  if (precond == FEM_PRECOND_JACOBI) {
+  if (precond == FEM_PRECOND_JACOBI && c->asm_valid && c->mv_variant == MV_ASSEMBLED) {
+    ++c->n_launches; launch_asm_diag(asm_args(c), c->dinv, block ? c->boff : nullptr, c->stream);
+    CKL();
+  } else if (precond == FEM_PRECOND_JACOBI) {
     DiagArgs a;
     a.m = c->mesh();
     a.matF = c->matF;
@@ -957,7 +1085,8 @@ struct ChainPdl {
 // Two-level PCG with the two-phase matvec: the matvec acts on z and its node
 // gather forms p = z + beta p, q = K z + beta q (no direction-update kernel).
 bool recurrence(const FemCtx* c, int kind) {
-  return kind == GRAPH_TWO_LEVEL && (c->mv_variant == MV_TWO_PHASE || c->mv_variant == MV_WARP_AGG || c->mv_variant == MV_PERSIST) &&
+  return kind == GRAPH_TWO_LEVEL && (c->mv_variant == MV_TWO_PHASE || c->mv_variant == MV_WARP_AGG ||
+                                     c->mv_variant == MV_PERSIST) &&
          c->direction_recurrence;
 }
 
@@ -1052,10 +1181,14 @@ CGState endless_cg() {
 }
 
 // Picks the matvec variant for the current material tables: the forced one
-// when fem_set_option set it, else the faster of the two on this mesh, timed
-// with CUDA events as they run inside CG (3 warm-up + 10 timed launches each,
-// p = 1 on free DOFs).  The CG state is reset by cg_init afterwards.
-int choose_matvec_variant(FemCtx* c) {
+// when fem_set_option set it; unless the option asks for timing, the
+// assembled product in the persistent PCG kernel for a plain solve (`plain`:
+// not the learned preconditioner, no option of the kernel chain set) of a
+// TET4 mesh that fits it, and the persistent element pass else; with timing,
+// the fastest of the element variants on this mesh, timed with CUDA events as
+// they run inside CG (3 warm-up + 10 timed launches each, p = 1 on free
+// DOFs).  The CG state is reset by cg_init afterwards.
+int choose_matvec_variant(FemCtx* c, bool plain) {
   if (c->npe == 8) {
     // HEX8 has the two-phase pass only
     c->mv_variant = MV_TWO_PHASE;
@@ -1067,6 +1200,14 @@ int choose_matvec_variant(FemCtx* c) {
     if (c->mv_variant == MV_ELEM_BLOCK && c->eb_size == 0)
       return build_eb_tables(c, c->eb_forced > 0 ? c->eb_forced : 512);
     if (c->mv_variant == MV_WARP_AGG) return build_wagg_tables(c);
+    return FEM_OK;
+  }
+  if (c->mv_forced == kMvRule) {
+    // (a batch of several workers overlaps its contexts' chains: one
+    // persistent kernel at a time took 196 ms where eight chains take 150)
+    plain = plain && !c->chain_forced && c->pcg_ok && !c->in_batch;
+    if (plain && (st = ensure_asm_tables(c))) return st;
+    c->mv_variant = plain && c->asm_built ? MV_ASSEMBLED : MV_PERSIST;
     return FEM_OK;
   }
   if (c->mv_tuned && c->mv_tuned_model == c->model_kind) return FEM_OK;
@@ -1188,6 +1329,10 @@ int drop_coarse(FemCtx* c) {
   for (void* p : c->coarse_bufs)
     if (p) cudaFree(p);
   c->coarse_bufs.clear();
+  for (void* p : c->pcg_coarse_bufs)
+    if (p) cudaFree(p);
+  c->pcg_coarse_bufs.clear();
+  c->pcg_coarse_built = false;
   c->cdev = CoarseDev{};
   c->coarse_have_inverse = false;
   c->tl_part = nullptr;
@@ -1212,7 +1357,7 @@ void invalidate_coarse(FemCtx* c) { c->coarse_valid = false; }
 
 int ensure_cg_graph(FemCtx* c, int kind) {
   int st;
-  if ((st = choose_matvec_variant(c))) return st;
+  if ((st = choose_matvec_variant(c, false))) return st;
   const bool fused = use_fused(c, kind);
   const bool pdl = use_pdl(c, kind);
   const int flags = (kind == GRAPH_LEARNED ? (c->learned_coarse ? 1 : 0) : 0) | (fused ? 2 : 0) | (pdl ? 4 : 0) |
@@ -1490,6 +1635,9 @@ int build_coarse(FemCtx* c) {
   cd.nb16 = (cd.n_dof + 63) / 64;
   const size_t nb = (size_t)cd.nb16;
   cd.Ainv = nullptr;
+  cd.Ainv32t = nullptr;
+  cd.Afull16 = nullptr;
+  cd.Afull32 = nullptr;
   cd.Ainv16 = nullptr;
   cd.yslots = nullptr;
   if (c->coarse_bf16) {
@@ -1498,6 +1646,13 @@ int build_coarse(FemCtx* c) {
   } else {
     if ((st = coarse_alloc(c, &cd.Ainv, nd * nd))) return st;
   }
+  // the persistent solve reads full rows up to 16 MB: they come from L2 in
+  // about the time that adding up the packed tiles' two products takes
+  const size_t ld = (nd + 7) / 8 * 8, full = nd * ld * (c->coarse_bf16 ? 2 : 4);
+  cd.full_ld = full <= (16u << 20) ? (int)ld : 0;
+  if (cd.full_ld && c->coarse_bf16 && (st = coarse_alloc(c, &cd.Afull16, nd * ld))) return st;
+  if (cd.full_ld && !c->coarse_bf16 && (st = coarse_alloc(c, &cd.Afull32, nd * ld))) return st;
+  if (!cd.full_ld && !c->coarse_bf16 && (st = coarse_alloc(c, &cd.Ainv32t, nb * (nb + 1) / 2 * 4096))) return st;
   cd.r_slices = coarse_restrict_slices(n_cells);
   if ((st = coarse_alloc(c, &cd.cell_r, (size_t)n_cells * cd.r_slices * 24))) return st;
   if ((st = coarse_alloc(c, &cd.yc, nb * 64))) return st;
@@ -1797,33 +1952,119 @@ void mpnn_sample(FemCtx* c, const float* R, const float* E, int k, bool coarse, 
   }
 }
 
-// Solves K_T x = b (b: FP64 internal order, fixed DOFs zero) into c->x.
-int run_pcg(FemCtx* c, const double* b_int, int precond, double rtol, int maxit, int* iters,
-            double* rel) {
-  if (!c->tangent_valid) return set_err(c, FEM_ERR_STATE, "no tangent state: evaluate forces first");
+// ───────────────────────── persistent PCG ─────────────────────────
+
+template <typename T>
+int pcg_upload(FemCtx* c, std::vector<void*>& bufs, const T** dst, const std::vector<T>& v) {
+  T* d = nullptr;
   int st;
-  if (c->npe == 8 && precond == FEM_PRECOND_LEARNED) {
-    // the learned network is trained on TET4 graphs: a HEX8 context runs
-    // these solves as Jacobi-PCG
-    ++c->n_coarse_fallbacks;
-    precond = FEM_PRECOND_JACOBI;
+  if ((st = dalloc(c, &d, v.size()))) return st;
+  bufs.push_back(d);
+  if (!v.empty()) CK(cudaMemcpyAsync(d, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, c->stream));
+  *dst = d;
+  return FEM_OK;
+}
+
+int ensure_pcg_tables(FemCtx* c, bool two_level) {
+  int st;
+  PcgDev& t = c->pcgdev;
+  if (!two_level || c->pcg_coarse_built) return FEM_OK;
+  std::vector<int> node_cell(c->Nn), corner(8 * (size_t)c->cdev.n_cells);
+  CK(cudaMemcpyAsync(node_cell.data(), c->cdev.node_cell, node_cell.size() * sizeof(int), cudaMemcpyDeviceToHost,
+                     c->stream));
+  CK(cudaMemcpyAsync(corner.data(), c->cdev.cell_corner, corner.size() * sizeof(int), cudaMemcpyDeviceToHost,
+                     c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  PcgCoarseHost h;
+  if (!pcg_coarse_tables(c->asm_cta_row, node_cell, corner, c->cdev.n_cn,
+                         c->cdev.full_ld ? 0 : (c->cdev.Ainv16 ? 2 : 4), &h)) {
+    c->pcg_ok = false;
+    return FEM_OK;
   }
-  const bool tl = precond == FEM_PRECOND_TWO_LEVEL;
-  const bool learned = precond == FEM_PRECOND_LEARNED;
-  const int kind = learned ? GRAPH_LEARNED : (tl ? GRAPH_TWO_LEVEL : GRAPH_JACOBI);
-  if (learned && !c->mpnn_has_weights)
-    return set_err(c, FEM_ERR_STATE, "learned preconditioner has no weights (fem_mpnn_set_weights)");
-  if ((st = compute_dinv(c, (tl || learned) ? FEM_PRECOND_JACOBI : precond, tl && c->block_jacobi))) return st;
-  if (tl && (st = ensure_coarse(c))) {
-    // no positive definite coarse operator on this lattice yet (e.g. cells
-    // finer than the elements of an anisotropic mesh): this solve runs as
-    // Jacobi-PCG instead of failing
-    if (st != FEM_ERR_NAN) return st;
-    ++c->n_coarse_fallbacks;
-    return run_pcg(c, b_int, FEM_PRECOND_JACOBI, rtol, maxit, iters, rel);
+  auto& bufs = c->pcg_coarse_bufs;
+  const int* seg_rows = nullptr;
+  float4* lat = nullptr;
+  if ((st = pcg_upload(c, bufs, &t.tab_ptr, h.tab_ptr))) return st;
+  if ((st = pcg_upload(c, bufs, &t.tab, h.tab))) return st;
+  if ((st = pcg_upload(c, bufs, &seg_rows, h.seg_rows))) return st;
+  if ((st = pcg_upload(c, bufs, &t.row_corners, h.row_corners))) return st;
+  if ((st = dalloc(c, &lat, (size_t)c->Nn))) return st;
+  bufs.push_back(lat);
+  launch_pcg_seg_lat(seg_rows, c->cdev.node_lat, c->Nn, lat, c->stream);
+  CKL();
+  t.seg_lat = lat;
+  if ((st = dalloc(c, &t.seg_r, 8 * (size_t)h.n_seg))) return st;
+  bufs.push_back(t.seg_r);
+  if ((st = dalloc(c, &t.ypart, 64 * (size_t)h.n_parts))) return st;
+  bufs.push_back(t.ypart);
+  t.max_tab = h.max_tab;
+  t.max_lblk = h.max_lblk;
+  t.max_loc = h.max_loc;
+  t.max_tiles = h.max_tiles;
+  CK(cudaStreamSynchronize(c->stream));  // the host tables go out of scope
+  c->pcg_coarse_built = true;
+  return FEM_OK;
+}
+
+// One launch at a time on a device: the kernel fills the GPU and its CTAs
+// wait for one another, so a second one could only hold SMs the first needs.
+std::mutex& pcg_mutex(int device) {
+  static std::mutex mu[64];
+  return mu[device & 63];
+}
+
+// The whole solve in one launch; the end state in h_cg.  *ran = false where
+// the plan or the launch was refused (the caller runs the chain).
+int run_persistent(FemCtx* c, const double* b_int, bool two_level, double rtol, int maxit, bool* ran) {
+  int st;
+  *ran = false;
+  if ((st = ensure_pcg_tables(c, two_level))) return st;
+  if (!c->pcg_ok) return FEM_OK;
+  PcgArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.m = c->mesh();
+  a.as = c->asmdev;
+  a.c = c->cdev;
+  a.t = c->pcgdev;
+  a.b = b_int;
+  a.r = c->r;
+  a.x = c->x;
+  a.p = c->p;
+  a.q = c->y;
+  a.z = c->tmpf;
+  a.dinv = c->dinv;
+  a.p2 = c->pcg_p2;
+  a.boff = two_level && c->block_jacobi ? c->boff : nullptr;
+  a.cg = c->cg;
+  a.part = c->pcg_part;
+  a.bar = c->pcg_bar;
+  a.rtol = rtol;
+  a.max_iter = maxit;
+  size_t smem = 0;
+  if (!pcg_plan(a, two_level, c->asm_prefix, &smem)) {
+    c->pcg_ok = false;
+    return FEM_OK;
   }
-  if (learned && c->learned_coarse && (st = ensure_coarse(c))) return st;
-  if (learned && (st = ensure_mpnn(c))) return st;
+  CK(cudaMemsetAsync(c->pcg_bar, 0, sizeof(unsigned int), c->stream));
+  std::lock_guard<std::mutex> lock(pcg_mutex(c->device));
+  const cudaError_t e = launch_pcg(a, two_level, smem, c->stream);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    c->pcg_ok = false;
+    return FEM_OK;
+  }
+  ++c->n_launches;
+  CK(cudaMemcpyAsync(c->h_cg, c->cg, sizeof(CGState), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  *ran = true;
+  return FEM_OK;
+}
+
+// The solve as a chain of kernels per iteration, replayed from captured
+// graphs; the end state in h_cg.
+int run_chain(FemCtx* c, const double* b_int, int kind, double rtol, int maxit) {
+  int st;
+  const bool tl = kind == GRAPH_TWO_LEVEL, learned = kind == GRAPH_LEARNED;
   if ((st = ensure_cg_graph(c, kind))) return st;
   const bool fused = (c->cg_graph_flags[kind] & 2) != 0;
   if (fused) CK(cudaMemsetAsync(c->step_bar, 0, 4 * sizeof(unsigned int), c->stream));
@@ -1870,6 +2111,41 @@ int run_pcg(FemCtx* c, const double* b_int, int precond, double rtol, int maxit,
     CK(cudaStreamSynchronize(c->stream));
     ++batches;
   }
+  return FEM_OK;
+}
+
+// Solves K_T x = b (b: FP64 internal order, fixed DOFs zero) into c->x.
+int run_pcg(FemCtx* c, const double* b_int, int precond, double rtol, int maxit, int* iters,
+            double* rel) {
+  if (!c->tangent_valid) return set_err(c, FEM_ERR_STATE, "no tangent state: evaluate forces first");
+  int st;
+  if (c->npe == 8 && precond == FEM_PRECOND_LEARNED) {
+    // the learned network is trained on TET4 graphs: a HEX8 context runs
+    // these solves as Jacobi-PCG
+    ++c->n_coarse_fallbacks;
+    precond = FEM_PRECOND_JACOBI;
+  }
+  const bool tl = precond == FEM_PRECOND_TWO_LEVEL;
+  const bool learned = precond == FEM_PRECOND_LEARNED;
+  const int kind = learned ? GRAPH_LEARNED : (tl ? GRAPH_TWO_LEVEL : GRAPH_JACOBI);
+  if (learned && !c->mpnn_has_weights)
+    return set_err(c, FEM_ERR_STATE, "learned preconditioner has no weights (fem_mpnn_set_weights)");
+  if ((st = choose_matvec_variant(c, !learned))) return st;
+  if (c->mv_variant == MV_ASSEMBLED && (st = ensure_assembled(c))) return st;
+  if ((st = compute_dinv(c, (tl || learned) ? FEM_PRECOND_JACOBI : precond, tl && c->block_jacobi))) return st;
+  if (tl && (st = ensure_coarse(c))) {
+    // no positive definite coarse operator on this lattice yet (e.g. cells
+    // finer than the elements of an anisotropic mesh): this solve runs as
+    // Jacobi-PCG instead of failing
+    if (st != FEM_ERR_NAN) return st;
+    ++c->n_coarse_fallbacks;
+    return run_pcg(c, b_int, FEM_PRECOND_JACOBI, rtol, maxit, iters, rel);
+  }
+  if (learned && c->learned_coarse && (st = ensure_coarse(c))) return st;
+  if (learned && (st = ensure_mpnn(c))) return st;
+  bool ran = false;
+  if (c->mv_variant == MV_ASSEMBLED && (st = run_persistent(c, b_int, tl, rtol, maxit, &ran))) return st;
+  if (!ran && (st = run_chain(c, b_int, kind, rtol, maxit))) return st;
   const CGState& h = *c->h_cg;
   c->n_cg_iters += h.iter;
   if ((tl || (learned && c->learned_coarse)) && c->coarse_reuse < 0 && h.done == 1 && h.rr0 > 0 && h.rr > 0) {
@@ -1889,8 +2165,8 @@ int run_pcg(FemCtx* c, const double* b_int, int precond, double rtol, int maxit,
     // the network's 6 kernels run until it is switched off (after 3 rejected steps)
     const int64_t net_steps = std::max<int64_t>(0, (int64_t)h.iter - h.n_alt + std::min(h.n_alt, 3));
     c->n_launches += (5LL + (c->learned_coarse ? 2 + coarse_product_kernels(c->cdev) : 0)) * h.iter + 6LL * net_steps;
-  } else {
-    c->n_launches += kernels_per_iter(c, kind, fused) * h.iter;
+  } else if (!ran) {
+    c->n_launches += kernels_per_iter(c, kind, (c->cg_graph_flags[kind] & 2) != 0) * h.iter;
   }
   if (learned) {
     c->n_alt_steps += h.n_alt;
@@ -2161,6 +2437,7 @@ int fem_set_option(void* ctx, int32_t key, int64_t value) {
         }
         c->use_loop_graph = value != 0;
       }
+      if (value == 0) c->chain_forced = true;
       return FEM_OK;
     case FEM_OPT_COARSE_MAX_NODES:
       if (value < 8 || value > kMaxCoarseNodesLimit)
@@ -2182,14 +2459,17 @@ int fem_set_option(void* ctx, int32_t key, int64_t value) {
     case FEM_OPT_DIRECTION_RECURRENCE:
       if (value != 0 && value != 1) return set_err(c, FEM_ERR_INVALID, "direction recurrence flag must be 0 or 1");
       c->direction_recurrence = value != 0;
+      c->chain_forced = true;
       return FEM_OK;
     case FEM_OPT_PDL:
       if (value != 0 && value != 1) return set_err(c, FEM_ERR_INVALID, "programmatic launch flag must be 0 or 1");
       c->pdl = value != 0;
+      c->chain_forced = true;
       return FEM_OK;
     case FEM_OPT_FUSED_STEP:
       if (value != 0 && value != 1) return set_err(c, FEM_ERR_INVALID, "fused step flag must be 0 or 1");
       c->fused_step = value != 0;
+      c->chain_forced = true;
       return FEM_OK;
     case FEM_OPT_COARSE_REUSE:
       if (value < -1 || value > (1 << 20))
@@ -2489,6 +2769,7 @@ int fem_set_materials(void* ctx, const FemMaterial* table, int32_t n, const uint
   c->has_j2 = has_j2;
   c->materials_set = true;
   c->tangent_valid = false;
+  c->asm_valid = false;
   invalidate_coarse(c);
   return FEM_OK;
 }
@@ -2509,6 +2790,7 @@ int fem_set_bc(void* ctx, const uint8_t* fixed_mask, const double* fixed_values,
     CK(cudaStreamSynchronize(c->stream));
     if (now != c->fixed_host) {
       c->fixed_host.swap(now);
+      c->asm_valid = false;  // rows of fixed DOFs are stored as zeros
       invalidate_coarse(c);
     }
   }
@@ -2574,14 +2856,18 @@ int fem_batch_solve(void** ctxs, int32_t n, const FemSolveParams* prm, int32_t l
     if ((st = check_ctx(c))) return st;
     if (!c->materials_set) return set_err(c, FEM_ERR_STATE, "materials not set");
     if (!c->tangent_valid && (st = eval_residual(c, nullptr, nullptr))) return st;
+    c->in_batch = workers > 1;
     const bool tl = p.precond == FEM_PRECOND_TWO_LEVEL;
     const bool learned = p.precond == FEM_PRECOND_LEARNED;
     if (learned && !c->mpnn_has_weights) return set_err(c, FEM_ERR_STATE, "learned preconditioner has no weights");
+    if ((st = choose_matvec_variant(c, !learned))) return st;
+    if (c->mv_variant == MV_ASSEMBLED && (st = ensure_assembled(c))) return st;
     if ((st = compute_dinv(c, (tl || learned) ? FEM_PRECOND_JACOBI : p.precond, tl && c->block_jacobi))) return st;
     if ((tl || (learned && c->learned_coarse)) && (st = ensure_coarse(c))) return st;
     if (learned && (st = ensure_mpnn(c))) return st;
-    c->in_batch = workers > 1;
-    if ((st = ensure_cg_graph(c, learned ? GRAPH_LEARNED : (tl ? GRAPH_TWO_LEVEL : GRAPH_JACOBI)))) return st;
+    const int kind = learned ? GRAPH_LEARNED : (tl ? GRAPH_TWO_LEVEL : GRAPH_JACOBI);
+    if (c->mv_variant == MV_ASSEMBLED && (st = ensure_pcg_tables(c, tl))) return st;
+    if ((c->mv_variant != MV_ASSEMBLED || !c->pcg_ok) && (st = ensure_cg_graph(c, kind))) return st;
   }
   std::atomic<int> next{0};
   auto work = [&]() {

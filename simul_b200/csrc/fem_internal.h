@@ -171,6 +171,34 @@ struct WaggDev {
   float4* parts;            // [prow[Nn]] partial rows
 };
 
+// Assembled tangent (fem_asm.cu): slices of 32 rows (one per lane of a warp),
+// a slice as many steps as its longest row has entries; a step holds one entry
+// of each row: 32 local columns (uint16), components 0-3 and 4-7 of the 32
+// blocks (float4 each), component 8.
+constexpr int kAsmStepWords = 16 + 128 + 128 + 32;
+constexpr int kAsmStepBytes = 4 * kAsmStepWords;
+constexpr int kPcgPiece = 3;        // matrix steps per bulk copy (3.6 KB, the size of a tile part)
+constexpr int kPcgThreads = 512;
+
+struct AsmDev {
+  int grid;                 // CTAs of the persistent solve
+  int n_slices;
+  int n_edges;
+  int max_slices, max_halo, max_cols;  // largest per CTA
+  int max_pieces;           // most pieces (kPcgPiece steps) that a warp of a CTA has
+  const int* cta_row;       // [grid + 1] rows of each CTA
+  const int* cta_slice;     // [grid + 1] slices of each CTA
+  const int* slice_step;    // [n_slices + 1]
+  const int* slice_rows;    // [n_slices * 32] node of each lane, -1: none
+  uint32_t* words;          // [steps * kAsmStepWords]
+  const uint2* edges;       // slots (step * 32 + lane) of (a, b) and (b, a)
+  const uint32_t* eptr;     // [n_edges + 1]
+  const uint32_t* list;
+  // local column l of a CTA: its row l (of n), or its halo node l - n
+  const int* halo_ptr;      // [grid + 1]
+  const int* halo;
+};
+
 struct MvArgs {
   MeshDev m;
   const DevMat<float>* matF;
@@ -201,7 +229,11 @@ struct MvArgs {
 // (fem_kernels.cu).
 // MV_PERSIST: the two-phase pair as persistent grid-stride kernels (one wave
 // of CTAs, the next element's streaming inputs prefetched).
-enum { MV_FUSED = 0, MV_TWO_PHASE = 1, MV_ELEM_BLOCK = 2, MV_WARP_AGG = 3, MV_PERSIST = 4, MV_N_VARIANTS = 5 };
+// MV_ASSEMBLED: the solves run as the persistent PCG kernel on the assembled
+// blocks (fem_pcg.cu).  Not among the variants a caller forces or has timed:
+// the rule of choose_matvec_variant takes it.
+enum { MV_FUSED = 0, MV_TWO_PHASE = 1, MV_ELEM_BLOCK = 2, MV_WARP_AGG = 3, MV_PERSIST = 4, MV_N_VARIANTS = 5,
+       MV_ASSEMBLED = 5 };
 
 // smallest element block of the element-block matvec (one element per
 // thread; blocks of 256, 512, 768 or 1024 elements)
@@ -246,9 +278,17 @@ struct CoarseDev {
   const float* Ac32;        // non-null: the inverse's lower triangle is here in FP32 instead (FP32 inversion)
   float* Ainv;              // [n_dof * n_dof] FP32 inverse (symmetric), or null
   // BF16 inverse, or null: the lower block triangle of 64 x 64 tiles, tile
-  // (I, J), I >= J, at index I (I + 1) / 2 + J, row-major inside the tile,
+  // (I, J), I >= J, at index I (I + 1) / 2 + J, row-major inside the tile (the
+  // 16-byte chunks of a row swizzled),
   // zero beyond n_dof (a diagonal tile holds both of its triangles)
   __nv_bfloat16* Ainv16;
+  // for the persistent solve (fem_pcg.cu): the inverse as full rows of
+  // full_ld words where that is small, BF16 or FP32; else (full_ld = 0) the
+  // packed tiles, for the FP32 inverse these
+  int full_ld;
+  __nv_bfloat16* Afull16;
+  float* Afull32;
+  float* Ainv32t;
   int nb16;                 // tiles per side: ceil(n_dof / 64)
   float* yslots;            // BF16 path: [nb16][nb16][64] slot (R, K) = Ainv_RK r_c,K
   float* cell_r;            // [n_cells][r_slices][24] restricted residual shares per cell

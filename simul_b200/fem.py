@@ -250,7 +250,10 @@ class FEMesh:
 
     def set_matvec_variant(self, variant, block_size=None):
         """Forces the tangent-matvec variant ("fused", "two_phase",
-        "element_block", "warp_agg", "persistent") or restores the timed choice (None); ``block_size``
+        "element_block", "warp_agg", "persistent") or times them on the next
+        solve and keeps the fastest (None).  Where it is never called, plain
+        TET4 solves run as one persistent kernel on the assembled tangent and
+        all others with "persistent".  ``block_size``
         fixes the element-block variant's elements per block (256, 512, 768
         or 1024; 0: timed; None: unchanged)."""
         code = {None: -1, "fused": 0, "two_phase": 1, "element_block": 2, "warp_agg": 3, "persistent": 4}[variant]

@@ -67,7 +67,8 @@ def main(argv=None):
                                  material_ids=ids, coarse_cell=args.coarse_cell) for case in args.cases]
     for inst in insts:
         inst.mesh.set_coarse_options(reuse=args.coarse_reuse)
-        inst.mesh.set_direction_recurrence(bool(args.recurrence))
+        if not args.recurrence:
+            inst.mesh.set_direction_recurrence(False)
         inst.mesh.set_block_smoother(bool(args.block_smoother))
         inst.mesh.set_extrapolation(bool(args.extrapolate))
     t_setup = time.perf_counter() - t0
