@@ -2953,6 +2953,18 @@ int fem_reference_quantities(void* ctx, double* dNdX_out, double* vol_out) {
   return FEM_OK;
 }
 
+static StressArgs stress_args(FemCtx* c) {
+  StressArgs a = {};
+  a.m = c->mesh();
+  a.matD = c->matD;
+  a.u = c->u;
+  a.ep_c = c->ep_c;
+  a.epe_c = c->epe_c;
+  a.perm_elem = c->d_perm_elem;
+  a.stage_d = c->stage_d;
+  return a;
+}
+
 int fem_compute_stress(void* ctx, const double* u, double* F_out, double* sigma_out) {
   FemCtx* c = static_cast<FemCtx*>(ctx);
   int st;
@@ -2962,8 +2974,10 @@ int fem_compute_stress(void* ctx, const double* u, double* F_out, double* sigma_
     ++c->n_launches; launch_gather_d(u, c->u, c->d_perm_node, c->Nn, c->stream);
     CKL();
   }
-  ++c->n_launches; launch_stress(c->mesh(), c->matD, c->model_kind, c->u, c->ep_c, c->epe_c, c->d_perm_elem, F_out,
-                sigma_out, c->stream);
+  StressArgs a = stress_args(c);
+  a.F_out = F_out;
+  a.sig_out = sigma_out;
+  ++c->n_launches; launch_stress(a, c->model_kind, c->stream);
   CKL();
   CK(cudaStreamSynchronize(c->stream));
   return FEM_OK;
@@ -2980,15 +2994,9 @@ int fem_nodal_mises(void* ctx, const double* u, double* mises_out, int32_t avera
     ++c->n_launches; launch_gather_d(u, c->u, c->d_perm_node, c->Nn, c->stream);
     CKL();
   }
-  double* sig = nullptr;
-  CK(cudaMallocAsync(reinterpret_cast<void**>(&sig), sizeof(double) * 9 * c->Nq, c->stream));
-  ++c->n_launches; launch_stress(c->mesh(), c->matD, c->model_kind, c->u, c->ep_c, c->epe_c, c->d_perm_elem,
-                                 nullptr, sig, c->stream);
-  ++c->n_launches; launch_nodal_mises(c->mesh(), c->d_perm_elem, c->d_perm_node, sig, average, mises_out,
-                                      c->stream);
-  const cudaError_t e = cudaGetLastError();
-  cudaFreeAsync(sig, c->stream);
-  if (e != cudaSuccess) return set_err(c, FEM_ERR_CUDA, "nodal Mises kernels failed: %s", cudaGetErrorString(e));
+  c->n_launches += 2; launch_nodal_mises(stress_args(c), c->model_kind, c->d_perm_node, average, mises_out,
+                                         c->stream);
+  CKL();
   CK(cudaStreamSynchronize(c->stream));
   return FEM_OK;
 }

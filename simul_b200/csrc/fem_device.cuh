@@ -521,4 +521,28 @@ __device__ __forceinline__ void diag_store(const float* acc, uint8_t fx, int nod
   reinterpret_cast<float4*>(boff)[node] = ov;
 }
 
+// Von Mises stress of a 3 x 3 stress.
+__device__ __forceinline__ double von_mises9(const double (&s)[9]) {
+  const double s11 = s[0], s22 = s[4], s33 = s[8], s12 = s[1], s23 = s[5], s13 = s[2];
+  return sqrt(0.5 * ((s11 - s22) * (s11 - s22) + (s22 - s33) * (s22 - s33) + (s33 - s11) * (s33 - s11) +
+                     6.0 * (s12 * s12 + s23 * s23 + s13 * s13)));
+}
+
+// One warp stores its rows of nine doubles: lane l (l < rows) holds row l,
+// which belongs at out + 9 * place.  Turned through row[32 * 9] so that one
+// store instruction covers three to four whole rows; called by the whole warp.
+__device__ __forceinline__ void store_rows9(const double (&v)[9], double* row, int lane, int rows, int place,
+                                            double* out) {
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < 9; ++k) row[9 * lane + k] = v[k];
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    const int i = 32 * k + lane, r = i / 9;
+    const int at = __shfl_sync(0xffffffffu, place, r);
+    if (r < rows) out[(size_t)9 * at + (i - 9 * r)] = row[i];
+  }
+}
+
 }  // namespace femb200

@@ -502,12 +502,20 @@ __global__ void __launch_bounds__(256) hex_diag_gather_kernel(const __grid_const
 
 // ───────────────────────── per-point outputs (FP64) ─────────────────────────
 
-template <int MODEL>
-__global__ void hex_stress_kernel(const MeshDev m, const DevMat<double>* matD, const double* u,
-                                  const double* ep_c, const double* epe_c, const int* perm_elem,
-                                  double* F_out, double* sig_out) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= m.n_elems) return;
+// MISES = false: F and / or the Cauchy stress per Gauss point in caller order,
+// rows of 72 bytes turned in shared memory as in the TET4 kernel.  MISES =
+// true: the von Mises stress of the element's Gauss-point mean stress
+// (core/mesh.py:470-474) at its eight slot positions.
+template <int MODEL, bool MISES>
+__global__ void __launch_bounds__(128) hex_stress_kernel(const __grid_constant__ StressArgs a) {
+  __shared__ double s_row[MISES ? 1 : 4][MISES ? 1 : 32 * 9];
+  const MeshDev& m = a.m;
+  const int lane = (int)threadIdx.x % 32;
+  const int e_raw = (int)(blockIdx.x * 128 + threadIdx.x);
+  const int rows = min(32, m.n_elems - (e_raw - lane));  // of this warp
+  if (rows <= 0) return;
+  // the last warp's spare lanes evaluate its last element and store nothing
+  const int e = min(e_raw, m.n_elems - 1);
   const size_t Ne = (size_t)m.n_elems, Nq = kHexGauss * Ne;
   int nid[8];
   hex_nodes(m, e, nid);
@@ -515,14 +523,15 @@ __global__ void hex_stress_kernel(const MeshDev m, const DevMat<double>* matD, c
   for (int k = 0; k < 8; ++k)
     for (int d = 0; d < 3; ++d) {
       xr[k][d] = m.X64[3 * nid[k] + d];
-      uv[k][d] = u[3 * nid[k] + d];
+      uv[k][d] = a.u[3 * nid[k] + d];
     }
   for (int k = 7; k >= 0; --k)
     for (int d = 0; d < 3; ++d) xr[k][d] -= xr[0][d];
-  const DevMat<double>& mat = matD[m.mat_id[e]];
+  const DevMat<double>& mat = a.matD[m.mat_id[e]];
   const double scale = (double)m.scale[e];
   const int model = MODEL >= 0 ? MODEL : mat.model;
-  const int eu = perm_elem[e];
+  const int eu = a.perm_elem[e];
+  double mean[9];
   for (int g = 0; g < kHexGauss; ++g) {
     const size_t q = (size_t)g * Ne + e;
     double dN[8][3], vol;
@@ -547,19 +556,31 @@ __global__ void hex_stress_kernel(const MeshDev m, const DevMat<double>* matD, c
               (P[3 * i] * F[3 * j] + P[3 * i + 1] * F[3 * j + 1] + P[3 * i + 2] * F[3 * j + 2]) / Js;
     } else if (model == M_J2) {
       double ep[6], epn[6], epe_n;
-      for (int k = 0; k < 6; ++k) ep[k] = ep_c[(size_t)k * Nq + q];
-      j2_stress(mat, scale, Hg, ep, epe_c[q], sig, epn, epe_n, pay);
+      for (int k = 0; k < 6; ++k) ep[k] = a.ep_c[(size_t)k * Nq + q];
+      j2_stress(mat, scale, Hg, ep, a.epe_c[q], sig, epn, epe_n, pay);
     } else if (model == M_TI) {
       ti_stress(mat, scale, Hg, sig);
     } else {
       le_stress(mat, scale, Hg, sig);
     }
-    // caller layout: point e * 8 + g (the reference's gp_idx)
-    const size_t o = (size_t)9 * ((size_t)eu * kHexGauss + g);
-    for (int k = 0; k < 9; ++k) {
-      if (F_out) F_out[o + k] = F[k];
-      if (sig_out) sig_out[o + k] = sig[k];
+    if (MISES) {
+#pragma unroll
+      for (int k = 0; k < 9; ++k) mean[k] = g ? mean[k] + sig[k] : sig[k];
+    } else {
+      // caller layout: point e * 8 + g (the reference's gp_idx)
+      double* row = s_row[threadIdx.x / 32];
+      if (a.F_out) store_rows9(F, row, lane, rows, eu * kHexGauss + g, a.F_out);
+      if (a.sig_out) store_rows9(sig, row, lane, rows, eu * kHexGauss + g, a.sig_out);
     }
+  }
+  if (MISES && lane < rows) {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) mean[k] /= (double)kHexGauss;
+    const double vm = von_mises9(mean);
+    const int4 p0 = __ldg(m.spos + 2 * (size_t)e), p1 = __ldg(m.spos + 2 * (size_t)e + 1);
+    const int pos[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+#pragma unroll
+    for (int k = 0; k < 8; ++k) __stcg(a.stage_d + pos[k], vm);
   }
 }
 
@@ -754,15 +775,21 @@ void launch_diag_hex(const DiagArgs& a, int model, cudaStream_t s) {
   a.boff ? hex_diag<true>(a, model, s) : hex_diag<false>(a, model, s);
 }
 
-void launch_stress_hex(const MeshDev& m, const DevMat<double>* matD, int model, const double* u,
-                       const double* ep_c, const double* epe_c, const int* perm_elem, double* F_out,
-                       double* sig_out, cudaStream_t s) {
-  const int t = 128, gb = nblk(m.n_elems, t);
+template <int MODEL>
+static void hex_stress_go(const StressArgs& a, bool mises, cudaStream_t s) {
+  const int g = nblk(a.m.n_elems, 128);
+  if (mises)
+    hex_stress_kernel<MODEL, true><<<g, 128, 0, s>>>(a);
+  else
+    hex_stress_kernel<MODEL, false><<<g, 128, 0, s>>>(a);
+}
+
+void launch_stress_hex(const StressArgs& a, int model, bool mises, cudaStream_t s) {
   switch (model) {
-    case M_LE: hex_stress_kernel<M_LE><<<gb, t, 0, s>>>(m, matD, u, ep_c, epe_c, perm_elem, F_out, sig_out); break;
-    case M_NH: hex_stress_kernel<M_NH><<<gb, t, 0, s>>>(m, matD, u, ep_c, epe_c, perm_elem, F_out, sig_out); break;
-    case M_J2: hex_stress_kernel<M_J2><<<gb, t, 0, s>>>(m, matD, u, ep_c, epe_c, perm_elem, F_out, sig_out); break;
-    default: hex_stress_kernel<-1><<<gb, t, 0, s>>>(m, matD, u, ep_c, epe_c, perm_elem, F_out, sig_out); break;
+    case M_LE: hex_stress_go<M_LE>(a, mises, s); break;
+    case M_NH: hex_stress_go<M_NH>(a, mises, s); break;
+    case M_J2: hex_stress_go<M_J2>(a, mises, s); break;
+    default: hex_stress_go<-1>(a, mises, s); break;
   }
 }
 

@@ -504,12 +504,22 @@ void launch_cg_update(float* x, float* r, const float* p, const float* y, const 
                       int precond_in_update = 1);
 void launch_cg_pupdate(float* p, const float* r, const float* dinv, int n_nodes, CGState* cg,
                        cudaStream_t s);
-void launch_stress(const MeshDev& m, const DevMat<double>* matD, int model, const double* u,
-                   const double* ep_c, const double* epe_c, const int* perm_elem, double* F_out,
-                   double* sig_out, cudaStream_t s);
-// nodal von Mises from caller-order element stresses (sum, or average)
-void launch_nodal_mises(const MeshDev& m, const int* perm_elem, const int* perm_node, const double* sig_user,
-                        int average, double* out_user, cudaStream_t s);
+struct StressArgs {
+  MeshDev m;
+  const DevMat<double>* matD;
+  const double* u;
+  const double* ep_c;
+  const double* epe_c;
+  const int* perm_elem;
+  double* F_out;      // caller order, may be null
+  double* sig_out;    // caller order, may be null
+  double* stage_d;    // nodal von Mises: element values in node_slots order
+};
+void launch_stress(const StressArgs& a, int model, cudaStream_t s);
+// nodal von Mises (sum over a node's elements, or average): two kernels, the
+// element pass through a.stage_d
+void launch_nodal_mises(const StressArgs& a, int model, const int* perm_node, int average, double* out_user,
+                        cudaStream_t s);
 void launch_refq(const MeshDev& m, const int* perm_elem, double* dNdX, double* vol,
                  cudaStream_t s);
 // HEX8 (fem_hex8.cu): element pass writing slot vectors in node_slots order
@@ -517,9 +527,7 @@ void launch_refq(const MeshDev& m, const int* perm_elem, double* dNdX, double* v
 void launch_residual_hex(const ResArgs& a, int model, cudaStream_t s);
 void launch_matvec_hex(const MvArgs& a, int model, cudaStream_t s);
 void launch_diag_hex(const DiagArgs& a, int model, cudaStream_t s);
-void launch_stress_hex(const MeshDev& m, const DevMat<double>* matD, int model, const double* u,
-                       const double* ep_c, const double* epe_c, const int* perm_elem, double* F_out,
-                       double* sig_out, cudaStream_t s);
+void launch_stress_hex(const StressArgs& a, int model, bool mises, cudaStream_t s);
 void launch_refq_hex(const MeshDev& m, const int* perm_elem, double* dNdX, double* vol, cudaStream_t s);
 // the node gather of the two-phase matvec (fem_kernels.cu)
 void launch_node_gather(const MvArgs& a, cudaStream_t s);
