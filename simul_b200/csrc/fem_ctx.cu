@@ -62,6 +62,7 @@ struct FemCtx {
 
   // device buffers
   double* X64 = nullptr;
+  double* X64r = nullptr;
   float4* X32 = nullptr;
   int4* conn = nullptr;
   uint8_t* mat_id = nullptr;
@@ -254,6 +255,7 @@ struct FemCtx {
     m.n_blocks = n_blocks;
     m.nb = nb;
     m.X64 = X64;
+    m.X64r = X64r;
     m.X32 = X32;
     m.conn = conn;
     m.mat_id = mat_id;
@@ -390,7 +392,7 @@ void free_ctx(FemCtx* c) {
   if (c->ho_x) cudaFree(c->ho_x);
   if (c->ho_rhs) cudaFree(c->ho_rhs);
   if (c->spos) cudaFree(c->spos);
-  void* ptrs[] = {c->X64, c->X32, c->conn, c->mat_id, c->scale, c->blk_ptr, c->blk_home,
+  void* ptrs[] = {c->X64, c->X64r, c->X32, c->conn, c->mat_id, c->scale, c->blk_ptr, c->blk_home,
                   c->blk_elems, c->node_row, c->node_slots, c->fixed, c->fixed_vals, c->fext,
                   c->fixed_vals_full, c->fext_full,
                   c->u, c->u_base, c->R, c->tmpd, c->payload, c->ep_c, c->epe_c, c->ep_t,
@@ -542,15 +544,16 @@ int build_tables(FemCtx* c, const double* X, const int32_t* conn_user) {
   c->blk_entries = (int64_t)blk_elems.size();
 
   // device uploads
-  std::vector<double> X64(3 * (size_t)Nn);
+  std::vector<double> X64(3 * (size_t)Nn), X64r(4 * (size_t)Nn, 0.0);
   std::vector<float4> X32(Nn);
   for (int i = 0; i < Nn; ++i) {
     const int iu = c->perm_node[i];
-    for (int d = 0; d < 3; ++d) X64[3 * i + d] = X[3 * iu + d];
+    for (int d = 0; d < 3; ++d) X64[3 * i + d] = X64r[4 * (size_t)i + d] = X[3 * iu + d];
     X32[i] = make_float4((float)X[3 * iu], (float)X[3 * iu + 1], (float)X[3 * iu + 2], 0.f);
   }
   int st;
   if ((st = dalloc(c, &c->X64, X64.size()))) return st;
+  if ((st = dalloc(c, &c->X64r, X64r.size()))) return st;
   if ((st = dalloc(c, &c->X32, (size_t)Nn))) return st;
   if ((st = dalloc(c, &c->conn, conn.size()))) return st;
   if ((st = dalloc(c, &c->blk_ptr, blk_ptr.size()))) return st;
@@ -562,6 +565,7 @@ int build_tables(FemCtx* c, const double* X, const int32_t* conn_user) {
   if ((st = dalloc(c, &c->d_perm_node, (size_t)Nn))) return st;
   if ((st = dalloc(c, &c->d_perm_elem, (size_t)Ne))) return st;
   CK(cudaMemcpyAsync(c->X64, X64.data(), X64.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(c->X64r, X64r.data(), X64r.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(c->X32, X32.data(), X32.size() * sizeof(float4), cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(c->conn, conn.data(), conn.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(c->blk_ptr, blk_ptr.data(), blk_ptr.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
@@ -606,7 +610,7 @@ int alloc_state(FemCtx* c) {
   if ((st = dalloc(c, &c->boff, nf))) return st;
   // slot vectors of the two-phase passes; HEX8 diagonal blocks take 2 per slot
   if ((st = dalloc(c, &c->stage, c->npe == 8 ? 16 * Ne : 4 * Ne))) return st;
-  if ((st = dalloc(c, &c->stage_d, (c->npe == 8 ? 24 : 12) * Ne))) return st;
+  if ((st = dalloc(c, &c->stage_d, (c->npe == 8 ? 32 : 16) * Ne))) return st;
   if ((st = dalloc(c, &c->matD, (size_t)FEM_MAX_MATERIALS))) return st;
   if ((st = dalloc(c, &c->matF, (size_t)FEM_MAX_MATERIALS))) return st;
   // every reducing kernel's grid must fit: node blocks and node-parallel blocks
@@ -1009,14 +1013,16 @@ int ensure_assembled(FemCtx* c) {
   return FEM_OK;
 }
 
-int eval_residual(FemCtx* c, double* fneg_out_int, double* rnorm2) {
+// fneg_out: the negative internal force in caller order (may be null)
+int eval_residual(FemCtx* c, double* fneg_out, double* rnorm2) {
   ResArgs a;
   a.m = c->mesh();
   a.matD = c->matD;
   a.u = c->u;
   a.f_ext = c->fext;
   a.R = c->R;
-  a.fneg = fneg_out_int;
+  a.fneg = fneg_out;
+  a.fneg_perm = c->d_perm_node;
   a.payload = c->payload;
   a.ep_c = c->ep_c;
   a.epe_c = c->epe_c;
@@ -3011,11 +3017,7 @@ int fem_element_forces(void* ctx, const double* u, double* f_out, double* residu
     CKL();
   }
   double r2 = 0;
-  if ((st = eval_residual(c, f_out ? c->tmpd : nullptr, &r2))) return st;
-  if (f_out) {
-    ++c->n_launches; launch_scatter_d(c->tmpd, f_out, c->d_perm_node, c->Nn, c->stream);
-    CKL();
-  }
+  if ((st = eval_residual(c, f_out, &r2))) return st;
   if (residual_out) {
     ++c->n_launches; launch_scatter_d(c->R, residual_out, c->d_perm_node, c->Nn, c->stream);
     CKL();
@@ -3323,6 +3325,7 @@ int fem_profile_kernels(void* ctx, int32_t reps, double* ms_out) {
   ra.f_ext = c->fext;
   ra.R = c->tmpd;
   ra.fneg = nullptr;
+  ra.fneg_perm = nullptr;
   ra.payload = c->payload;
   ra.ep_c = c->ep_c;
   ra.epe_c = c->epe_c;

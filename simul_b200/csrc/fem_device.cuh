@@ -521,6 +521,29 @@ __device__ __forceinline__ void diag_store(const float* acc, uint8_t fx, int nod
   reinterpret_cast<float4*>(boff)[node] = ov;
 }
 
+// 32-byte rows of doubles (x, y, z, unused), one load or store instruction
+// and one whole sector per row; rows are 32-byte aligned.
+__device__ __forceinline__ void load_row3(const double* p, double (&v)[3]) {
+  double w;
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(w) : "l"(p));
+}
+__device__ __forceinline__ void load_row3_nc(const double* p, double (&v)[3]) {
+  double w;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(w) : "l"(p));
+}
+__device__ __forceinline__ void store_row3(double* p, double x, double y, double z) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(x), "d"(y), "d"(z), "d"(0.0) : "memory");
+}
+
+// One thread's own 8-byte asynchronous copies into shared memory: the thread
+// that issued them reads them after copy8_wait, no barrier between.
+__device__ __forceinline__ void copy8(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy8_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void copy8_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
+
 // Von Mises stress of a 3 x 3 stress.
 __device__ __forceinline__ double von_mises9(const double (&s)[9]) {
   const double s11 = s[0], s22 = s[4], s33 = s[8], s12 = s[1], s23 = s[5], s13 = s[2];

@@ -210,12 +210,30 @@ __device__ __forceinline__ void hex_vertex(const T A[7][3], int a, T f[3]) {
 
 // ───────────────────────── residual (FP64) ─────────────────────────
 
+// One thread per element, its eight points in turn.  What bounds it: 229
+// registers leave 8 warps an SM, and a point's history came from memory right
+// before its return map.  The histories of all eight points are copied to the
+// thread's own slice of shared memory first, beside the gathers: 49 us against
+// 60 at 113,000 J2 elements, both kernels repeated 61 us against 77.  Held to
+// 168 registers for 12 warps an SM it spills, 56 us.
 template <int MODEL>
 __global__ void __launch_bounds__(128) hex_res_elem_kernel(const __grid_constant__ ResArgs a) {
   const MeshDev& m = a.m;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= m.n_elems) return;
   const size_t Ne = (size_t)m.n_elems, Nq = kHexGauss * Ne;
+  extern __shared__ double s_h[];
+  double* h = s_h + threadIdx.x;   // point g, word k at h[128 * (7 * g + k)]
+  if constexpr (MODEL == M_J2) {
+#pragma unroll 1
+    for (int g = 0; g < kHexGauss; ++g) {
+      const size_t q = (size_t)g * Ne + e;
+#pragma unroll
+      for (int k = 0; k < 6; ++k) copy8(h + 128 * (7 * g + k), a.ep_c + (size_t)k * Nq + q);
+      copy8(h + 128 * (7 * g + 6), a.epe_c + q);
+    }
+    copy8_commit();
+  }
   int nid[8];
   hex_nodes(m, e, nid);
   double cx[7][3], cu[7][3];
@@ -224,10 +242,9 @@ __global__ void __launch_bounds__(128) hex_res_elem_kernel(const __grid_constant
 #pragma unroll
     for (int k = 0; k < 8; ++k)
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        xr[k][d] = __ldg(m.X64 + 3 * nid[k] + d);
-        uv[k][d] = __ldg(a.u + 3 * nid[k] + d);
-      }
+      for (int d = 0; d < 3; ++d) uv[k][d] = __ldg(a.u + 3 * nid[k] + d);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) load_row3_nc(m.X64r + 4 * (size_t)nid[k], xr[k]);
     hex_coeffs(xr, cx);   // the monomial coefficients do not see the position
     hex_coeffs(uv, cu);
   }
@@ -235,6 +252,7 @@ __global__ void __launch_bounds__(128) hex_res_elem_kernel(const __grid_constant
   const double scale = (double)__ldg(m.scale + e);
   const int model = MODEL >= 0 ? MODEL : mat.model;
   const int npay = model_pay_words(model);
+  if constexpr (MODEL == M_J2) copy8_wait<0>();
   double A[7][3];
 #pragma unroll
   for (int k = 0; k < 7; ++k) A[k][0] = A[k][1] = A[k][2] = 0.0;
@@ -260,8 +278,8 @@ __global__ void __launch_bounds__(128) hex_res_elem_kernel(const __grid_constant
     } else if (model == M_J2) {
       double ep[6], epn[6], epe_n;
 #pragma unroll
-      for (int k = 0; k < 6; ++k) ep[k] = a.ep_c[(size_t)k * Nq + q];
-      j2_stress(mat, scale, Hg, ep, a.epe_c[q], S, epn, epe_n, pay);
+      for (int k = 0; k < 6; ++k) ep[k] = MODEL == M_J2 ? h[128 * (7 * g + k)] : a.ep_c[(size_t)k * Nq + q];
+      j2_stress(mat, scale, Hg, ep, MODEL == M_J2 ? h[128 * (7 * g + 6)] : a.epe_c[q], S, epn, epe_n, pay);
 #pragma unroll
       for (int k = 0; k < 6; ++k) a.ep_t[(size_t)k * Nq + q] = epn[k];
       a.epe_t[q] = epe_n;
@@ -281,8 +299,7 @@ __global__ void __launch_bounds__(128) hex_res_elem_kernel(const __grid_constant
   for (int k = 0; k < 8; ++k) {
     double f[3];
     hex_vertex(A, k, f);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) a.stage_d[3 * (size_t)pos[k] + d] = f[d];
+    store_row3(a.stage_d + 4 * (size_t)pos[k], f[0], f[1], f[2]);
   }
 }
 
@@ -295,13 +312,20 @@ __global__ void __launch_bounds__(256) hex_res_gather_kernel(const __grid_consta
   if (n < m.n_nodes) {
     double acc[3] = {0.0, 0.0, 0.0};
     const int j0 = __ldg(m.node_row + n), j1 = __ldg(m.node_row + n + 1);
-    for (int j = j0; j < j1; ++j)
+    for (int j = j0; j < j1; j += 8) {   // eight rows in flight, added in order
+      double v[8][3];
 #pragma unroll
-      for (int d = 0; d < 3; ++d) acc[d] += a.stage_d[3 * (size_t)j + d];
+      for (int k = 0; k < 8; ++k) load_row3(a.stage_d + 4 * (size_t)min(j + k, j1 - 1), v[k]);
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (j + k < j1)
+#pragma unroll
+          for (int d = 0; d < 3; ++d) acc[d] += v[k][d];
+    }
     const uint8_t fx = m.fixed[n];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      if (a.fneg) a.fneg[3 * n + d] = acc[d];
+      if (a.fneg) a.fneg[3 * (a.fneg_perm ? a.fneg_perm[n] : n) + d] = acc[d];
       const double r = ((fx >> d) & 1) ? 0.0 : a.f_ext[3 * n + d] + acc[d];
       a.R[3 * n + d] = r;
       r2 += r * r;
@@ -723,16 +747,22 @@ void launch_coarse_cells_hex(const CoarseArgs& a, int model, cudaStream_t s) {
   }
 }
 
+template <int MODEL>
+static void hex_res(const ResArgs& a, cudaStream_t s) {
+  constexpr size_t smem = MODEL == M_J2 ? sizeof(double) * 7 * kHexGauss * 128 : 0;
+  if (smem) raise_smem_limit_k(hex_res_elem_kernel<MODEL>);
+  hex_res_elem_kernel<MODEL><<<nblk(a.m.n_elems, 128), 128, smem, s>>>(a);
+}
+
 void launch_residual_hex(const ResArgs& a, int model, cudaStream_t s) {
-  const int ge = nblk(a.m.n_elems, 128);
   switch (model) {
-    case M_LE: hex_res_elem_kernel<M_LE><<<ge, 128, 0, s>>>(a); break;
-    case M_NH: hex_res_elem_kernel<M_NH><<<ge, 128, 0, s>>>(a); break;
-    case M_MR: hex_res_elem_kernel<M_MR><<<ge, 128, 0, s>>>(a); break;
-    case M_J2: hex_res_elem_kernel<M_J2><<<ge, 128, 0, s>>>(a); break;
-    case M_TI: hex_res_elem_kernel<M_TI><<<ge, 128, 0, s>>>(a); break;
-    case M_FMR: hex_res_elem_kernel<M_FMR><<<ge, 128, 0, s>>>(a); break;
-    default: hex_res_elem_kernel<-1><<<ge, 128, 0, s>>>(a); break;
+    case M_LE: hex_res<M_LE>(a, s); break;
+    case M_NH: hex_res<M_NH>(a, s); break;
+    case M_MR: hex_res<M_MR>(a, s); break;
+    case M_J2: hex_res<M_J2>(a, s); break;
+    case M_TI: hex_res<M_TI>(a, s); break;
+    case M_FMR: hex_res<M_FMR>(a, s); break;
+    default: hex_res<-1>(a, s); break;
   }
   hex_res_gather_kernel<<<nblk(a.m.n_nodes, 256), 256, 0, s>>>(a);
 }

@@ -70,6 +70,7 @@ struct MeshDev {
   int n_blocks;
   int nb;
   const double* X64;        // [3 Nn]
+  const double* X64r;       // [4 Nn] the same in 32-byte rows
   const float4* X32;        // [Nn]
   const int4* conn;         // [Ne]
   const uint8_t* mat_id;    // [Ne]
@@ -128,7 +129,8 @@ struct ResArgs {
   double* rnorm2;           // [1] ||R||^2 (free DOFs)
   Reduce red;
   int red_site;
-  double* stage_d;          // HEX8: [3 * 8 Ne] element slot forces in node_slots order
+  double* stage_d;          // [4 * npe Ne] element slot forces in node_slots order, 32-byte rows
+  const int* fneg_perm;     // if set, row n of fneg goes to row fneg_perm[n]
 };
 
 // Element-block matvec tables (MV_ELEM_BLOCK, TET4).  Element block k holds

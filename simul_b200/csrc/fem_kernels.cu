@@ -80,19 +80,20 @@ __device__ __forceinline__ void gather_chunk_w(const uint32_t* s_slots, const fl
 // Element e's four slot forces (FP64, the negative internal force of its
 // vertices) from u; with write_state also its tangent payload and J2 trial
 // history.
+// staged_h, if set: the element's committed history (6 strains, 1 equivalent
+// strain at stride 128), already in shared memory.
 template <int MODEL>
-__device__ __forceinline__ void res_element(const ResArgs& a, int e, bool write_state, double f[4][3]) {
+__device__ __forceinline__ void res_element(const ResArgs& a, int e, const int4 cn, const double* staged_h,
+                                            bool write_state, double f[4][3]) {
   const MeshDev& m = a.m;
-  const int4 cn = __ldg(m.conn + e);
   const int nid[4] = {cn.x, cn.y, cn.z, cn.w};
   double xv[4][3], uv[4][3];
 #pragma unroll
-  for (int k = 0; k < 4; ++k)
+  for (int k = 0; k < 4; ++k) {
+    load_row3_nc(m.X64r + 4 * (size_t)nid[k], xv[k]);
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      xv[k][d] = __ldg(m.X64 + 3 * nid[k] + d);
-      uv[k][d] = __ldg(a.u + 3 * nid[k] + d);
-    }
+    for (int d = 0; d < 3; ++d) uv[k][d] = __ldg(a.u + 3 * nid[k] + d);
+  }
   TetGeom<double> g;
   tet_geom(xv[0], xv[1], xv[2], xv[3], g);
   double D[3][3];
@@ -114,8 +115,8 @@ __device__ __forceinline__ void res_element(const ResArgs& a, int e, bool write_
   } else if (model == M_J2) {
     double ep[6], epn[6], epe_n;
 #pragma unroll
-    for (int k = 0; k < 6; ++k) ep[k] = a.ep_c[(size_t)k * m.n_elems + e];
-    const double epe = a.epe_c[e];
+    for (int k = 0; k < 6; ++k) ep[k] = staged_h ? staged_h[128 * k] : a.ep_c[(size_t)k * m.n_elems + e];
+    const double epe = staged_h ? staged_h[128 * 6] : a.epe_c[e];
     j2_stress(mat, scale, Hg, ep, epe, S, epn, epe_n, pay);
     if (write_state) {
 #pragma unroll
@@ -158,7 +159,8 @@ __global__ void __launch_bounds__(NB) residual_kernel(const __grid_constant__ Re
     const int idx = c0 + tid;
     if (idx < e1) {
       double f[4][3];
-      res_element<MODEL>(a, __ldg(m.blk_elems + idx), idx < home_end, f);
+      const int e = __ldg(m.blk_elems + idx);
+      res_element<MODEL>(a, e, __ldg(m.conn + e), nullptr, idx < home_end, f);
 #pragma unroll
       for (int s = 0; s < 4; ++s)
 #pragma unroll
@@ -175,7 +177,7 @@ __global__ void __launch_bounds__(NB) residual_kernel(const __grid_constant__ Re
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       const double fn = accs[d];
-      if (a.fneg) a.fneg[3 * node + d] = fn;
+      if (a.fneg) a.fneg[3 * (a.fneg_perm ? a.fneg_perm[node] : node) + d] = fn;
       const double r = ((fx >> d) & 1) ? 0.0 : a.f_ext[3 * node + d] + fn;
       a.R[3 * node + d] = r;
       r2 += r * r;
@@ -194,24 +196,59 @@ __global__ void __launch_bounds__(NB) residual_kernel(const __grid_constant__ Re
 // Two-phase FP64 residual.  res_elem_kernel: one thread per element, each
 // element evaluated once (the fused node-block kernel above evaluates an
 // element shared by several node blocks in each of them), its four slot
-// forces stored at their positions in node-slot order (stage_d, three doubles
-// per slot).  res_gather_kernel: kGatherLanes lanes per node add the node's
+// forces stored at their positions in node-slot order (stage_d, one 32-byte
+// row per slot).  res_gather_kernel: kGatherLanes lanes per node add the node's
 // contiguous slot range (lane k: slots k, k + kGatherLanes, ...; then xor
 // steps in a fixed order), R = f_ext + f on free DOFs and the fixed-order
 // FP64 sum of ||R||^2.  Bitwise reproducible; the node sums are associated
 // differently from the fused kernel's (agreement to rounding).
+//
+// What bounds it: with 95 registers 20 warps fit an SM, too few to cover a
+// chain of streamed loads, gathers and FP64 arithmetic, and 8-byte accesses
+// at 24-byte rows kept the L1 pipe at two thirds.  So the next element's
+// connectivity, slots and material and its J2 history (its own slice of shared
+// memory) are under way while the current element is evaluated, and
+// coordinates and slot forces move as whole 32-byte rows: 35 us against 46 at
+// 566,000 J2 elements (caches cold), the pair of kernels 59 us against 68 when
+// repeated.  More warps do not help: held to 96 registers it spills, 41 us.
 template <int MODEL>
 __global__ void __launch_bounds__(128) res_elem_kernel(const __grid_constant__ ResArgs a) {
+  constexpr bool kStage = MODEL == M_J2;
+  __shared__ double s_h[kStage ? 2 : 1][kStage ? 7 * 128 : 1];
+  const MeshDev& m = a.m;
+  const int n = m.n_elems, stride = (int)gridDim.x * 128, tid = (int)threadIdx.x;
+  int e = (int)blockIdx.x * 128 + tid;
+  if (e >= n) return;
+  auto fetch = [&](int el, int b) {
+    if constexpr (kStage) {
+#pragma unroll
+      for (int k = 0; k < 6; ++k) copy8(&s_h[b][128 * k + tid], a.ep_c + (size_t)k * n + el);
+      copy8(&s_h[b][128 * 6 + tid], a.epe_c + el);
+      copy8_commit();
+    }
+  };
+  int4 cn = __ldg(m.conn + e);
+  fetch(e, 0);
   // persistent: one wave of CTAs walks the elements in grid-stride order
-  for (int e = (int)blockIdx.x * 128 + (int)threadIdx.x; e < a.m.n_elems; e += (int)gridDim.x * 128) {
+  for (int b = 0;; b ^= 1) {
+    const int4 sp = __ldg(m.spos + e);
+    const int next = e + stride;
+    int4 cn_next = cn;
+    if (next < n) {
+      cn_next = __ldg(m.conn + next);
+      fetch(next, b ^ 1);
+      if (kStage) copy8_wait<1>();
+    } else if (kStage) {
+      copy8_wait<0>();
+    }
     double f[4][3];
-    res_element<MODEL>(a, e, true, f);
-    const int4 sp = __ldg(a.m.spos + e);
+    res_element<MODEL>(a, e, cn, kStage ? &s_h[b][tid] : nullptr, true, f);
     const int pos[4] = {sp.x, sp.y, sp.z, sp.w};
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-#pragma unroll
-      for (int d = 0; d < 3; ++d) __stcg(a.stage_d + 3 * (size_t)pos[k] + d, f[k][d]);
+    for (int k = 0; k < 4; ++k) store_row3(a.stage_d + 4 * (size_t)pos[k], f[k][0], f[k][1], f[k][2]);
+    if (next >= n) break;
+    e = next;
+    cn = cn_next;
   }
 }
 
@@ -691,16 +728,33 @@ __global__ void __launch_bounds__(256) node_gather_persist_kernel(const __grid_c
 }
 
 // One node's residual row (LANES lanes of a group add its slot range; the
-// group's lane 0 stores R and fneg) and its ||R||^2 term (lane 0).
+// group's lane 0 stores R and fneg) and its ||R||^2 term (lane 0).  The row
+// loads of a lane are issued together, and with them what the end needs: the
+// group's time is one round trip after the row bounds, not one per slot.
 template <int LANES>
 __device__ __forceinline__ double res_gather_node(const ResArgs& a, int n, int sub) {
   const MeshDev& m = a.m;
-  double acc[3] = {0.0, 0.0, 0.0};
+  double acc[3] = {0.0, 0.0, 0.0}, fe[3] = {0.0, 0.0, 0.0};
+  int fx = 0, to = n;
   if (n < m.n_nodes) {
     const int j0 = __ldg(m.node_row + n), j1 = __ldg(m.node_row + n + 1);
-    for (int j = j0 + sub; j < j1; j += LANES)
+    if (sub == 0) {
+      fx = m.fixed[n];
+      if (a.fneg && a.fneg_perm) to = __ldg(a.fneg_perm + n);
 #pragma unroll
-      for (int d = 0; d < 3; ++d) acc[d] += __ldcg(a.stage_d + 3 * (size_t)j + d);
+      for (int d = 0; d < 3; ++d) fe[d] = __ldg(a.f_ext + 3 * (size_t)n + d);
+    }
+    constexpr int kBatch = 6;
+    for (int j = j0 + sub; j < j1; j += kBatch * LANES) {
+      double v[kBatch][3];
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k) load_row3(a.stage_d + 4 * (size_t)min(j + k * LANES, j1 - 1), v[k]);
+#pragma unroll
+      for (int k = 0; k < kBatch; ++k)
+        if (j + k * LANES < j1)
+#pragma unroll
+          for (int d = 0; d < 3; ++d) acc[d] += v[k][d];
+    }
   }
 #pragma unroll
   for (int o = 1; o < LANES; o <<= 1)
@@ -708,11 +762,10 @@ __device__ __forceinline__ double res_gather_node(const ResArgs& a, int n, int s
     for (int d = 0; d < 3; ++d) acc[d] += __shfl_xor_sync(0xffffffffu, acc[d], o);
   double r2 = 0.0;
   if (n < m.n_nodes && sub == 0) {
-    const uint8_t fx = m.fixed[n];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      if (a.fneg) a.fneg[3 * n + d] = acc[d];
-      const double r = ((fx >> d) & 1) ? 0.0 : a.f_ext[3 * n + d] + acc[d];
+      if (a.fneg) a.fneg[3 * (size_t)to + d] = acc[d];
+      const double r = ((fx >> d) & 1) ? 0.0 : fe[d] + acc[d];
       a.R[3 * n + d] = r;
       r2 += r * r;
     }
