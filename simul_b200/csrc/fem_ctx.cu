@@ -966,7 +966,7 @@ int ensure_asm_tables(FemCtx* c) {
       (st = up(&edges, h.edges)) || (st = up(&eptr, h.eptr)) || (st = up(&list, h.list)))
     return st;
   if ((st = asm_upload(c, &words, (const uint32_t*)nullptr, (size_t)h.slice_step.back() * kAsmStepWords))) return st;
-  if ((st = asm_upload(c, &c->pcg_part, (const double*)nullptr, 3 * (size_t)h.grid))) return st;
+  if ((st = asm_upload(c, &c->pcg_part, (const double*)nullptr, 4 * (size_t)h.grid))) return st;
   if ((st = asm_upload(c, &c->pcg_bar, (const unsigned int*)nullptr, (size_t)1))) return st;
   if ((st = asm_upload(c, &c->pcg_p2, (const float*)nullptr, 4 * (size_t)c->Nn))) return st;
   S.grid = h.grid;
@@ -974,7 +974,7 @@ int ensure_asm_tables(FemCtx* c) {
   S.n_edges = (int)h.edges.size();
   S.max_slices = h.max_slices;
   S.max_halo = h.max_halo;
-  S.max_cols = h.max_cols;
+  S.max_cols = (h.max_cols + 3) & ~3;  // (float4 arrays follow the planes)
   S.max_pieces = h.max_pieces;
   S.cta_row = cta_row;
   S.cta_slice = cta_slice;
@@ -1981,8 +1981,13 @@ int ensure_pcg_tables(FemCtx* c, bool two_level) {
   CK(cudaMemcpyAsync(corner.data(), c->cdev.cell_corner, corner.size() * sizeof(int), cudaMemcpyDeviceToHost,
                      c->stream));
   CK(cudaStreamSynchronize(c->stream));
+  std::vector<int> halo_ptr(c->asm_cta_row.size());
+  CK(cudaMemcpy(halo_ptr.data(), c->asmdev.halo_ptr, halo_ptr.size() * sizeof(int), cudaMemcpyDeviceToHost));
+  std::vector<int> halo((size_t)halo_ptr.back());
+  if (!halo.empty())
+    CK(cudaMemcpy(halo.data(), c->asmdev.halo, halo.size() * sizeof(int), cudaMemcpyDeviceToHost));
   PcgCoarseHost h;
-  if (!pcg_coarse_tables(c->asm_cta_row, node_cell, corner, c->cdev.n_cn,
+  if (!pcg_coarse_tables(c->asm_cta_row, halo_ptr, halo, node_cell, corner, c->cdev.n_cn,
                          c->cdev.full_ld ? 0 : (c->cdev.Ainv16 ? 2 : 4), &h)) {
     c->pcg_ok = false;
     return FEM_OK;
@@ -1993,7 +1998,9 @@ int ensure_pcg_tables(FemCtx* c, bool two_level) {
   if ((st = pcg_upload(c, bufs, &t.tab_ptr, h.tab_ptr))) return st;
   if ((st = pcg_upload(c, bufs, &t.tab, h.tab))) return st;
   if ((st = pcg_upload(c, bufs, &seg_rows, h.seg_rows))) return st;
-  if ((st = pcg_upload(c, bufs, &t.row_corners, h.row_corners))) return st;
+  if ((st = pcg_upload(c, bufs, &t.col_corners, h.col_corners))) return st;
+  if ((st = pcg_upload(c, bufs, &t.cn_ptr, h.cn_ptr))) return st;
+  t.merged = c->cdev.full_ld && 8 * h.n_seg <= kPcgMergedShares;
   if ((st = dalloc(c, &lat, (size_t)c->Nn))) return st;
   bufs.push_back(lat);
   launch_pcg_seg_lat(seg_rows, c->cdev.node_lat, c->Nn, lat, c->stream);

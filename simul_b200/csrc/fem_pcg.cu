@@ -3,23 +3,28 @@
 // iteration are separated by grid-wide barriers instead of kernel
 // boundaries.
 //
-//   A   p = z + beta p, q = K p, p.q                       | barrier
-//   B   x += alpha p, r -= alpha q, ||r||^2, P^T r shares  | barrier
-//   C1  r_c                                                | barrier
-//   C2  tiles of Ac^-1 r_c                                 | barrier
-//   D   z = S r + P y_c, r.z                               | barrier
+//   A   z = S r + P y_c, p = z + beta p, q = K p, p.q           | barrier
+//   B   x += alpha p, r -= alpha q, ||r||^2, S r, r.S r, shares
+//       of P^T r                                               | barrier
+//   C1  r_c                                                    | barrier
+//   C2  y_c = Ac^-1 r_c, r_c.y_c                               | barrier
 //
-// (Jacobi: A, and B with z = D^-1 r and r.z in it.)  The recurrences, the
+// (r.z = r.S r + r_c.y_c, so no phase of its own forms z before beta is known.
+// A small coarse space: every CTA adds up r_c itself, no barrier after C1.)
+// (Jacobi: A and B with z = D^-1 r.)  The recurrences, the
 // FP64 sums in a fixed order and the stopping tests are those of the kernel
 // chain.
 //
 // What bounds it: below about 50,000 rows the matrix stays in shared memory
 // for the whole solve and the phases' latencies are left: 2,700 cycles per
-// barrier and about 2,500 of dependent loads and sums per phase, 38,000 cycles
-// (20 us) an iteration at 16,000 rows against 30 us for the chain's seven
-// kernels.  At 121,000 rows the matrix (55 MB) and the packed BF16 coarse
-// inverse (60 MB) stream once per iteration, 85,000 cycles (45 us) against
-// 70 us: the rings hold 20 MB of them, the rest comes at 7 TB/s.
+// barrier and about 2,500 of dependent loads and sums per phase, 35,000 cycles
+// (18 us) an iteration at 16,000 rows against 30 us for the chain's seven
+// kernels (42,000 with z in a phase of its own, a barrier more, and one warp
+// per slice).  At 121,000 rows the matrix (55 MB) and the packed BF16 coarse
+// inverse (60 MB) stream once per iteration, 81,000 cycles (43 us) against
+// 70 us: the rings hold 20 MB of them, the rest comes at 7 TB/s.  All 128
+// registers are in use: loads held over a barrier beyond those of A spill and
+// cost more than they hide (the first row of C2: 92,000 cycles).
 //
 // The reference factorises the assembled tangent on the host
 // (backend/fea/fem/solver/static_solver.py:399-462).
@@ -36,7 +41,8 @@ namespace femb200 {
 
 // ───────────────────────── tables (host) ─────────────────────────
 
-bool pcg_coarse_tables(const std::vector<int>& cta_row, const std::vector<int>& node_cell,
+bool pcg_coarse_tables(const std::vector<int>& cta_row, const std::vector<int>& halo_ptr,
+                       const std::vector<int>& halo, const std::vector<int>& node_cell,
                        const std::vector<int>& cell_corner, int n_cn, int parts, PcgCoarseHost* o) {
   const int G = (int)cta_row.size() - 1, Nn = cta_row[G], n_dof = 3 * n_cn, nb = (n_dof + 63) / 64;
   std::vector<std::vector<int>> tabs(G, std::vector<int>(kTabWords, 0));
@@ -45,10 +51,11 @@ bool pcg_coarse_tables(const std::vector<int>& cta_row, const std::vector<int>& 
     tabs[g][word] = (int)tabs[g].size();
     tabs[g].insert(tabs[g].end(), v.begin(), v.end());
   };
-  // rows of each CTA by cell; the coarse nodes they interpolate from
+  // rows of each CTA by cell; the coarse nodes that its columns (its rows, then
+  // its halo) interpolate from
   std::vector<std::vector<int>> shares(n_cn), loc(G);
   o->seg_rows.reserve(Nn);
-  o->row_corners.resize(Nn);
+  o->col_corners.resize((size_t)Nn + halo.size());
   std::vector<std::pair<int, int>> by_cell;
   std::vector<int> seen(n_cn, -1), local(n_cn, 0), sptr;
   for (int g = 0; g < G; ++g) {
@@ -62,44 +69,52 @@ bool pcg_coarse_tables(const std::vector<int>& cta_row, const std::vector<int>& 
       const int cell = by_cell[j].first;
       size_t j1 = j;
       while (j1 < by_cell.size() && by_cell[j1].first == cell) ++j1;
-      uint32_t idx[8];
-      for (int q = 0; q < 8; ++q) {
-        const int cn = cell_corner[8 * (size_t)cell + q];
-        shares[cn].push_back(o->n_seg * 8 + q);
-        if (seen[cn] != g) {
-          seen[cn] = g;
-          local[cn] = (int)loc[g].size();
-          loc[g].push_back(cn);
-        }
-        idx[q] = (uint32_t)local[cn];
-        if (idx[q] > 0xffffu) return false;
-      }
-      const uint4 w = make_uint4(idx[0] | idx[1] << 16, idx[2] | idx[3] << 16, idx[4] | idx[5] << 16,
-                                 idx[6] | idx[7] << 16);
-      for (; j < j1; ++j) {
-        o->seg_rows.push_back(by_cell[j].second);
-        o->row_corners[by_cell[j].second] = w;
-      }
+      for (int q = 0; q < 8; ++q) shares[cell_corner[8 * (size_t)cell + q]].push_back(o->n_seg * 8 + q);
+      for (; j < j1; ++j) o->seg_rows.push_back(by_cell[j].second);
       sptr.push_back((int)j1);
       ++o->n_seg;
     }
     tabs[g][TAB_NSEG] = (int)sptr.size() - 1;
     put(g, TAB_SPTR, sptr);
+    const int nrow = cta_row[g + 1] - cta_row[g], nh = halo_ptr[g + 1] - halo_ptr[g];
+    // (ascending, so that neighbouring threads read neighbouring words of y_c)
+    auto cell_of = [&](int i) { return node_cell[i < nrow ? cta_row[g] + i : halo[halo_ptr[g] + i - nrow]]; };
+    std::vector<int>& lg = loc[g];
+    for (int i = 0; i < nrow + nh; ++i)
+      for (int q = 0; q < 8; ++q) {
+        const int cn = cell_corner[8 * (size_t)cell_of(i) + q];
+        if (seen[cn] != g) {
+          seen[cn] = g;
+          lg.push_back(cn);
+        }
+      }
+    if (lg.size() > 65536) return false;
+    std::sort(lg.begin(), lg.end());
+    for (size_t k = 0; k < lg.size(); ++k) local[lg[k]] = (int)k;
+    uint4* cc = o->col_corners.data() + cta_row[g] + halo_ptr[g];
+    for (int i = 0; i < nrow + nh; ++i) {
+      uint32_t idx[8];
+      for (int q = 0; q < 8; ++q) idx[q] = (uint32_t)local[cell_corner[8 * (size_t)cell_of(i) + q]];
+      cc[i] = make_uint4(idx[0] | idx[1] << 16, idx[2] | idx[3] << 16, idx[4] | idx[5] << 16, idx[6] | idx[7] << 16);
+    }
     tabs[g][TAB_NLOC] = (int)loc[g].size();
     put(g, TAB_LOC, loc[g]);
     o->max_loc = std::max(o->max_loc, (int)loc[g].size());
   }
+  // the shares of a coarse node lie together: each share's place
+  std::vector<int> place(8 * (size_t)o->n_seg);
+  o->cn_ptr.assign(1, 0);
+  for (int c = 0, at = 0; c < n_cn; ++c) {
+    for (int j : shares[c]) place[j] = at++;
+    o->cn_ptr.push_back(at);
+  }
   for (int g = 0; g < G; ++g) {
     const int c0 = (int)((int64_t)n_cn * g / G), c1 = (int)((int64_t)n_cn * (g + 1) / G);
-    std::vector<int> ptr(1, 0), list;
-    for (int c = c0; c < c1; ++c) {
-      list.insert(list.end(), shares[c].begin(), shares[c].end());
-      ptr.push_back((int)list.size());
-    }
     tabs[g][TAB_CN0] = c0;
     tabs[g][TAB_NCN] = c1 - c0;
-    put(g, TAB_CPTR, ptr);
-    put(g, TAB_CLIST, list);
+    put(g, TAB_CPTR, std::vector<int>(o->cn_ptr.begin() + c0, o->cn_ptr.begin() + c1 + 1));
+    const size_t s0 = 8 * (size_t)tabs[g][TAB_SEG0], n8 = 8 * (size_t)tabs[g][TAB_NSEG];
+    put(g, TAB_SPOS, std::vector<int>(place.begin() + s0, place.begin() + s0 + n8));
   }
   if (parts) {
     // tiles in super-blocks of about one CTA's share, so that a CTA touches
@@ -183,7 +198,6 @@ bool pcg_coarse_tables(const std::vector<int>& cta_row, const std::vector<int>& 
 namespace {
 
 constexpr int kWarps = kPcgThreads / 32;
-constexpr int kTileElems = 64 * 64;
 
 // This CTA's sum of v over its threads, in thread 0.
 __device__ __forceinline__ double cta_sum(double v, double* sred) {
@@ -198,6 +212,29 @@ __device__ __forceinline__ double cta_sum(double v, double* sred) {
     for (int o = kWarps / 2; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
   }
   return t;
+}
+
+// The same for two sums at once.
+__device__ __forceinline__ void cta_sum2(double& v, double& w, double* sv, double* sw) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    v += __shfl_down_sync(0xffffffffu, v, o);
+    w += __shfl_down_sync(0xffffffffu, w, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    sv[threadIdx.x >> 5] = v;
+    sw[threadIdx.x >> 5] = w;
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    v = threadIdx.x < kWarps ? sv[threadIdx.x] : 0.0;
+    w = threadIdx.x < kWarps ? sw[threadIdx.x] : 0.0;
+#pragma unroll
+    for (int o = kWarps / 2; o > 0; o >>= 1) {
+      v += __shfl_down_sync(0xffffffffu, v, o);
+      w += __shfl_down_sync(0xffffffffu, w, o);
+    }
+  }
 }
 
 // Grid-wide barrier number `epoch` (1, 2, ...): every CTA's earlier writes
@@ -518,20 +555,17 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_kernel(const __grid_consta
     }
     return buf;
   };
-  bool loaded = true;
+  bool loaded = false;   // this warp has waited for its resident slices
+  uint32_t total = 0;    // bytes of those it copies itself
   {
-    uint32_t total = 0;
     for (int s = warp; s < res; s += kWarps) total += (uint32_t)((s_step[s + 1] - s_step[s]) * kAsmStepBytes);
-    if (total > 0) {
-      loaded = false;
-      if (lane == 0) {
-        bulk::expect(bar + 2, total);
-        for (int s = warp; s < res; s += kWarps)
-          if (s_step[s + 1] > s_step[s])
-            bulk::copy(s_dyn + (size_t)(s_step[s] - s_step[0]) * kAsmStepBytes,
-                       a.as.words + (size_t)s_step[s] * kAsmStepWords,
-                       (uint32_t)((s_step[s + 1] - s_step[s]) * kAsmStepBytes), bar + 2);
-      }
+    if (total > 0 && lane == 0) {
+      bulk::expect(bar + 2, total);
+      for (int s = warp; s < res; s += kWarps)
+        if (s_step[s + 1] > s_step[s])
+          bulk::copy(s_dyn + (size_t)(s_step[s] - s_step[0]) * kAsmStepBytes,
+                     a.as.words + (size_t)s_step[s] * kAsmStepWords,
+                     (uint32_t)((s_step[s + 1] - s_step[s]) * kAsmStepBytes), bar + 2);
     }
     if (any)
       for (int k = 0; k < ns; ++k) issue();
@@ -540,7 +574,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_kernel(const __grid_consta
   double rz = 0.0, nrz = 0.0, rr0 = 0.0, tol2 = 0.0, rr = 0.0, pAp = 0.0, alpha = 0.0, beta = 0.0;
   bool first = true;  // the iteration after the initial residual: beta = 0, the old p and q are not read
   int iter = 0, done = 0, status = 0;
-  double *part_a = a.part, *part_b = a.part + G, *part_d = a.part + 2 * G;
+  double *part_a = a.part, *part_b = a.part + G, *part_d = a.part + 2 * G, *part_e = a.part + 3 * G;
   // this CTA's share of a sum (thread 0 stores it)
   auto post = [&](double* slot, double v, double* sh) {
     const double t = cta_sum(v, sh);
@@ -561,42 +595,123 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_kernel(const __grid_consta
     }
   };
 
+  // The operands of this thread's first kCols columns of A, loaded under the
+  // barrier in front of it: S r, the old p, and (two levels) the lattice
+  // coordinates, the corners' places in s_yc and the fixed bits
+  constexpr int kCols = TL ? 2 : 4;
+  const int nc = nrow + nh, col0 = row0 + a.as.halo_ptr[g];
+  float4 zv[kCols], pv[kCols], lv[kCols];
+  uint4 cv[kCols];
+  int fv[kCols];
+  auto col_load = [&](int i0, const float4* pold, bool no_p) {
+#pragma unroll
+    for (int u = 0; u < kCols; ++u) {
+      const int i = i0 + u * kPcgThreads;
+      if (i < nc) {
+        const int n = i < nrow ? row0 + i : s_halo[i - nrow];
+        zv[u] = z4[n];
+        pv[u] = no_p ? make_float4(0.f, 0.f, 0.f, 0.f) : pold[n];
+        if (TL) {
+          lv[u] = __ldg(a.c.node_lat + n);
+          cv[u] = __ldg(a.t.col_corners + col0 + i);
+          fv[u] = (int)a.m.fixed[n];
+        }
+      }
+    }
+  };
+  // B: rows of this thread
+  constexpr int kRows = 1;
+  float *px = scratch, *py = px + a.as.max_cols, *pz = py + a.as.max_cols;
+  float4 rv[kRows], xv[kRows], dv[kRows], ov[kRows];
+  auto row_load = [&](int i0, bool init) {
+#pragma unroll
+    for (int u = 0; u < kRows; ++u) {
+      const int n = row0 + i0 + u * kPcgThreads;
+      if (n < row1) {
+        if (!init) {
+          rv[u] = r4[n];
+          xv[u] = x4[n];
+        }
+        dv[u] = d4[n];
+        ov[u] = o4 ? o4[n] : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+  };
+  // Few slices: 2^split warps share the steps of one (a lone warp walks a
+  // row's entries one dependent load after another: 4,800 cycles for a slice
+  // that takes 1,000 of the SM's shared-memory time)
+  int split = 0;
+  if (res == nsl && nsl > 0)
+    while (nsl << (split + 1) <= kWarps) ++split;
+  float* s_split = scratch + 3 * a.as.max_cols + (TL ? 4 * a.t.max_loc : 0);  // [kWarps][3][32]
+
   for (bool init = true;; init = false) {
     if (!init) {
-      // ── A: p = z + beta p, q = K p ──
+      // ── A: z = S r + P y_c, p = z + beta p, q = K p ──
       // The CTA's columns of p (its rows, then its halo) go to shared memory
       // as three planes (gathering z by 16-byte loads per entry took 32 L1
       // cycles a warp, 34,000 cycles a product at 820 rows per CTA); the
       // rows' p also to the other buffer: neighbours still read the old one.
+      // Every CTA forms z and p of its halo itself, from the same operands in
+      // the same order as their owner: a sixth phase with its barrier cost
+      // more (5,000 cycles) than the halo's interpolation.
       const float4* po4 = p4;
       p4 = pn4;
       pn4 = const_cast<float4*>(po4);
-      const double lz = sum_load(part_d);
-      const int nc = nrow + nh;
+      const double lz = sum_load(part_d) + (TL ? sum_load(part_e) : 0.0);
       float *sx = scratch, *sy = sx + a.as.max_cols, *sz = sy + a.as.max_cols;
-      constexpr int kCols = 4;
-      for (int i0 = tid; i0 < nc || i0 == tid; i0 += kCols * kPcgThreads) {
-        float4 zv[kCols], pv[kCols];
+      float4* s_yc = reinterpret_cast<float4*>(sz + a.as.max_cols);  // y_c of the coarse nodes these columns use
+      if (TL) {
+        if (a.c.full_ld) {
+          const int* loc = tab + tab[TAB_LOC];
+          for (int k = tid; k < 3 * tab[TAB_NLOC]; k += kPcgThreads)
+            reinterpret_cast<float*>(s_yc + k / 3)[k % 3] = __ldcg(a.c.yc + 3 * loc[k / 3] + k % 3);
+        } else {
+          const int *yidx = tab + tab[TAB_YIDX], *yptr = tab + tab[TAB_YPTR], *ylist = tab + tab[TAB_YLIST];
+          for (int k = tid; k < 3 * tab[TAB_NLOC]; k += kPcgThreads) {
+            const int id = yidx[k], j1 = yptr[(id >> 6) + 1];
+            float s = 0.f;
+            constexpr int kU = 24;
+            for (int j = yptr[id >> 6]; j < j1; j += kU) {
+              float v[kU];
 #pragma unroll
-        for (int u = 0; u < kCols; ++u) {
-          const int i = i0 + u * kPcgThreads;
-          if (i < nc) {
-            const int n = i < nrow ? row0 + i : s_halo[i - nrow];
-            zv[u] = z4[n];
-            pv[u] = first ? make_float4(0.f, 0.f, 0.f, 0.f) : po4[n];
+              for (int u = 0; u < kU; ++u)
+                v[u] = j + u < j1 ? __ldcg(a.t.ypart + 64 * (size_t)ylist[j + u] + (id & 63)) : 0.f;
+#pragma unroll
+              for (int u = 0; u < kU; ++u) s += v[u];
+            }
+            reinterpret_cast<float*>(s_yc + k / 3)[k % 3] = s;
           }
         }
-        if (i0 == tid) {
-          nrz = sum_end(lz, ssum[2]);
-          beta = first ? 0.0 : nrz / rz;
-        }
-        const float bt = (float)beta;
+      } else {
+        col_load(tid, po4, first);
+      }
+      nrz = sum_end(lz, ssum[2]);  // (its barrier also covers s_yc)
+      beta = first ? 0.0 : nrz / rz;
+      const float bt = (float)beta;
+      for (int i0 = tid; i0 < nc; i0 += kCols * kPcgThreads) {
+        if (i0 != tid) col_load(i0, po4, first);
 #pragma unroll
         for (int u = 0; u < kCols; ++u) {
           const int i = i0 + u * kPcgThreads;
           if (i < nc) {
-            const float4 v =
-                make_float4(zv[u].x + bt * pv[u].x, zv[u].y + bt * pv[u].y, zv[u].z + bt * pv[u].z, 0.f);
+            float z0 = zv[u].x, z1 = zv[u].y, z2 = zv[u].z;
+            if (TL) {
+              const uint32_t cpk[4] = {cv[u].x, cv[u].y, cv[u].z, cv[u].w};
+              float c0 = 0.f, c1 = 0.f, c2 = 0.f;
+#pragma unroll
+              for (int k = 0; k < 8; ++k) {
+                const float4 y = s_yc[(cpk[k >> 1] >> (16 * (k & 1))) & 0xffffu];
+                const float w = tri_weight(lv[u].x, lv[u].y, lv[u].z, k);
+                c0 += w * y.x;
+                c1 += w * y.y;
+                c2 += w * y.z;
+              }
+              z0 = (fv[u] & 1) ? 0.f : z0 + c0;
+              z1 = (fv[u] & 2) ? 0.f : z1 + c1;
+              z2 = (fv[u] & 4) ? 0.f : z2 + c2;
+            }
+            const float4 v = make_float4(z0 + bt * pv[u].x, z1 + bt * pv[u].y, z2 + bt * pv[u].z, 0.f);
             sx[i] = v.x;
             sy[i] = v.y;
             sz[i] = v.z;
@@ -615,14 +730,19 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_kernel(const __grid_consta
       }
       __syncthreads();
       double pap = 0.0;
-      for (int s = warp; s < nsl; s += kWarps) {
-        const int t0 = s_step[s], t1 = s_step[s + 1];
+      for (int s = warp >> split; s < nsl; s += kWarps >> split) {
+        int t0 = s_step[s], t1 = s_step[s + 1];
+        if (split) {
+          const int n = t1 - t0, h = warp & ((1 << split) - 1);
+          t1 = t0 + (n * (h + 1) >> split);
+          t0 += n * h >> split;
+        }
         const int node = __ldg(a.as.slice_rows + 32 * (size_t)(sl0 + s) + lane);
         const int la = node >= 0 ? node - row0 : 0;
         const float xa = sx[la], ya = sy[la], za = sz[la];
         float y0 = 0.f, y1 = 0.f, y2 = 0.f;
-        if (s < res && !loaded) {
-          ok = bulk::wait(bar + 2, 0u) && ok;
+        if (s < res && !loaded && s_step[s + 1] > s_step[s]) {
+          ok = bulk::wait(bars + 3 * (s % kWarps) + 2, 0u) && ok;
           loaded = true;
         }
         for (int t = t0; t < t1; t += kPcgPiece) {
@@ -645,9 +765,31 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_kernel(const __grid_consta
             issue();
           }
         }
-        if (node >= 0) {
+        if (split) {
+          float* o = s_split + 96 * warp + lane;
+          o[0] = y0;
+          o[32] = y1;
+          o[64] = y2;
+        } else if (node >= 0) {
           q4[node] = make_float4(y0, y1, y2, 0.f);
           pap += (double)y0 * xa + (double)y1 * ya + (double)y2 * za;
+        }
+      }
+      if (split) {
+        __syncthreads();
+        if (warp < nsl) {  // a warp per slice adds its parts
+          const int node = __ldg(a.as.slice_rows + 32 * (size_t)(sl0 + warp) + lane);
+          float y[3];
+#pragma unroll
+          for (int d = 0; d < 3; ++d) {
+            y[d] = 0.f;
+            for (int h = 0; h < 1 << split; ++h) y[d] += s_split[96 * ((warp << split) + h) + 32 * d + lane];
+          }
+          if (node >= 0) {
+            const int la = node - row0;
+            q4[node] = make_float4(y[0], y[1], y[2], 0.f);
+            pap += (double)y[0] * sx[la] + (double)y[1] * sy[la] + (double)y[2] * sz[la];
+          }
         }
       }
       if (!ok) pap = __longlong_as_double(0x7ff8000000000000LL);
@@ -658,16 +800,18 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_kernel(const __grid_consta
       seg_load(warp);
     }
 
-    // ── B: x, r, ||r||^2 (Jacobi: also z = D^-1 r and r.z) ──
+    // ── B: x, r, ||r||^2, S r and r.S r ──
+    // (p comes from the planes, whose own rows then take r for the restriction)
     const double la = init ? 0.0 : sum_load(part_a);
-    float4 rv0, xv0, pv0, qv0;  // this thread's first row, in flight with the shares of p.q
-    if (!init && row0 + tid < row1) {
-      rv0 = r4[row0 + tid];
-      xv0 = x4[row0 + tid];
-      pv0 = p4[row0 + tid];
-      qv0 = q4[row0 + tid];
-    }
+    float4 qv[kRows];
+    auto q_load = [&](int i0) {
+#pragma unroll
+      for (int u = 0; u < kRows; ++u)
+        if (i0 + u * kPcgThreads < nrow) qv[u] = q4[row0 + i0 + u * kPcgThreads];
+    };
     if (!init) {
+      row_load(tid, false);
+      q_load(tid);
       pAp = sum_end(la, ssum[0]);
       if (!(pAp > 0.0) || !isfinite(pAp)) {
         done = status = 3;
@@ -679,42 +823,55 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_kernel(const __grid_consta
 
     const float al = (float)alpha;
     double lrr = 0.0, lrz = 0.0;
-    for (int n = row0 + tid; n < row1; n += kPcgThreads) {
-      float4 rv;
-      if (init) {
-        rv = make_float4((float)a.b[3 * (size_t)n], (float)a.b[3 * (size_t)n + 1], (float)a.b[3 * (size_t)n + 2], 0.f);
-        x4[n] = make_float4(0.f, 0.f, 0.f, 0.f);
-      } else {
-        const bool first = n == row0 + tid;
-        rv = first ? rv0 : r4[n];
-        float4 xv = first ? xv0 : x4[n];
-        const float4 pv = first ? pv0 : p4[n], qv = first ? qv0 : q4[n];
-        xv.x += al * pv.x; xv.y += al * pv.y; xv.z += al * pv.z;
-        rv.x -= al * qv.x; rv.y -= al * qv.y; rv.z -= al * qv.z;
-        x4[n] = xv;
-      }
-      r4[n] = rv;
-      lrr += (double)rv.x * rv.x + (double)rv.y * rv.y + (double)rv.z * rv.z;
-      if (!TL) {
-        const float4 dv = d4[n];
-        const float4 zv = make_float4(dv.x * rv.x, dv.y * rv.y, dv.z * rv.z, 0.f);
-        z4[n] = zv;
-        lrz += (double)rv.x * zv.x + (double)rv.y * zv.y + (double)rv.z * zv.z;
+    for (int i0 = tid; i0 < nrow; i0 += kRows * kPcgThreads) {
+      if (init || i0 != tid) row_load(i0, init);
+      if (!init && i0 != tid) q_load(i0);
+#pragma unroll
+      for (int u = 0; u < kRows; ++u) {
+        const int i = i0 + u * kPcgThreads, n = row0 + i;
+        if (i >= nrow) break;
+        float4 r = rv[u];
+        if (init) {
+          r = make_float4((float)a.b[3 * (size_t)n], (float)a.b[3 * (size_t)n + 1], (float)a.b[3 * (size_t)n + 2],
+                          0.f);
+          x4[n] = make_float4(0.f, 0.f, 0.f, 0.f);
+        } else {
+          r.x -= al * qv[u].x; r.y -= al * qv[u].y; r.z -= al * qv[u].z;
+          x4[n] = make_float4(xv[u].x + al * px[i], xv[u].y + al * py[i], xv[u].z + al * pz[i], 0.f);
+        }
+        r4[n] = r;
+        if (TL) {
+          px[i] = r.x;
+          py[i] = r.y;
+          pz[i] = r.z;
+        }
+        lrr += (double)r.x * r.x + (double)r.y * r.y + (double)r.z * r.z;
+        float4 sv = make_float4(dv[u].x * r.x, dv[u].y * r.y, dv[u].z * r.z, 0.f);
+        if (o4) {
+          sv.x += ov[u].x * r.y + ov[u].y * r.z;
+          sv.y += ov[u].x * r.x + ov[u].z * r.z;
+          sv.z += ov[u].y * r.x + ov[u].z * r.y;
+        }
+        z4[n] = sv;
+        lrz += (double)r.x * sv.x + (double)r.y * sv.y + (double)r.z * sv.z;
       }
     }
-    post(part_b, lrr, sred[0]);
-    if (!TL) post(part_d, lrz, sred[1]);
+    cta_sum2(lrr, lrz, sred[0], sred[1]);
+    if (tid == 0) {
+      part_b[g] = lrr;
+      part_d[g] = lrz;
+    }
     if (TL) {
       // restricted shares of the CTA's rows, a warp per cell, three cells in
-      // flight (the residuals above are this CTA's own, ordered by post's
+      // flight (the residuals above are this CTA's own, ordered by the sums'
       // barrier)
       for (int s0 = warp; s0 < nseg; s0 += kSegs * kWarps) {
         if (s0 != warp) seg_load(s0);
-        float4 rv[kSegs];
+        float3 sr[kSegs];
 #pragma unroll
         for (int u = 0; u < kSegs; ++u) {
-          const int n = __float_as_int(lt[u].w);
-          rv[u] = n >= 0 ? r4[n] : make_float4(0.f, 0.f, 0.f, 0.f);
+          const int i = __float_as_int(lt[u].w) - row0;
+          sr[u] = i >= 0 ? make_float3(px[i], py[i], pz[i]) : make_float3(0.f, 0.f, 0.f);
         }
 #pragma unroll
         for (int u = 0; u < kSegs; ++u) {
@@ -724,14 +881,15 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_kernel(const __grid_consta
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
             const float w = tri_weight(lt[u].x, lt[u].y, lt[u].z, k);
-            acc[4 * k] = w * rv[u].x;
-            acc[4 * k + 1] = w * rv[u].y;
-            acc[4 * k + 2] = w * rv[u].z;
+            acc[4 * k] = w * sr[u].x;
+            acc[4 * k + 1] = w * sr[u].y;
+            acc[4 * k + 2] = w * sr[u].z;
             acc[4 * k + 3] = 0.f;
           }
           for (int j = sptr[s] + 32 + lane; j < sptr[s + 1]; j += 32) {
             const float4 l = __ldg(lat + j);
-            const float4 v = r4[__float_as_int(l.w)];
+            const int i = __float_as_int(l.w) - row0;
+            const float3 v = make_float3(px[i], py[i], pz[i]);
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
               const float w = tri_weight(l.x, l.y, l.z, k);
@@ -751,45 +909,54 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_kernel(const __grid_consta
               acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
             }
           }
-          reinterpret_cast<float*>(a.t.seg_r)[(size_t)(tab[TAB_SEG0] + s) * 32 + lane] = acc[0];
+          reinterpret_cast<float*>(a.t.seg_r + (tab + tab[TAB_SPOS])[8 * s + (lane >> 2)])[lane & 3] = acc[0];
         }
       }
     }
     if (!grid_barrier(a.bar, ++epoch)) break;
     const double lr = sum_load(part_b);
+    const bool merged = TL && a.t.merged;
     if (TL) {
-      // ── C1: r_c, eight lanes per coarse node (before the stopping test: the
-      // shares of ||r||^2 arrive under it) ──
-      {
-        const int *cptr = tab + tab[TAB_CPTR], *clist = tab + tab[TAB_CLIST];
-        const int ncn = tab[TAB_NCN], sub = lane & 7;
-        for (int k = tid >> 3; k < ((ncn + 3) & ~3); k += kPcgThreads / 8) {
-          float v0 = 0.f, v1 = 0.f, v2 = 0.f;
-          if (k < ncn) {
-            const int j1 = cptr[k + 1];
-            constexpr int kU = 4;
-            for (int j = cptr[k] + sub; j < j1; j += 8 * kU) {
-              float4 v[kU];
+      // ── C1: r_c from its shares (before the stopping test: the shares of
+      // ||r||^2 arrive under it), a warp per coarse node where that is one
+      // round, else eight lanes; merged, every CTA adds up all of r_c for
+      // itself and the barrier falls away ──
+      const int* cptr = merged ? a.t.cn_ptr : tab + tab[TAB_CPTR];
+      const int ncn = merged ? a.c.n_cn : tab[TAB_NCN];
+      const int lanes = ncn <= kWarps ? 32 : 8, per = 32 / lanes, sub = lane & (lanes - 1);
+      float* out = merged ? scratch : a.c.rc + 3 * tab[TAB_CN0];
+      const int n4 = (ncn + per - 1) & ~(per - 1);
+      // (merged: the CTAs start at different nodes, so that they do not all
+      // read the same words of L2 at once)
+      const int rot = merged ? (int)((int64_t)g * n4 / G) & ~(per - 1) : 0;
+      for (int kr = tid / lanes; kr < n4; kr += kPcgThreads / lanes) {
+        const int k = kr + rot < n4 ? kr + rot : kr + rot - n4;
+        float v0 = 0.f, v1 = 0.f, v2 = 0.f;
+        if (k < ncn) {
+          const int j1 = cptr[k + 1];
+          constexpr int kU = 4;
+          for (int j = cptr[k] + sub; j < j1; j += lanes * kU) {
+            float4 v[kU];
 #pragma unroll
-              for (int u = 0; u < kU; ++u)
-                v[u] = j + 8 * u < j1 ? __ldcg(a.t.seg_r + clist[j + 8 * u]) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int u = 0; u < kU; ++u)
+              v[u] = j + lanes * u < j1 ? __ldcg(a.t.seg_r + j + lanes * u) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-              for (int u = 0; u < kU; ++u) {
-                v0 += v[u].x;
-                v1 += v[u].y;
-                v2 += v[u].z;
-              }
+            for (int u = 0; u < kU; ++u) {
+              v0 += v[u].x;
+              v1 += v[u].y;
+              v2 += v[u].z;
             }
           }
-#pragma unroll
-          for (int o = 4; o > 0; o >>= 1) {
-            v0 += __shfl_xor_sync(0xffffffffu, v0, o);
-            v1 += __shfl_xor_sync(0xffffffffu, v1, o);
-            v2 += __shfl_xor_sync(0xffffffffu, v2, o);
-          }
-          if (k < ncn && sub < 3) a.c.rc[3 * (tab[TAB_CN0] + k) + sub] = sub == 0 ? v0 : (sub == 1 ? v1 : v2);
         }
+        for (int o = lanes / 2; o > 0; o >>= 1) {
+          v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+          v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+          v2 += __shfl_xor_sync(0xffffffffu, v2, o);
+        }
+        if (k < ncn && sub < 3) out[3 * k + sub] = sub == 0 ? v0 : (sub == 1 ? v1 : v2);
       }
+      if (merged)
+        for (int k = 3 * ncn + tid; k < a.c.full_ld; k += kPcgThreads) scratch[k] = 0.f;
     }
     rr = sum_end(lr, ssum[1]);
     if (init) {
@@ -819,15 +986,18 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_kernel(const __grid_consta
       }
     }
     if (TL) {
-      if (!grid_barrier(a.bar, ++epoch)) break;
-      // ── C2: y_c = Ac^-1 r_c ──
+      if (!merged && !grid_barrier(a.bar, ++epoch)) break;
+      // ── C2: y_c = Ac^-1 r_c, and r_c.y_c = r.P y_c ──
+      double lrc = 0.0;
       if (a.c.full_ld) {
         // full rows, a warp each
         const int ld = a.c.full_ld, nd = a.c.n_dof;
         // (r_c is zero beyond n_dof)
-        for (int k = tid; k < ld / 4; k += kPcgThreads)
-          reinterpret_cast<float4*>(scratch)[k] = __ldcg(reinterpret_cast<const float4*>(a.c.rc) + k);
-        __syncthreads();
+        if (!merged) {
+          for (int k = tid; k < ld / 4; k += kPcgThreads)
+            reinterpret_cast<float4*>(scratch)[k] = __ldcg(reinterpret_cast<const float4*>(a.c.rc) + k);
+          __syncthreads();
+        }  // (merged: the stopping test's sum had the barrier)
         for (int row = g * kWarps + warp; row < nd; row += G * kWarps) {
           float s = 0.f;
           if (a.c.Afull16) {
@@ -866,7 +1036,10 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_kernel(const __grid_consta
           }
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-          if (lane == 0) a.c.yc[row] = s;
+          if (lane == 0) {
+            a.c.yc[row] = s;
+            lrc += (double)s * scratch[row];
+          }
         }
       } else {
         // this CTA's tiles, 4 KB parts from the warps' rings; outputs staged
@@ -934,71 +1107,16 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_kernel(const __grid_consta
         }
         for (int k = tid; k < 16 * nl; k += kPcgThreads)
           reinterpret_cast<float4*>(a.t.ypart + 64 * (size_t)b0)[k] = reinterpret_cast<const float4*>(s_y)[k];
-      }
-      // the first row's operands that do not wait for y_c, in flight under the barrier
-      const int nd0 = row0 + tid;
-      float4 drv, ddv, dov, dlt;
-      uint4 dcw;
-      if (nd0 < row1) {
-        drv = r4[nd0];
-        ddv = d4[nd0];
-        dov = o4 ? o4[nd0] : make_float4(0.f, 0.f, 0.f, 0.f);
-        dlt = __ldg(a.c.node_lat + nd0);
-        dcw = a.t.row_corners[nd0];
-      }
-      if (!grid_barrier(a.bar, ++epoch)) break;
-      // ── D: z = S r + P y_c, r.z ──
-      float* s_yc = scratch;  // [max_loc][3] y_c of the coarse nodes these rows use
-      if (a.c.full_ld) {
-        const int* loc = tab + tab[TAB_LOC];
-        for (int k = tid; k < 3 * tab[TAB_NLOC]; k += kPcgThreads) s_yc[k] = __ldcg(a.c.yc + 3 * loc[k / 3] + k % 3);
-      } else {
-        const int *yidx = tab + tab[TAB_YIDX], *yptr = tab + tab[TAB_YPTR], *ylist = tab + tab[TAB_YLIST];
-        for (int k = tid; k < 3 * tab[TAB_NLOC]; k += kPcgThreads) {
-          const int id = yidx[k], j1 = yptr[(id >> 6) + 1];
-          float s = 0.f;
-          constexpr int kU = 12;
-          for (int j = yptr[id >> 6]; j < j1; j += kU) {
-            float v[kU];
-#pragma unroll
-            for (int u = 0; u < kU; ++u)
-              v[u] = j + u < j1 ? __ldcg(a.t.ypart + 64 * (size_t)ylist[j + u] + (id & 63)) : 0.f;
-#pragma unroll
-            for (int u = 0; u < kU; ++u) s += v[u];
-          }
-          s_yc[k] = s;
+        // (BF16: the three parts add up to r_c exactly)
+        for (int k = tid; k < 64 * nl; k += kPcgThreads) {
+          const __nv_bfloat16* x3 = s_x3 + 192 * (k >> 6) + (k & 63);
+          const float x = a.c.Ainv16 ? __bfloat162float(x3[0]) + (__bfloat162float(x3[64]) + __bfloat162float(x3[128]))
+                                     : s_x[k];
+          lrc += (double)x * s_y[k];
         }
       }
-      __syncthreads();
-      for (int n = nd0; n < row1; n += kPcgThreads) {
-        if (n != nd0) {
-          drv = r4[n];
-          ddv = d4[n];
-          if (o4) dov = o4[n];
-          dlt = __ldg(a.c.node_lat + n);
-          dcw = a.t.row_corners[n];
-        }
-        const float4 rv = drv;
-        const uint32_t cpk[4] = {dcw.x, dcw.y, dcw.z, dcw.w};
-        const float t[3] = {dlt.x, dlt.y, dlt.z};
-        float cz[3] = {0.f, 0.f, 0.f};
-        const float sm[3] = {ddv.x * rv.x + dov.x * rv.y + dov.y * rv.z, ddv.y * rv.y + dov.x * rv.x + dov.z * rv.z,
-                             ddv.z * rv.z + dov.y * rv.x + dov.z * rv.y};
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float* y = s_yc + 3 * ((cpk[k >> 1] >> (16 * (k & 1))) & 0xffffu);
-          const float w = tri_weight(t[0], t[1], t[2], k);
-          cz[0] += w * y[0];
-          cz[1] += w * y[1];
-          cz[2] += w * y[2];
-        }
-        const int fx = (int)a.m.fixed[n];
-        const float4 zv = make_float4((fx & 1) ? 0.f : sm[0] + cz[0], (fx & 2) ? 0.f : sm[1] + cz[1],
-                                      (fx & 4) ? 0.f : sm[2] + cz[2], 0.f);
-        z4[n] = zv;
-        lrz += (double)rv.x * zv.x + (double)rv.y * zv.y + (double)rv.z * zv.z;
-      }
-      post(part_d, lrz, sred[0]);
+      post(part_e, lrc, sred[0]);
+      col_load(tid, p4, init);
       if (!grid_barrier(a.bar, ++epoch)) break;
     }
     first = init;
@@ -1006,7 +1124,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_kernel(const __grid_consta
   // copies still in flight land before the CTA's shared memory goes away
   if (any)
     for (int k = 0; k < ns; ++k) take();
-  if (!loaded) bulk::wait(bar + 2, 0u);
+  if (total > 0) bulk::wait(bar + 2, 0u);
   if (g == 0 && tid == 0) {
     CGState* st = a.cg;
     st->rz = rz;
@@ -1039,7 +1157,9 @@ bool pcg_plan(PcgArgs& a, bool two_level, const std::vector<int>& prefix, size_t
   a.items_off = (uint32_t)tab;
   tab += sizeof(uint2) * kWarps * (size_t)a.max_items;
   size_t base = sizeof(float) * 3 * (size_t)a.as.max_cols;
-  if (two_level) base = std::max(base, sizeof(float) * std::max(3 * (size_t)a.t.max_loc, (size_t)a.c.full_ld));
+  if (two_level) base += sizeof(float) * 4 * (size_t)a.t.max_loc;
+  base += sizeof(float) * 96 * kWarps;  // few slices: the warps' parts
+  if (two_level) base = std::max(base, sizeof(float) * (size_t)a.c.full_ld);
   const int nsl = a.as.max_slices;
   // the coarse tiles staged at once: all of the CTA's, or as many as fit
   for (int batch = tiles ? (a.t.max_tiles + kWarps - 1) / kWarps * kWarps : 0;; batch -= kWarps) {
