@@ -31,6 +31,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <mutex>
 #include <thread>
 
 #include "fem_asm.h"
@@ -43,7 +44,7 @@ namespace {
 
 // f(begin, end) over [0, n) on up to 16 host threads, `grain` or more each
 template <typename F>
-void parallel_ranges(int n, F f, int grain = 4096) {
+void parallel_ranges(int n, F f, int grain = 1024) {
   const int hw = std::max(1, (int)std::thread::hardware_concurrency());
   const int nt = std::max(1, std::min(std::min(hw, 16), n / grain));
   std::vector<std::thread> pool;
@@ -70,29 +71,37 @@ bool build_asm_host(const int4* conn4, int Nn, int Ne, int npe, int sms, AsmHost
   // neighbours of each node (ascending), edges to higher nodes and the
   // (element, vertex pair) lists of those edges: count, then fill
   std::vector<int64_t> nrow(Nn + 1, 0), erow(Nn + 1, 0), lrow(Nn + 1, 0);
-  auto neighbours = [&](int a, std::vector<int>& nb) {
-    nb.clear();
-    for (int j = arow[a]; j < arow[a + 1]; ++j) {
-      const int* cn = conn + (size_t)npe * (acol[j] / npe);
-      for (int k = 0; k < npe; ++k)
-        if (cn[k] != a) nb.push_back(cn[k]);
-    }
-    std::sort(nb.begin(), nb.end());
-    nb.erase(std::unique(nb.begin(), nb.end()), nb.end());
+  struct Part {
+    int a0;
+    std::vector<int> cols;
   };
+  std::vector<Part> found;  // the neighbours, by the threads' runs of nodes
+  std::mutex mu;
   parallel_ranges(Nn, [&](int a0, int a1) {
-    std::vector<int> nb;
+    Part p{a0, {}};
+    p.cols.reserve((size_t)(a1 - a0) * (npe == 8 ? 27 : 15));
+    // (rows are short: scanning the ones found so far beats sorting all repeats)
     for (int a = a0; a < a1; ++a) {
-      neighbours(a, nb);
-      nrow[a + 1] = (int64_t)nb.size();
-      erow[a + 1] = nb.end() - std::upper_bound(nb.begin(), nb.end(), a);
+      const size_t base = p.cols.size();
       int64_t l = 0;
       for (int j = arow[a]; j < arow[a + 1]; ++j) {
         const int* cn = conn + (size_t)npe * (acol[j] / npe);
-        for (int k = 0; k < npe; ++k) l += cn[k] > a;
+        for (int k = 0; k < npe; ++k) {
+          const int b = cn[k];
+          if (b == a) continue;
+          l += b > a;
+          size_t q = base;
+          while (q < p.cols.size() && p.cols[q] != b) ++q;
+          if (q == p.cols.size()) p.cols.push_back(b);
+        }
       }
+      std::sort(p.cols.begin() + base, p.cols.end());
+      nrow[a + 1] = (int64_t)(p.cols.size() - base);
+      erow[a + 1] = p.cols.end() - std::upper_bound(p.cols.begin() + base, p.cols.end(), a);
       lrow[a + 1] = l;
     }
+    std::lock_guard<std::mutex> lock(mu);
+    found.push_back(std::move(p));
   });
   for (int a = 0; a < Nn; ++a) {
     nrow[a + 1] += nrow[a];
@@ -103,13 +112,10 @@ bool build_asm_host(const int4* conn4, int Nn, int Ne, int npe, int sms, AsmHost
   if (nnz > 0x7fffffffLL || lrow[Nn] > 0x7fffffffLL || (uint64_t)Ne * npe * npe > 0xffffffffULL) return false;
   out->cols.resize((size_t)nnz);
   out->row.assign(nrow.begin(), nrow.end());
-  parallel_ranges(Nn, [&](int a0, int a1) {
-    std::vector<int> nb;
-    for (int a = a0; a < a1; ++a) {
-      neighbours(a, nb);
-      std::copy(nb.begin(), nb.end(), out->cols.begin() + nrow[a]);
-    }
-  });
+  parallel_ranges((int)found.size(), [&](int p0, int p1) {
+    for (int p = p0; p < p1; ++p)
+      std::copy(found[p].cols.begin(), found[p].cols.end(), out->cols.begin() + nrow[found[p].a0]);
+  }, 1);
   // runs of rows with equal entries (a row counts as 4 more) per CTA
   const int G = std::max(1, std::min(sms, Nn / kAsmMinRows));
   out->grid = G;
@@ -179,20 +185,9 @@ bool build_asm_host(const int4* conn4, int Nn, int Ne, int npe, int sms, AsmHost
     for (int k = 0; k <= out->max_slices; ++k)
       out->prefix[k] = std::max(out->prefix[k], csteps[g][std::min(k, (int)csteps[g].size() - 1)]);
   // slots
-  out->entry.resize((size_t)steps * 32);
   out->edges.resize((size_t)erow[Nn]);
   out->eptr.resize((size_t)erow[Nn] + 1);
   out->list.resize((size_t)lrow[Nn]);
-  const int ns = (int)out->slice_step.size() - 1;
-  parallel_ranges(ns, [&](int s0, int s1) {
-    for (int s = s0; s < s1; ++s)
-      for (int l = 0; l < 32; ++l) {
-        const int r = out->slice_rows[32 * (size_t)s + l];
-        const int deg = r >= 0 ? (int)(nrow[r + 1] - nrow[r]) : 0;
-        for (int k = 0; k < out->slice_step[s + 1] - out->slice_step[s]; ++k)
-          out->entry[((size_t)out->slice_step[s] + k) * 32 + l] = make_int2(r, k < deg ? out->cols[nrow[r] + k] : -1);
-      }
-  }, 64);
   parallel_ranges(Nn, [&](int a0, int a1) {
     std::vector<int> cnt;
     for (int a = a0; a < a1; ++a) {
@@ -229,19 +224,19 @@ bool build_asm_host(const int4* conn4, int Nn, int Ne, int npe, int sms, AsmHost
   return true;
 }
 
-// Local columns of the steps; one CTA per CTA of the solve.
-__global__ void __launch_bounds__(256) asm_fill_kernel(const __grid_constant__ AsmDev S, const int2* entry) {
-  const int g = blockIdx.x, r0 = S.cta_row[g], r1 = S.cta_row[g + 1];
+// Local columns of the steps; one CTA per CTA of the solve, a warp per slice.
+__global__ void __launch_bounds__(512) asm_fill_kernel(const __grid_constant__ AsmDev S, const int* row, const int* cols) {
+  const int g = blockIdx.x, lane = threadIdx.x & 31, r0 = S.cta_row[g], r1 = S.cta_row[g + 1];
   const int* halo = S.halo + S.halo_ptr[g];
   const int nh = S.halo_ptr[g + 1] - S.halo_ptr[g];
-  const int64_t i0 = 32 * (int64_t)S.slice_step[S.cta_slice[g]], i1 = 32 * (int64_t)S.slice_step[S.cta_slice[g + 1]];
-  for (int64_t i = i0 + threadIdx.x; i < i1; i += 256) {
-    const int2 en = entry[i];
-    int l = 0;
-    if (en.x >= 0) {
-      const int n = en.y >= 0 ? en.y : en.x;
-      l = n - r0;
-      if (n < r0 || n >= r1) {
+  for (int s = S.cta_slice[g] + ((int)threadIdx.x >> 5); s < S.cta_slice[g + 1]; s += 16) {
+    const int r = S.slice_rows[32 * (size_t)s + lane];
+    const int j0 = r >= 0 ? row[r] : 0, deg = r >= 0 ? row[r + 1] - j0 : 0;
+    const int t0 = S.slice_step[s], t1 = S.slice_step[s + 1];
+    for (int t = t0; t < t1; ++t) {
+      const int n = t - t0 < deg ? cols[j0 + t - t0] : r;  // padding: the row itself
+      int l = n < 0 ? 0 : n - r0;
+      if (n >= 0 && (n < r0 || n >= r1)) {
         int lo = 0, hi = nh;
         while (lo < hi) {
           const int mid = (lo + hi) >> 1;
@@ -252,25 +247,12 @@ __global__ void __launch_bounds__(256) asm_fill_kernel(const __grid_constant__ A
         }
         l = r1 - r0 + lo;
       }
+      reinterpret_cast<uint16_t*>(S.words + (size_t)t * kAsmStepWords)[lane] = (uint16_t)l;
     }
-    reinterpret_cast<uint16_t*>(S.words + (size_t)(i >> 5) * kAsmStepWords)[i & 31] = (uint16_t)l;
   }
 }
 
 // ───────────────────────── assembly ─────────────────────────
-
-// One block into its slot, rows of fixed DOFs (bits of fx) as zeros.
-__device__ __forceinline__ void asm_store(const AsmDev& S, uint32_t slot, float k00, float k01, float k02, float k10,
-                                          float k11, float k12, float k20, float k21, float k22, int fx) {
-  uint32_t* w = S.words + (size_t)(slot >> 5) * kAsmStepWords;
-  const int lane = (int)(slot & 31u);
-  if (fx & 1) k00 = k01 = k02 = 0.f;
-  if (fx & 2) k10 = k11 = k12 = 0.f;
-  if (fx & 4) k20 = k21 = k22 = 0.f;
-  reinterpret_cast<float4*>(w + 16)[lane] = make_float4(k00, k01, k02, k10);
-  reinterpret_cast<float4*>(w + 144)[lane] = make_float4(k11, k12, k20, k21);
-  reinterpret_cast<float*>(w + 272)[lane] = k22;
-}
 
 // One thread per edge (a, b), a < b: K_ab summed over the elements on the
 // edge in ascending element order, and K_ba = K_ab^T.  Column i of an
@@ -367,11 +349,15 @@ __global__ void __launch_bounds__(128) asm_diag_kernel(const __grid_constant__ A
 
 // ───────────────────────── launchers ─────────────────────────
 
-void launch_asm_fill(const AsmDev& S, const int2* entry, cudaStream_t s) {
-  asm_fill_kernel<<<S.grid, 256, 0, s>>>(S, entry);
+void launch_asm_fill(const AsmDev& S, const int* row, const int* cols, cudaStream_t s) {
+  asm_fill_kernel<<<S.grid, 512, 0, s>>>(S, row, cols);
 }
 
 void launch_asm(const AsmArgs& a, int model, cudaStream_t s) {
+  if (a.m.npe == 8) {
+    launch_asm_hex(a, model, s);
+    return;
+  }
   const int g = (a.s.n_edges + 127) / 128;
   switch (model) {
     case M_LE: asm_edge_kernel<M_LE><<<g, 128, 0, s>>>(a); break;

@@ -13,7 +13,6 @@ constexpr int kAsmMinRows = 64;
 struct AsmHost {
   std::vector<int> cols;           // neighbours of each node, ascending (CSR with row)
   std::vector<int> row;
-  std::vector<int2> entry;         // per slot of a step (step * 32 + lane): node, column (-1: padding)
   std::vector<uint2> edges;        // slots of (a, b) and (b, a) of each edge a < b
   std::vector<uint32_t> eptr;      // [edges + 1] into list
   std::vector<uint32_t> list;      // (element * npe + vertex a) * npe + vertex b, per edge
@@ -38,10 +37,28 @@ struct AsmArgs {
   const float* payload;
 };
 
-// local columns of every slot (row: CTA of each node's row; cols: the slots' columns, -1: padding)
-void launch_asm_fill(const AsmDev& S, const int2* entry, cudaStream_t s);
+// One block into its slot, rows of fixed DOFs (bits of fx) as zeros.
+static __device__ __forceinline__ void asm_store(const AsmDev& S, uint32_t slot, float k00, float k01, float k02, float k10,
+                                          float k11, float k12, float k20, float k21, float k22, int fx) {
+  uint32_t* w = S.words + (size_t)(slot >> 5) * kAsmStepWords;
+  const int lane = (int)(slot & 31u);
+  if (fx & 1) k00 = k01 = k02 = 0.f;
+  if (fx & 2) k10 = k11 = k12 = 0.f;
+  if (fx & 4) k20 = k21 = k22 = 0.f;
+  reinterpret_cast<float4*>(w + 16)[lane] = make_float4(k00, k01, k02, k10);
+  reinterpret_cast<float4*>(w + 144)[lane] = make_float4(k11, k12, k20, k21);
+  reinterpret_cast<float*>(w + 272)[lane] = k22;
+}
+
+// local columns of every slot of the steps, from the neighbour lists
+void launch_asm_fill(const AsmDev& S, const int* row, const int* cols, cudaStream_t s);
 // values at the tangent state of `payload`
 void launch_asm(const AsmArgs& a, int model, cudaStream_t s);
+// HEX8: places of the elements' blocks in s.list (hpos, [32 Ne], preset to
+// kNoPlace), and the two assembly kernels (fem_hex8.cu)
+constexpr uint32_t kNoPlace = 0xffffffffu;
+void launch_asm_hex_places(const uint32_t* list, size_t n, uint32_t* hpos, cudaStream_t s);
+void launch_asm_hex(const AsmArgs& a, int model, cudaStream_t s);
 // dinv (and boff: nodal 3 x 3 block inverse) from the assembled blocks
 void launch_asm_diag(const AsmArgs& a, float* dinv, float* boff, cudaStream_t s);
 

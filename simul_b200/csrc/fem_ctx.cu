@@ -914,7 +914,7 @@ MvArgs make_mv(const FemCtx* c) {
   mv.m = c->mesh();
   // the assembled product runs in the persistent PCG kernel only: a single
   // product with a new tangent is cheaper by elements than with an assembly
-  mv.variant = c->mv_variant == MV_ASSEMBLED ? MV_PERSIST : c->mv_variant;
+  mv.variant = c->mv_variant != MV_ASSEMBLED ? c->mv_variant : (c->npe == 8 ? MV_TWO_PHASE : MV_PERSIST);
   mv.stage = c->stage;
   mv.eb = c->ebdev;
   mv.wa = c->wadev;
@@ -965,6 +965,18 @@ int ensure_asm_tables(FemCtx* c) {
       (st = up(&slice_rows, h.slice_rows)) || (st = up(&halo_ptr, h.halo_ptr)) || (st = up(&halo, h.halo)) ||
       (st = up(&edges, h.edges)) || (st = up(&eptr, h.eptr)) || (st = up(&list, h.list)))
     return st;
+  if (c->npe == 8) {
+    const size_t n = h.list.size();
+    uint32_t* hpos = nullptr;
+    if ((st = asm_upload(c, &hpos, (const uint32_t*)nullptr, 32 * (size_t)c->Ne)) ||
+        (st = asm_upload(c, &S.hblk4, (const float4*)nullptr, 2 * n)) ||
+        (st = asm_upload(c, &S.hblk1, (const float*)nullptr, n)))
+      return st;
+    CK(cudaMemsetAsync(hpos, 0xff, 32 * sizeof(uint32_t) * (size_t)c->Ne, c->stream));  // kNoPlace
+    launch_asm_hex_places(list, n, hpos, c->stream);
+    CKL();
+    S.hpos = hpos;
+  }
   if ((st = asm_upload(c, &words, (const uint32_t*)nullptr, (size_t)h.slice_step.back() * kAsmStepWords))) return st;
   if ((st = asm_upload(c, &c->pcg_part, (const double*)nullptr, 4 * (size_t)h.grid))) return st;
   if ((st = asm_upload(c, &c->pcg_bar, (const unsigned int*)nullptr, (size_t)1))) return st;
@@ -988,15 +1000,18 @@ int ensure_asm_tables(FemCtx* c) {
   S.halo = halo;
   c->asm_cta_row = h.cta_row;
   c->asm_prefix = h.prefix;
-  int2* entry = nullptr;
-  CK(cudaMalloc(reinterpret_cast<void**>(&entry), std::max<size_t>(h.entry.size(), 1) * sizeof(int2)));
-  cudaError_t e = cudaMemcpyAsync(entry, h.entry.data(), h.entry.size() * sizeof(int2), cudaMemcpyHostToDevice, c->stream);
+  int* lists = nullptr;  // the neighbour lists, for the fill only
+  const size_t nr = h.row.size(), nc = h.cols.size();
+  CK(cudaMalloc(reinterpret_cast<void**>(&lists), (nr + nc) * sizeof(int)));
+  cudaError_t e = cudaMemcpyAsync(lists, h.row.data(), nr * sizeof(int), cudaMemcpyHostToDevice, c->stream);
+  if (e == cudaSuccess && nc)
+    e = cudaMemcpyAsync(lists + nr, h.cols.data(), nc * sizeof(int), cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) {
-    launch_asm_fill(S, entry, c->stream);
+    launch_asm_fill(S, lists, lists + nr, c->stream);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);  // the host tables go out of scope
-  cudaFree(entry);
+  cudaFree(lists);
   CK(e);
   c->asm_built = true;
   c->asm_valid = false;
@@ -1007,7 +1022,7 @@ int ensure_asm_tables(FemCtx* c) {
 int ensure_assembled(FemCtx* c) {
   if (c->asm_valid) return FEM_OK;
   launch_asm(asm_args(c), c->model_kind, c->stream);
-  ++c->n_launches;
+  c->n_launches += c->npe == 8 ? 2 : 1;
   CKL();
   c->asm_valid = true;
   return FEM_OK;
@@ -1195,12 +1210,12 @@ CGState endless_cg() {
 // they run inside CG (3 warm-up + 10 timed launches each, p = 1 on free
 // DOFs).  The CG state is reset by cg_init afterwards.
 int choose_matvec_variant(FemCtx* c, bool plain) {
-  if (c->npe == 8) {
-    // HEX8 has the two-phase pass only
+  int st;
+  if (c->npe == 8 && c->mv_forced != kMvRule) {
+    // of the element passes HEX8 has the two-phase one only
     c->mv_variant = MV_TWO_PHASE;
     return FEM_OK;
   }
-  int st;
   if (c->mv_forced >= 0) {
     c->mv_variant = c->mv_forced;
     if (c->mv_variant == MV_ELEM_BLOCK && c->eb_size == 0)
@@ -1213,7 +1228,7 @@ int choose_matvec_variant(FemCtx* c, bool plain) {
     // persistent kernel at a time took 196 ms where eight chains take 150)
     plain = plain && !c->chain_forced && c->pcg_ok && !c->in_batch;
     if (plain && (st = ensure_asm_tables(c))) return st;
-    c->mv_variant = plain && c->asm_built ? MV_ASSEMBLED : MV_PERSIST;
+    c->mv_variant = plain && c->asm_built ? MV_ASSEMBLED : (c->npe == 8 ? MV_TWO_PHASE : MV_PERSIST);
     return FEM_OK;
   }
   if (c->mv_tuned && c->mv_tuned_model == c->model_kind) return FEM_OK;

@@ -16,6 +16,7 @@
 // which keeps the FP32 tangent's Jacobian free of the absolute position.
 #include <cuda_runtime.h>
 
+#include "fem_asm.h"
 #include "fem_internal.h"
 #include "fem_lattice.cuh"
 #include "fem_reduce.cuh"
@@ -430,6 +431,133 @@ __global__ void __launch_bounds__(128, 5) hex_mv_elem_kernel(const __grid_consta
     hex_mv_one<MODEL, CG, false>(a, e);
 }
 
+// ───────────────────────── assembled tangent (FP32) ─────────────────────────
+//
+// An element has 28 vertex pairs.  Eight lanes per element: lane b forms the
+// columns of vertex b, K_ab = sum over the points of vol dN_a . dP[e_i x dN_b],
+// for a = b + 1, b + 2, b + 3 and, where b < 4, b + 4 (mod 8), which covers each
+// pair once.  Each block goes to the pair's place in the edges' element list
+// (transposed where the list has the pair the other way round), and a second
+// kernel adds an edge's blocks in that order.  One thread per edge with its
+// elements in turn, as for TET4, would evaluate each point's geometry 28 times
+// (200 us at 48,000 elements by its operations).
+
+__global__ void __launch_bounds__(256) hex_asm_places_kernel(const uint32_t* list, size_t n, uint32_t* hpos) {
+  const size_t l = (size_t)blockIdx.x * 256 + threadIdx.x;
+  if (l >= n) return;
+  const uint32_t en = list[l];
+  const int la = (int)(en >> 3) & 7, lb = (int)en & 7, d = (la - lb) & 7;
+  const bool turn = d > 4 || (d == 4 && lb >= 4);
+  const int b = turn ? la : lb, t = (turn ? (8 - d) : d) - 1;
+  hpos[32 * (size_t)(en >> 6) + 4 * b + t] = (uint32_t)(2 * l) | (turn ? 1u : 0u);
+}
+
+template <int MODEL>
+__global__ void __launch_bounds__(128) hex_asm_elem_kernel(const __grid_constant__ AsmArgs a) {
+  constexpr unsigned kFull = 0xffffffffu;
+  const MeshDev& m = a.m;
+  const size_t t0 = (size_t)blockIdx.x * 128 + threadIdx.x;
+  const int b = (int)threadIdx.x & 7, base = (int)threadIdx.x & 24;
+  const bool act = (t0 >> 3) < (size_t)m.n_elems;
+  const int e = act ? (int)(t0 >> 3) : m.n_elems - 1;  // (spare lanes take part in the shuffles)
+  const size_t Ne = (size_t)m.n_elems, Nq = kHexGauss * Ne;
+  float cx[7][3];
+  {
+    const float4 X = __ldg(m.X32 + __ldg(reinterpret_cast<const int*>(m.conn) + 8 * (size_t)e + b));
+    float xr[8][3];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      xr[k][0] = __shfl_sync(kFull, X.x, base + k);
+      xr[k][1] = __shfl_sync(kFull, X.y, base + k);
+      xr[k][2] = __shfl_sync(kFull, X.z, base + k);
+    }
+#pragma unroll
+    for (int k = 7; k >= 0; --k)
+#pragma unroll
+      for (int d = 0; d < 3; ++d) xr[k][d] -= xr[0][d];
+    hex_coeffs(xr, cx);
+  }
+  const DevMat<float>& mat = a.matF[__ldg(m.mat_id + e)];
+  const float scale = __ldg(m.scale + e);
+  const int npay = model_pay_words(MODEL >= 0 ? MODEL : mat.model);
+  const float s0 = (float)hex_sign(b, 0), s1 = (float)hex_sign(b, 1), s2 = (float)hex_sign(b, 2);
+  float K[4][9];
+#pragma unroll
+  for (int t = 0; t < 4; ++t)
+#pragma unroll
+    for (int k = 0; k < 9; ++k) K[t][k] = 0.f;
+#pragma unroll 1
+  for (int g = 0; g < kHexGauss; ++g) {
+    const size_t q = (size_t)g * Ne + e;
+    float pay[kPay];
+#pragma unroll
+    for (int k = 0; k < kPay; ++k) pay[k] = (k < npay) ? __ldg(a.payload + (size_t)k * Nq + q) : 0.f;
+    const float gx = (float)hex_sign(g, 0) * (float)kGaussHex;
+    const float gy = (float)hex_sign(g, 1) * (float)kGaussHex;
+    const float gz = (float)hex_sign(g, 2) * (float)kGaussHex;
+    float J[3][3], Ji[3][3], vol;
+    hex_nat_grad(cx, gx, gy, gz, J);
+    hex_inv(J, Ji, vol);
+    const float u0 = 1.f + s0 * gx, u1 = 1.f + s1 * gy, u2 = 1.f + s2 * gz;
+    const float d0 = 0.125f * s0 * u1 * u2, d1 = 0.125f * s1 * u0 * u2, d2 = 0.125f * s2 * u0 * u1;
+    float nb[3], na[4][3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) nb[k] = d0 * Ji[0][k] + d1 * Ji[1][k] + d2 * Ji[2][k];
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) na[t][k] = vol * __shfl_sync(kFull, nb[k], base + ((b + 1 + t) & 7));
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      float dF[9], dP[9];
+#pragma unroll
+      for (int k = 0; k < 9; ++k) dF[k] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) dF[3 * i + j] = nb[j];
+      dP_any<MODEL>(mat, scale, pay, dF, dP);
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+          K[t][3 * r + i] += dP[3 * r] * na[t][0] + dP[3 * r + 1] * na[t][1] + dP[3 * r + 2] * na[t][2];
+    }
+  }
+  if (!act) return;
+  const uint4 hp = __ldg(reinterpret_cast<const uint4*>(a.s.hpos) + 8 * (size_t)e + b);
+  const uint32_t place[4] = {hp.x, hp.y, hp.z, hp.w};
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    if (place[t] == kNoPlace) continue;
+    const bool turn = place[t] & 1u;
+    const size_t l = place[t] >> 1;
+    const float* k = K[t];
+    __stcg(a.s.hblk4 + 2 * l, make_float4(k[0], turn ? k[3] : k[1], turn ? k[6] : k[2], turn ? k[1] : k[3]));
+    __stcg(a.s.hblk4 + 2 * l + 1, make_float4(k[4], turn ? k[7] : k[5], turn ? k[2] : k[6], turn ? k[5] : k[7]));
+    __stcg(a.s.hblk1 + l, k[8]);
+  }
+}
+
+// One thread per edge: its elements' blocks (contiguous), to both slots.
+__global__ void __launch_bounds__(128) hex_asm_edge_kernel(const __grid_constant__ AsmArgs a) {
+  const int t = blockIdx.x * 128 + threadIdx.x;
+  if (t >= a.s.n_edges) return;
+  const uint2 ed = __ldg(a.s.edges + t);
+  const uint32_t l0 = __ldg(a.s.eptr + t), l1 = __ldg(a.s.eptr + t + 1);
+  const uint32_t en = __ldg(a.s.list + l0);
+  const int* cn = reinterpret_cast<const int*>(a.m.conn) + 8 * (size_t)(en >> 6);
+  const int na = __ldg(cn + ((en >> 3) & 7u)), nb = __ldg(cn + (en & 7u));
+  float4 A = make_float4(0.f, 0.f, 0.f, 0.f), B = A;
+  float C = 0.f;
+  for (uint32_t l = l0; l < l1; ++l) {
+    const float4 x = __ldcg(a.s.hblk4 + 2 * (size_t)l), y = __ldcg(a.s.hblk4 + 2 * (size_t)l + 1);
+    C += __ldcg(a.s.hblk1 + l);
+    A.x += x.x; A.y += x.y; A.z += x.z; A.w += x.w;
+    B.x += y.x; B.y += y.y; B.z += y.z; B.w += y.w;
+  }
+  asm_store(a.s, ed.x, A.x, A.y, A.z, A.w, B.x, B.y, B.z, B.w, C, a.m.fixed[na]);
+  asm_store(a.s, ed.y, A.x, A.w, B.z, A.y, B.x, B.w, A.z, B.y, C, a.m.fixed[nb]);
+}
+
 // ───────────────────────── Jacobi diagonal (FP32) ─────────────────────────
 
 template <int MODEL, bool BLOCK>
@@ -745,6 +873,24 @@ void launch_coarse_cells_hex(const CoarseArgs& a, int model, cudaStream_t s) {
     case M_FMR: coarse_cell_hex_kernel<M_FMR><<<g, 128, 0, s>>>(a); break;
     default: coarse_cell_hex_kernel<-1><<<g, 128, 0, s>>>(a); break;
   }
+}
+
+void launch_asm_hex_places(const uint32_t* list, size_t n, uint32_t* hpos, cudaStream_t s) {
+  if (n) hex_asm_places_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(list, n, hpos);
+}
+
+void launch_asm_hex(const AsmArgs& a, int model, cudaStream_t s) {
+  const unsigned g = (unsigned)((8 * (size_t)a.m.n_elems + 127) / 128);
+  switch (model) {
+    case M_LE: hex_asm_elem_kernel<M_LE><<<g, 128, 0, s>>>(a); break;
+    case M_NH: hex_asm_elem_kernel<M_NH><<<g, 128, 0, s>>>(a); break;
+    case M_MR: hex_asm_elem_kernel<M_MR><<<g, 128, 0, s>>>(a); break;
+    case M_J2: hex_asm_elem_kernel<M_J2><<<g, 128, 0, s>>>(a); break;
+    case M_TI: hex_asm_elem_kernel<M_TI><<<g, 128, 0, s>>>(a); break;
+    case M_FMR: hex_asm_elem_kernel<M_FMR><<<g, 128, 0, s>>>(a); break;
+    default: hex_asm_elem_kernel<-1><<<g, 128, 0, s>>>(a); break;
+  }
+  if (a.s.n_edges) hex_asm_edge_kernel<<<nblk(a.s.n_edges, 128), 128, 0, s>>>(a);
 }
 
 template <int MODEL>

@@ -183,6 +183,9 @@ constexpr int kPcgPiece = 3;        // matrix steps per bulk copy (3.6 KB, the s
 constexpr int kPcgThreads = 512;
 
 struct AsmDev {
+  const uint32_t* hpos;   // HEX8: [Ne][8][4] place of each vertex pair's block (2 * list index | transposed)
+  float4* hblk4;          // HEX8: the elements' blocks in list order: components 0-7,
+  float* hblk1;           //   component 8
   int grid;                 // CTAs of the persistent solve
   int n_slices;
   int n_edges;
