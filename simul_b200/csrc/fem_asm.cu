@@ -32,29 +32,12 @@
 
 #include <algorithm>
 #include <mutex>
-#include <thread>
 
 #include "fem_asm.h"
 
 namespace femb200 {
 
 // ───────────────────────── tables (host) ─────────────────────────
-
-namespace {
-
-// f(begin, end) over [0, n) on up to 16 host threads, `grain` or more each
-template <typename F>
-void parallel_ranges(int n, F f, int grain = 1024) {
-  const int hw = std::max(1, (int)std::thread::hardware_concurrency());
-  const int nt = std::max(1, std::min(std::min(hw, 16), n / grain));
-  std::vector<std::thread> pool;
-  for (int t = 1; t < nt; ++t)
-    pool.emplace_back([=] { f((int)((int64_t)n * t / nt), (int)((int64_t)n * (t + 1) / nt)); });
-  f(0, (int)((int64_t)n / nt));
-  for (auto& th : pool) th.join();
-}
-
-}  // namespace
 
 bool build_asm_host(const int4* conn4, int Nn, int Ne, int npe, int sms, AsmHost* out) {
   const int* conn = &conn4[0].x;
@@ -131,7 +114,8 @@ bool build_asm_host(const int4* conn4, int Nn, int Ne, int npe, int sms, AsmHost
     for (int k = G - 1; k > 0; --k) out->cta_row[k] = std::min(out->cta_row[k], out->cta_row[k + 1] - 1);
   }
   // slices; halos
-  std::vector<uint32_t> slot0(Nn);  // slot of each row's first entry (entry k: + 32 k)
+  std::vector<uint32_t>& slot0 = out->slot0;
+  slot0.assign(Nn, 0u);
   std::vector<std::vector<int>> halo(G), order(G);
   parallel_ranges(G, [&](int g0, int g1) {
     for (int g = g0; g < g1; ++g) {
@@ -184,44 +168,48 @@ bool build_asm_host(const int4* conn4, int Nn, int Ne, int npe, int sms, AsmHost
   for (int g = 0; g < G; ++g)
     for (int k = 0; k <= out->max_slices; ++k)
       out->prefix[k] = std::max(out->prefix[k], csteps[g][std::min(k, (int)csteps[g].size() - 1)]);
-  // slots
-  out->edges.resize((size_t)erow[Nn]);
-  out->eptr.resize((size_t)erow[Nn] + 1);
-  out->list.resize((size_t)lrow[Nn]);
-  parallel_ranges(Nn, [&](int a0, int a1) {
-    std::vector<int> cnt;
-    for (int a = a0; a < a1; ++a) {
-      const int* cols = out->cols.data() + nrow[a];
-      const int deg = (int)(nrow[a + 1] - nrow[a]);
-      const int up = deg - (int)(erow[a + 1] - erow[a]);
-      cnt.assign(deg - up + 1, 0);
-      for (int j = arow[a]; j < arow[a + 1]; ++j) {
-        const int* cn = conn + (size_t)npe * (acol[j] / npe);
-        for (int k = 0; k < npe; ++k)
-          if (cn[k] > a) cnt[std::lower_bound(cols + up, cols + deg, cn[k]) - (cols + up) + 1]++;
-      }
-      for (int q = 0; q < deg - up; ++q) cnt[q + 1] += cnt[q];
-      for (int q = 0; q < deg - up; ++q) {
-        const int b = cols[up + q];
-        const int* cb = out->cols.data() + nrow[b];
-        const int db = (int)(nrow[b + 1] - nrow[b]);
-        const uint32_t back = (uint32_t)(std::lower_bound(cb, cb + db, a) - cb);
-        out->edges[erow[a] + q] = make_uint2(slot0[a] + 32u * (uint32_t)(up + q), slot0[b] + 32u * back);
-        out->eptr[erow[a] + q] = (uint32_t)(lrow[a] + cnt[q]);
-      }
-      for (int j = arow[a]; j < arow[a + 1]; ++j) {
-        const uint32_t e = acol[j] / npe, la = acol[j] % npe;
-        const int* cn = conn + (size_t)npe * e;
-        for (int k = 0; k < npe; ++k)
-          if (cn[k] > a) {
-            const int q = (int)(std::lower_bound(cols + up, cols + deg, cn[k]) - (cols + up));
-            out->list[lrow[a] + cnt[q]++] = (e * npe + la) * npe + (uint32_t)k;
-          }
-      }
-    }
-  });
-  out->eptr.back() = (uint32_t)lrow[Nn];
+  out->erow.assign(erow.begin(), erow.end());
+  out->lrow.assign(lrow.begin(), lrow.end());
   return true;
+}
+
+// Edges to higher nodes, their slots and their (element, vertex pair) lists,
+// a thread per node: the elements on the node in its slot order.  (On the host
+// this took a third of the tables' time, and its upload as long as the rest.)
+template <int SH>
+__global__ void __launch_bounds__(128) asm_list_kernel(const MeshDev m, const __grid_constant__ AsmLists t, uint2* edges,
+                                                       uint32_t* eptr, uint32_t* list) {
+  const int a = blockIdx.x * 128 + threadIdx.x;
+  if (a >= m.n_nodes) return;
+  constexpr int kN = 1 << SH;
+  const int j0 = t.row[a], deg = t.row[a + 1] - j0;
+  const uint32_t e0 = t.erow[a], ne = t.erow[a + 1] - e0;
+  uint32_t l = t.lrow[a];
+  const int up = deg - (int)ne;
+  const int base = m.blk_ptr[a / m.nb], s0 = m.node_row[a], s1 = m.node_row[a + 1];
+  for (uint32_t q = 0; q < ne; ++q) {
+    const int b = t.cols[j0 + up + (int)q];
+    int lo = t.row[b], hi = t.row[b + 1];
+    const int b0 = lo;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (t.cols[mid] < a)
+        lo = mid + 1;
+      else
+        hi = mid;
+    }
+    edges[e0 + q] = make_uint2(t.slot0[a] + 32u * (uint32_t)(up + (int)q), t.slot0[b] + 32u * (uint32_t)(lo - b0));
+    eptr[e0 + q] = l;
+    for (int j = s0; j < s1; ++j) {
+      const uint32_t code = m.node_slots[j];
+      const uint32_t e = (uint32_t)m.blk_elems[base + (int)(code >> SH)], la = code & (uint32_t)(kN - 1);
+      const int* cn = reinterpret_cast<const int*>(m.conn) + kN * (size_t)e;
+#pragma unroll
+      for (int k = 0; k < kN; ++k)
+        if (cn[k] == b) list[l++] = (e * kN + la) * kN + (uint32_t)k;
+    }
+  }
+  if (a == m.n_nodes - 1) eptr[e0 + ne] = l;
 }
 
 // Local columns of the steps; one CTA per CTA of the solve, a warp per slice.
@@ -348,6 +336,14 @@ __global__ void __launch_bounds__(128) asm_diag_kernel(const __grid_constant__ A
 }
 
 // ───────────────────────── launchers ─────────────────────────
+
+void launch_asm_lists(const MeshDev& m, const AsmLists& t, uint2* edges, uint32_t* eptr, uint32_t* list, cudaStream_t s) {
+  const int g = (m.n_nodes + 127) / 128;
+  if (m.npe == 8)
+    asm_list_kernel<3><<<g, 128, 0, s>>>(m, t, edges, eptr, list);
+  else
+    asm_list_kernel<2><<<g, 128, 0, s>>>(m, t, edges, eptr, list);
+}
 
 void launch_asm_fill(const AsmDev& S, const int* row, const int* cols, cudaStream_t s) {
   asm_fill_kernel<<<S.grid, 512, 0, s>>>(S, row, cols);

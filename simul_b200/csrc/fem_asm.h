@@ -1,6 +1,8 @@
 // Tables and launchers of the assembled tangent (fem_asm.cu).
 #pragma once
+#include <algorithm>
 #include <cstdint>
+#include <thread>
 #include <vector>
 
 #include "fem_internal.h"
@@ -10,12 +12,24 @@ namespace femb200 {
 // A CTA of the persistent solve takes at least this many rows (two warps').
 constexpr int kAsmMinRows = 64;
 
+// f(begin, end) over [0, n) on up to 16 host threads, `grain` or more each
+template <typename F>
+void parallel_ranges(int n, F f, int grain = 1024) {
+  const int hw = std::max(1, (int)std::thread::hardware_concurrency());
+  const int nt = std::max(1, std::min(std::min(hw, 16), n / grain));
+  std::vector<std::thread> pool;
+  for (int t = 1; t < nt; ++t)
+    pool.emplace_back([=] { f((int)((int64_t)n * t / nt), (int)((int64_t)n * (t + 1) / nt)); });
+  f(0, (int)((int64_t)n / nt));
+  for (auto& th : pool) th.join();
+}
+
 struct AsmHost {
   std::vector<int> cols;           // neighbours of each node, ascending (CSR with row)
   std::vector<int> row;
-  std::vector<uint2> edges;        // slots of (a, b) and (b, a) of each edge a < b
-  std::vector<uint32_t> eptr;      // [edges + 1] into list
-  std::vector<uint32_t> list;      // (element * npe + vertex a) * npe + vertex b, per edge
+  std::vector<uint32_t> erow;      // [Nn + 1] edges to higher nodes before each node
+  std::vector<uint32_t> lrow;      // [Nn + 1] (element, vertex pair) entries before each node's edges
+  std::vector<uint32_t> slot0;     // slot (step * 32 + lane) of each row's first entry (entry k: + 32 k)
   int grid = 0;
   std::vector<int> cta_row;        // [grid + 1] first row of each CTA
   std::vector<int> cta_slice;      // [grid + 1]
@@ -50,6 +64,14 @@ static __device__ __forceinline__ void asm_store(const AsmDev& S, uint32_t slot,
   reinterpret_cast<float*>(w + 272)[lane] = k22;
 }
 
+// AsmHost's lists on the device
+struct AsmLists {
+  const int *row, *cols;
+  const uint32_t *erow, *lrow, *slot0;
+};
+// the edges' slots, and per edge the elements on it as (element * npe +
+// vertex a) * npe + vertex b
+void launch_asm_lists(const MeshDev& m, const AsmLists& t, uint2* edges, uint32_t* eptr, uint32_t* list, cudaStream_t s);
 // local columns of every slot of the steps, from the neighbour lists
 void launch_asm_fill(const AsmDev& S, const int* row, const int* cols, cudaStream_t s);
 // values at the tangent state of `payload`

@@ -962,28 +962,20 @@ int ensure_asm_tables(FemCtx* c) {
   uint2* edges = nullptr;
   uint32_t *eptr = nullptr, *list = nullptr;
   if ((st = up(&cta_row, h.cta_row)) || (st = up(&cta_slice, h.cta_slice)) || (st = up(&slice_step, h.slice_step)) ||
-      (st = up(&slice_rows, h.slice_rows)) || (st = up(&halo_ptr, h.halo_ptr)) || (st = up(&halo, h.halo)) ||
-      (st = up(&edges, h.edges)) || (st = up(&eptr, h.eptr)) || (st = up(&list, h.list)))
+      (st = up(&slice_rows, h.slice_rows)) || (st = up(&halo_ptr, h.halo_ptr)) || (st = up(&halo, h.halo)))
     return st;
-  if (c->npe == 8) {
-    const size_t n = h.list.size();
-    uint32_t* hpos = nullptr;
-    if ((st = asm_upload(c, &hpos, (const uint32_t*)nullptr, 32 * (size_t)c->Ne)) ||
-        (st = asm_upload(c, &S.hblk4, (const float4*)nullptr, 2 * n)) ||
-        (st = asm_upload(c, &S.hblk1, (const float*)nullptr, n)))
-      return st;
-    CK(cudaMemsetAsync(hpos, 0xff, 32 * sizeof(uint32_t) * (size_t)c->Ne, c->stream));  // kNoPlace
-    launch_asm_hex_places(list, n, hpos, c->stream);
-    CKL();
-    S.hpos = hpos;
-  }
+  const size_t n_edges = h.erow.back(), n_list = h.lrow.back();
+  if ((st = asm_upload(c, &edges, (const uint2*)nullptr, n_edges)) ||
+      (st = asm_upload(c, &eptr, (const uint32_t*)nullptr, n_edges + 1)) ||
+      (st = asm_upload(c, &list, (const uint32_t*)nullptr, n_list)))
+    return st;
   if ((st = asm_upload(c, &words, (const uint32_t*)nullptr, (size_t)h.slice_step.back() * kAsmStepWords))) return st;
   if ((st = asm_upload(c, &c->pcg_part, (const double*)nullptr, 4 * (size_t)h.grid))) return st;
   if ((st = asm_upload(c, &c->pcg_bar, (const unsigned int*)nullptr, (size_t)1))) return st;
   if ((st = asm_upload(c, &c->pcg_p2, (const float*)nullptr, 4 * (size_t)c->Nn))) return st;
   S.grid = h.grid;
   S.n_slices = (int)h.slice_step.size() - 1;
-  S.n_edges = (int)h.edges.size();
+  S.n_edges = (int)n_edges;
   S.max_slices = h.max_slices;
   S.max_halo = h.max_halo;
   S.max_cols = (h.max_cols + 3) & ~3;  // (float4 arrays follow the planes)
@@ -1000,19 +992,43 @@ int ensure_asm_tables(FemCtx* c) {
   S.halo = halo;
   c->asm_cta_row = h.cta_row;
   c->asm_prefix = h.prefix;
-  int* lists = nullptr;  // the neighbour lists, for the fill only
-  const size_t nr = h.row.size(), nc = h.cols.size();
-  CK(cudaMalloc(reinterpret_cast<void**>(&lists), (nr + nc) * sizeof(int)));
-  cudaError_t e = cudaMemcpyAsync(lists, h.row.data(), nr * sizeof(int), cudaMemcpyHostToDevice, c->stream);
-  if (e == cudaSuccess && nc)
-    e = cudaMemcpyAsync(lists + nr, h.cols.data(), nc * sizeof(int), cudaMemcpyHostToDevice, c->stream);
+  // the lists the device derives the rest from, for that only
+  uint32_t* tmp = nullptr;
+  const size_t nr = h.row.size(), nc = h.cols.size(), nn = (size_t)c->Nn;
+  CK(cudaMalloc(reinterpret_cast<void**>(&tmp), (3 * nr + nc + nn) * sizeof(uint32_t)));
+  cudaError_t e = cudaSuccess;
+  size_t at = 0;
+  auto put = [&](const void* src, size_t n) {
+    const uint32_t* d = tmp + at;
+    if (e == cudaSuccess && n) e = cudaMemcpyAsync(tmp + at, src, n * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream);
+    at += n;
+    return d;
+  };
+  AsmLists t;
+  t.row = reinterpret_cast<const int*>(put(h.row.data(), nr));
+  t.erow = put(h.erow.data(), nr);
+  t.lrow = put(h.lrow.data(), nr);
+  t.slot0 = put(h.slot0.data(), nn);
+  t.cols = reinterpret_cast<const int*>(put(h.cols.data(), nc));
   if (e == cudaSuccess) {
-    launch_asm_fill(S, lists, lists + nr, c->stream);
+    launch_asm_fill(S, t.row, t.cols, c->stream);
+    launch_asm_lists(c->mesh(), t, edges, eptr, list, c->stream);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);  // the host tables go out of scope
-  cudaFree(lists);
+  cudaFree(tmp);
   CK(e);
+  if (c->npe == 8) {
+    uint32_t* hpos = nullptr;
+    if ((st = asm_upload(c, &hpos, (const uint32_t*)nullptr, 32 * (size_t)c->Ne)) ||
+        (st = asm_upload(c, &S.hblk4, (const float4*)nullptr, 2 * n_list)) ||
+        (st = asm_upload(c, &S.hblk1, (const float*)nullptr, n_list)))
+      return st;
+    CK(cudaMemsetAsync(hpos, 0xff, 32 * sizeof(uint32_t) * (size_t)c->Ne, c->stream));  // kNoPlace
+    launch_asm_hex_places(list, n_list, hpos, c->stream);
+    CKL();
+    S.hpos = hpos;
+  }
   c->asm_built = true;
   c->asm_valid = false;
   return FEM_OK;

@@ -57,7 +57,7 @@ bool pcg_coarse_tables(const std::vector<int>& cta_row, const std::vector<int>& 
   o->seg_rows.reserve(Nn);
   o->col_corners.resize((size_t)Nn + halo.size());
   std::vector<std::pair<int, int>> by_cell;
-  std::vector<int> seen(n_cn, -1), local(n_cn, 0), sptr;
+  std::vector<int> sptr;
   for (int g = 0; g < G; ++g) {
     by_cell.clear();
     for (int r = cta_row[g]; r < cta_row[g + 1]; ++r) by_cell.push_back({node_cell[r], r});
@@ -76,27 +76,34 @@ bool pcg_coarse_tables(const std::vector<int>& cta_row, const std::vector<int>& 
     }
     tabs[g][TAB_NSEG] = (int)sptr.size() - 1;
     put(g, TAB_SPTR, sptr);
-    const int nrow = cta_row[g + 1] - cta_row[g], nh = halo_ptr[g + 1] - halo_ptr[g];
-    // (ascending, so that neighbouring threads read neighbouring words of y_c)
-    auto cell_of = [&](int i) { return node_cell[i < nrow ? cta_row[g] + i : halo[halo_ptr[g] + i - nrow]]; };
-    std::vector<int>& lg = loc[g];
-    for (int i = 0; i < nrow + nh; ++i)
-      for (int q = 0; q < 8; ++q) {
-        const int cn = cell_corner[8 * (size_t)cell_of(i) + q];
-        if (seen[cn] != g) {
-          seen[cn] = g;
-          lg.push_back(cn);
+  }
+  parallel_ranges(G, [&](int g0, int g1) {
+    std::vector<int> seen(n_cn, -1), local(n_cn, 0);
+    for (int g = g0; g < g1; ++g) {
+      const int nrow = cta_row[g + 1] - cta_row[g], nh = halo_ptr[g + 1] - halo_ptr[g];
+      // (ascending, so that neighbouring threads read neighbouring words of y_c)
+      auto cell_of = [&](int i) { return node_cell[i < nrow ? cta_row[g] + i : halo[halo_ptr[g] + i - nrow]]; };
+      std::vector<int>& lg = loc[g];
+      for (int i = 0; i < nrow + nh; ++i)
+        for (int q = 0; q < 8; ++q) {
+          const int cn = cell_corner[8 * (size_t)cell_of(i) + q];
+          if (seen[cn] != g) {
+            seen[cn] = g;
+            lg.push_back(cn);
+          }
         }
+      std::sort(lg.begin(), lg.end());
+      for (size_t k = 0; k < lg.size(); ++k) local[lg[k]] = (int)k;
+      uint4* cc = o->col_corners.data() + cta_row[g] + halo_ptr[g];
+      for (int i = 0; i < nrow + nh; ++i) {
+        uint32_t idx[8];
+        for (int q = 0; q < 8; ++q) idx[q] = (uint32_t)local[cell_corner[8 * (size_t)cell_of(i) + q]];
+        cc[i] = make_uint4(idx[0] | idx[1] << 16, idx[2] | idx[3] << 16, idx[4] | idx[5] << 16, idx[6] | idx[7] << 16);
       }
-    if (lg.size() > 65536) return false;
-    std::sort(lg.begin(), lg.end());
-    for (size_t k = 0; k < lg.size(); ++k) local[lg[k]] = (int)k;
-    uint4* cc = o->col_corners.data() + cta_row[g] + halo_ptr[g];
-    for (int i = 0; i < nrow + nh; ++i) {
-      uint32_t idx[8];
-      for (int q = 0; q < 8; ++q) idx[q] = (uint32_t)local[cell_corner[8 * (size_t)cell_of(i) + q]];
-      cc[i] = make_uint4(idx[0] | idx[1] << 16, idx[2] | idx[3] << 16, idx[4] | idx[5] << 16, idx[6] | idx[7] << 16);
     }
+  }, 1);
+  for (int g = 0; g < G; ++g) {
+    if (loc[g].size() > 65536) return false;
     tabs[g][TAB_NLOC] = (int)loc[g].size();
     put(g, TAB_LOC, loc[g]);
     o->max_loc = std::max(o->max_loc, (int)loc[g].size());
