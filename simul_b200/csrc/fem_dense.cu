@@ -22,8 +22,16 @@
 //
 // The SIMT tile products run on a micro-kernel: 256 threads, each an
 // (B/16) x (B/16) block of the output tile, operands staged in shared memory
-// in chunks of kKC of the inner dimension.  These replace the cuSOLVER
-// potrf / potri and cuBLAS trsm / syrk calls the coarse set-up made before.
+// in chunks of kKC of the inner dimension, the next chunk on its way in
+// registers meanwhile (a 128^3 FP32 product 21 us against 24 without, a 64^3
+// FP64 one 9 against 13; 8.6 us would be the FMA rate of its one SM).  These
+// replace the cuSOLVER potrf / potri and cuBLAS trsm / syrk calls the coarse
+// set-up made before.
+//
+// What bounds the whole: the chain diagonal -> panel -> column update, one after
+// the other for each tile column, most of it the diagonal tile's 32 dependent
+// pivots per panel (55 us a tile in FP32, 34 in FP64; 61 and 42 with the inverse
+// as a pass of its own).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -40,11 +48,11 @@ template <typename T>
 struct DenseCfg;
 template <>
 struct DenseCfg<float> {
-  static constexpr int B = 128, TM = 8;
+  static constexpr int B = 128, TM = 8, kDiagThreads = 512;
 };
 template <>
 struct DenseCfg<double> {
-  static constexpr int B = 64, TM = 4;
+  static constexpr int B = 64, TM = 4, kDiagThreads = 256;
 };
 constexpr int kDenseThreads = 256;
 constexpr int kKC = 16;  // inner-dimension chunk staged in shared memory
@@ -72,35 +80,52 @@ constexpr int dense_ld() {  // shared row stride of a staged operand chunk
   return DenseCfg<T>::B + 4;
 }
 
-// Stages rows k0 .. k0 + kKC - 1 of the inner dimension of one B-row
-// operand into s[k][m]: element (m, k) is p[k * ld + m] (m contiguous, a
-// column-major tile) or, with KC, p[m * ld + k] (k contiguous).  16-byte
-// global loads along the contiguous index (all operand tiles start on a
-// multiple of B elements and ld is a multiple of B, so they are aligned).
+// Rows k0 .. k0 + kKC - 1 of the inner dimension of one B-row operand, into
+// registers (dense_fetch) and from there into s[k][m] (dense_put): element
+// (m, k) is p[k * ld + m] (m contiguous, a column-major tile) or, with KC,
+// p[m * ld + k] (k contiguous).  16-byte global loads along the contiguous
+// index (all operand tiles start on a multiple of B elements and ld is a
+// multiple of B, so they are aligned).
+template <typename T>
+constexpr int dense_nv() {  // a thread's vectors of a chunk
+  return DenseCfg<T>::B * kKC / Vec16<T>::W / kDenseThreads;
+}
+
 template <typename T, bool KC>
-__device__ __forceinline__ void dense_stage(const T* __restrict__ p, int ld, int k0, T* s) {
+__device__ __forceinline__ void dense_fetch(const T* __restrict__ p, int ld, int k0,
+                                            typename Vec16<T>::V (&v)[dense_nv<T>()]) {
   using VT = Vec16<T>;
   constexpr int B = DenseCfg<T>::B, W = VT::W;
-  constexpr int LD = dense_ld<T>();
-  constexpr int NV = B * kKC / W;  // vectors per chunk
 #pragma unroll
-  for (int q = threadIdx.x; q < NV; q += kDenseThreads) {
-    T v[W];
+  for (int i = 0; i < dense_nv<T>(); ++i) {
+    const int q = (int)threadIdx.x + i * kDenseThreads;
+    const size_t at = KC ? (size_t)(q / (kKC / W)) * ld + k0 + (q % (kKC / W)) * W
+                         : (size_t)(k0 + q / (B / W)) * ld + (q % (B / W)) * W;
+    v[i] = __ldcg(reinterpret_cast<const typename VT::V*>(p + at));
+  }
+}
+
+template <typename T, bool KC>
+__device__ __forceinline__ void dense_put(const typename Vec16<T>::V (&v)[dense_nv<T>()], T* s) {
+  using VT = Vec16<T>;
+  constexpr int B = DenseCfg<T>::B, W = VT::W, LD = dense_ld<T>();
+#pragma unroll
+  for (int i = 0; i < dense_nv<T>(); ++i) {
+    const int q = (int)threadIdx.x + i * kDenseThreads;
     if (KC) {
       const int m = q / (kKC / W), k = (q % (kKC / W)) * W;
-      VT::unpack(__ldcg(reinterpret_cast<const typename VT::V*>(p + (size_t)m * ld + k0 + k)), v);
+      T o[W];
+      VT::unpack(v[i], o);
 #pragma unroll
-      for (int w = 0; w < W; ++w) s[(k + w) * LD + m] = v[w];
+      for (int w = 0; w < W; ++w) s[(k + w) * LD + m] = o[w];
     } else {
-      const int k = q / (B / W), m = (q % (B / W)) * W;
-      *reinterpret_cast<typename VT::V*>(s + k * LD + m) =
-          __ldcg(reinterpret_cast<const typename VT::V*>(p + (size_t)(k0 + k) * ld + m));
+      *reinterpret_cast<typename VT::V*>(s + (q / (B / W)) * LD + (q % (B / W)) * W) = v[i];
     }
   }
 }
 
 // acc(r, c) += sum_k A(r, k) Bt(c, k) over one tile of the inner dimension
-// (k < B); A and Bt are B-row operands (see dense_stage).  Thread t owns the
+// (k < B); A and Bt are B-row operands (see dense_fetch).  Thread t owns the
 // rows ty * H + [0, H) and B/2 + ty * H + [0, H), ty = t % 16, and the same
 // columns with tx = t / 16 (H = TM / 2), so the lanes of a warp cover
 // consecutive rows: coalesced stores of a column-major tile.
@@ -111,11 +136,19 @@ __device__ __forceinline__ void dense_mma(T (&acc)[DenseCfg<T>::TM][DenseCfg<T>:
   constexpr int B = DenseCfg<T>::B, TM = DenseCfg<T>::TM, H = TM / 2, LD = dense_ld<T>();
   static_assert(H == VT::W, "a thread's half-row block is one 16-byte vector");
   const int ty = threadIdx.x & 15, tx = threadIdx.x >> 4;
+  // the next chunk is on its way while this one is multiplied
+  typename VT::V va[dense_nv<T>()], vb[dense_nv<T>()];
+  dense_fetch<T, AK>(A, lda, 0, va);
+  dense_fetch<T, BK>(Bt, ldb, 0, vb);
   for (int k0 = 0; k0 < B; k0 += kKC) {
     __syncthreads();
-    dense_stage<T, AK>(A, lda, k0, sA);
-    dense_stage<T, BK>(Bt, ldb, k0, sB);
+    dense_put<T, AK>(va, sA);
+    dense_put<T, BK>(vb, sB);
     __syncthreads();
+    if (k0 + kKC < B) {
+      dense_fetch<T, AK>(A, lda, k0 + kKC, va);
+      dense_fetch<T, BK>(Bt, ldb, k0 + kKC, vb);
+    }
 #pragma unroll
     for (int k = 0; k < kKC; ++k) {
       T a[TM], b[TM];
@@ -213,39 +246,48 @@ __device__ __forceinline__ double dense_rsqrt(double x) { return rsqrt(x); }
 // times per panel:
 //   Cholesky, panel p (columns j0 .. j0 + 31):
 //     warp 0 factors the 32 x 32 diagonal block in registers (lane = row,
-//     the pivot column passed by shuffles) and inverts it (lane = column,
-//     the factor read back as shared-memory broadcasts),
-//     the rows below are L_ip = A_ip X_pp^T (16 columns per thread),
+//     the pivot column passed by shuffles) and with the same shuffled values
+//     inverts it (lane = column): a second pass over the factor in shared
+//     memory took a third of the kernel,
+//     the rows below are L_ip = A_ip X_pp^T (8 columns per thread),
 //     the rank-32 update of the trailing lower triangle runs on 4 x 4
 //     register tiles;
 //   then block row k is finished (X_kq = X_kk R_kq, q < k) and subtracted
 //   from the rows below (R_iq -= L_ik X_kq), for k = 0, 1, ...
 template <typename T>
-__global__ void __launch_bounds__(kDenseThreads) dense_diag_kernel(T* A, T* W, int N, int k, int* info) {
-  constexpr int B = DenseCfg<T>::B, S = B + 1, P = 32, NP = B / P;
+__global__ void __launch_bounds__(DenseCfg<T>::kDiagThreads) dense_diag_kernel(T* A, T* W, int N, int k, int* info) {
+  constexpr int B = DenseCfg<T>::B, S = B + 1, P = 32, NP = B / P, kDT = DenseCfg<T>::kDiagThreads;
   constexpr unsigned kFull = 0xffffffffu;
   extern __shared__ __align__(16) unsigned char s_raw[];
   T* L = reinterpret_cast<T*>(s_raw);  // L[c * S + r]
   T* X = L + B * S;                     // X[c * S + r] = (L^-1)(r, c)
   T* Xt = X + B * S;                    // Xt[l * P + j] = (L_pp^-1)(j, l), current panel
-  __shared__ T s_rinv[32];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const size_t off = (size_t)k * B * N + (size_t)k * B;
+  using VB = Vec16<T>;
+  constexpr int WB = VB::W;
 #pragma unroll 8
-  for (int it = 0; it < B * B / kDenseThreads; ++it) {
-    const int q = tid + it * kDenseThreads, c = q / B, r = q % B;
-    const T v = A[off + (size_t)c * N + r];
-    L[c * S + r] = r >= c ? v : T(0);
-    X[c * S + r] = T(0);
+  for (int it = 0; it < B * B / WB / kDT; ++it) {
+    const int q = tid + it * kDT, c = q / (B / WB), r = (q % (B / WB)) * WB;
+    T v[WB];
+    VB::unpack(*reinterpret_cast<const typename VB::V*>(A + off + (size_t)c * N + r), v);
+#pragma unroll
+    for (int w = 0; w < WB; ++w) {
+      L[c * S + r + w] = r + w >= c ? v[w] : T(0);
+      X[c * S + r + w] = T(0);
+    }
   }
   __syncthreads();
   for (int p = 0; p < NP; ++p) {
     const int j0 = p * P;
     if (warp == 0) {
       T a[P];  // row j0 + lane of the diagonal block
-      T rinv = T(0);  // lane r: 1 / L(j0 + r, j0 + r)
+      T x[P];  // column lane of its inverse: before step j, delta(r, lane) - sum_{l < j} L(r, l) x[l]
 #pragma unroll
-      for (int c = 0; c < P; ++c) a[c] = c <= lane ? L[(j0 + c) * S + j0 + lane] : T(0);
+      for (int c = 0; c < P; ++c) {
+        a[c] = c <= lane ? L[(j0 + c) * S + j0 + lane] : T(0);
+        x[c] = c == lane ? T(1) : T(0);
+      }
 #pragma unroll
       for (int j = 0; j < P; ++j) {
         T d = __shfl_sync(kFull, a[j], j);
@@ -254,34 +296,21 @@ __global__ void __launch_bounds__(kDenseThreads) dense_diag_kernel(T* A, T* W, i
           d = T(1);
         }
         const T rs = dense_rsqrt(d);  // 1 / L(j, j)
-        if (lane == j) {
-          a[j] = d * rs;
-          rinv = rs;
-        }
+        if (lane == j) a[j] = d * rs;
         if (lane > j) a[j] *= rs;
+        x[j] *= rs;
 #pragma unroll
         for (int c = 1; c < P; ++c) {  // c > j: constant trip counts unroll fully
           if (c > j) {
             const T lc = __shfl_sync(kFull, a[j], c);
             if (lane >= c) a[c] -= a[j] * lc;
+            x[c] -= lc * x[j];
           }
         }
       }
 #pragma unroll
       for (int c = 0; c < P; ++c)
         if (c <= lane) L[(j0 + c) * S + j0 + lane] = a[c];
-      s_rinv[lane] = rinv;
-      __syncwarp();
-      // column lane of L_pp^-1: x[r] = (delta(r, lane) - sum_{l < r} L(r, l) x[l]) / L(r, r)
-      T x[P];
-#pragma unroll
-      for (int r = 0; r < P; ++r) {
-        T acc = r == lane ? T(1) : T(0);
-#pragma unroll
-        for (int l = 0; l < P - 1; ++l)
-          if (l < r) acc -= L[(j0 + l) * S + j0 + r] * x[l];
-        x[r] = acc * s_rinv[r];
-      }
 #pragma unroll
       for (int r = 0; r < P; ++r) {
         X[(j0 + lane) * S + j0 + r] = x[r];
@@ -292,8 +321,8 @@ __global__ void __launch_bounds__(kDenseThreads) dense_diag_kernel(T* A, T* W, i
     const int rows = B - j0 - P;  // rows below the diagonal block
     if (rows == 0) break;
     {
-      // L(r, j0 + j) = sum_{l <= j} A(r, j0 + l) Xt[l * P + j], columns 16 cg .. 16 cg + 15
-      constexpr int CG = 16;
+      // L(r, j0 + j) = sum_{l <= j} A(r, j0 + l) Xt[l * P + j], columns 8 cg .. 8 cg + 7
+      constexpr int CG = 8;
       using VT = Vec16<T>;
       constexpr int W = VT::W;
       const bool act = tid < rows * (P / CG);
@@ -325,7 +354,7 @@ __global__ void __launch_bounds__(kDenseThreads) dense_diag_kernel(T* A, T* W, i
     {
       // trailing lower triangle on 4 x 4 tiles: L(r, c) -= sum_l L(r, j0 + l) L(c, j0 + l)
       const int nt4 = rows / 4, ntri = nt4 * (nt4 + 1) / 2, base = j0 + P;
-      for (int q = tid; q < ntri; q += kDenseThreads) {
+      for (int q = tid; q < ntri; q += kDT) {
         int ti, tj;  // tj <= ti
         dense_tri(q, ti, tj);
         const int r0 = base + 4 * ti, c0 = base + 4 * tj;
@@ -360,7 +389,7 @@ __global__ void __launch_bounds__(kDenseThreads) dense_diag_kernel(T* A, T* W, i
   // accumulated in place), then R_iq -= L_ik X_kq for the row blocks below,
   // for kb = 0, 1, ...: register-tiled, lane = row, the other operand
   // broadcast from shared memory
-  constexpr int NW = kDenseThreads / 32;
+  constexpr int NW = kDT / 32;
   for (int kb = 0; kb < NP; ++kb) {
     const int k0 = kb * P;
     if (kb > 0) {
@@ -404,16 +433,23 @@ __global__ void __launch_bounds__(kDenseThreads) dense_diag_kernel(T* A, T* W, i
       __syncthreads();
     }
   }
-  for (int q = tid; q < B * B; q += kDenseThreads) {
-    const int c = q / B, r = q % B;
-    A[off + (size_t)c * N + r] = L[c * S + r];
-    W[off + (size_t)c * N + r] = X[c * S + r];
+#pragma unroll 4
+  for (int it = 0; it < B * B / WB / kDT; ++it) {
+    const int q = tid + it * kDT, c = q / (B / WB), r = (q % (B / WB)) * WB;
+    T v[WB], x[WB];
+#pragma unroll
+    for (int w = 0; w < WB; ++w) {
+      v[w] = L[c * S + r + w];
+      x[w] = X[c * S + r + w];
+    }
+    *reinterpret_cast<typename VB::V*>(A + off + (size_t)c * N + r) = VB::pack(v);
+    *reinterpret_cast<typename VB::V*>(W + off + (size_t)c * N + r) = VB::pack(x);
   }
 }
 
 // L_ik = A_ik W_kk^T for i = k + 1 + blockIdx.x
 template <typename T>
-__global__ void __launch_bounds__(kDenseThreads) dense_panel_kernel(T* A, const T* W, int N, int k) {
+__global__ void __launch_bounds__(kDenseThreads, 2) dense_panel_kernel(T* A, const T* W, int N, int k) {
   constexpr int B = DenseCfg<T>::B, TM = DenseCfg<T>::TM;
   __shared__ __align__(16) T sA[kKC * dense_ld<T>()];
   __shared__ __align__(16) T sB[kKC * dense_ld<T>()];
@@ -432,7 +468,7 @@ __global__ void __launch_bounds__(kDenseThreads) dense_panel_kernel(T* A, const 
 // (i = k + 1 + blockIdx.x), else the triangle j >= k + 1 + j_ofs (blockIdx.x
 // in row order).
 template <typename T, bool COL>
-__global__ void __launch_bounds__(kDenseThreads) dense_update_kernel(T* A, int N, int k, int j_ofs) {
+__global__ void __launch_bounds__(kDenseThreads, 2) dense_update_kernel(T* A, int N, int k, int j_ofs) {
   constexpr int B = DenseCfg<T>::B, TM = DenseCfg<T>::TM;
   __shared__ __align__(16) T sA[kKC * dense_ld<T>()];
   __shared__ __align__(16) T sB[kKC * dense_ld<T>()];
@@ -453,7 +489,7 @@ __global__ void __launch_bounds__(kDenseThreads) dense_update_kernel(T* A, int N
 // subtracts it from the rows below (dense_wupd_kernel: R_ij -= L_ik W_kj,
 // i > k, j <= k), one tile product per CTA.
 template <typename T>
-__global__ void __launch_bounds__(kDenseThreads) dense_wfin_kernel(T* W, int N, int k) {
+__global__ void __launch_bounds__(kDenseThreads, 2) dense_wfin_kernel(T* W, int N, int k) {
   constexpr int B = DenseCfg<T>::B, TM = DenseCfg<T>::TM;
   __shared__ __align__(16) T sA[kKC * dense_ld<T>()];
   __shared__ __align__(16) T sB[kKC * dense_ld<T>()];
@@ -468,7 +504,7 @@ __global__ void __launch_bounds__(kDenseThreads) dense_wfin_kernel(T* W, int N, 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kDenseThreads) dense_wupd_kernel(const T* A, T* W, int N, int k) {
+__global__ void __launch_bounds__(kDenseThreads, 2) dense_wupd_kernel(const T* A, T* W, int N, int k) {
   constexpr int B = DenseCfg<T>::B, TM = DenseCfg<T>::TM;
   __shared__ __align__(16) T sA[kKC * dense_ld<T>()];
   __shared__ __align__(16) T sB[kKC * dense_ld<T>()];
@@ -687,7 +723,7 @@ static cudaError_t dense_inverse_t(const double* Ac, int n, T* A, T* W, int* inf
   cudaEventRecord(ev[nt], s);
   cudaStreamWaitEvent(crit, ev[nt], 0);
   for (int k = 0; k < nt; ++k) {
-    dense_diag_kernel<T><<<1, kDenseThreads, diag_smem, crit>>>(A, W, N, k, info);
+    dense_diag_kernel<T><<<1, DenseCfg<T>::kDiagThreads, diag_smem, crit>>>(A, W, N, k, info);
     ++nl;
     const int m = last[k] - k;  // nonzero tiles below the diagonal in column k
     if (m > 0) {
