@@ -1044,7 +1044,8 @@ int ensure_assembled(FemCtx* c) {
   return FEM_OK;
 }
 
-// fneg_out: the negative internal force in caller order (may be null)
+// fneg_out: the negative internal force in caller order (may be null).
+// rnorm2: ||R||^2; null: neither read back nor waited for.
 int eval_residual(FemCtx* c, double* fneg_out, double* rnorm2) {
   ResArgs a;
   a.m = c->mesh();
@@ -1066,8 +1067,10 @@ int eval_residual(FemCtx* c, double* fneg_out, double* rnorm2) {
   c->n_launches += c->npe == 8 ? 2 : 1;
   launch_residual(a, c->model_kind, c->stream);
   CKL();
-  CK(cudaMemcpyAsync(c->h_scalars, c->scalars, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  if (rnorm2) {
+    CK(cudaMemcpyAsync(c->h_scalars, c->scalars, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+  }
   c->tangent_valid = true;
   // linear models have no tangent payload: their blocks stay those of the materials
   if (c->model_kind != M_LE && c->model_kind != M_TI) c->asm_valid = false;
@@ -3055,7 +3058,7 @@ int fem_element_forces(void* ctx, const double* u, double* f_out, double* residu
     CKL();
   }
   double r2 = 0;
-  if ((st = eval_residual(c, f_out, &r2))) return st;
+  if ((st = eval_residual(c, f_out, rnorm ? &r2 : nullptr))) return st;
   if (residual_out) {
     ++c->n_launches; launch_scatter_d(c->R, residual_out, c->d_perm_node, c->Nn, c->stream);
     CKL();

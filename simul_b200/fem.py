@@ -50,6 +50,13 @@ def _ptr(t: Optional[torch.Tensor]):
     return C.c_void_p(t.data_ptr())
 
 
+def _ptrs(*tensors: torch.Tensor):
+    """``_ptr`` of several tensors of one device, waiting for torch's pending
+    writes once (a wait costs the host 4 us, as much as a small kernel)."""
+    first, rest = tensors[0], tensors[1:]
+    return [_ptr(first)] + [C.c_void_p(t.data_ptr()) for t in rest]
+
+
 def _check(rc: int, ctx=None, what: str = ""):
     if rc in (_lib.FEM_OK, _lib.FEM_NOT_CONVERGED):
         return rc
@@ -378,7 +385,7 @@ class FEMesh:
                                      parameter="material")
         if getattr(self, "mises", None) is None:
             self.mises = torch.zeros(self.n_nodes, dtype=torch.float64, device=self.device)
-        _check(_lib.load().fem_nodal_mises(self.ctx, _ptr(self.u.contiguous()), _ptr(self.mises), int(average)),
+        _check(_lib.load().fem_nodal_mises(self.ctx, *_ptrs(self.u.contiguous(), self.mises), int(average)),
                self.ctx, "fem_nodal_mises")
 
 
@@ -440,16 +447,16 @@ class MaterialBase:
     def compute_stress(self, mesh: FEMesh):
         """Cauchy stress per Gauss point into ``mesh.stress`` (and F into ``mesh.F``)."""
         self._ensure_bound(mesh)
-        _check(_lib.load().fem_compute_stress(mesh.ctx, _ptr(mesh.u.contiguous()), _ptr(mesh.F),
-                                              _ptr(mesh.stress)), mesh.ctx, "fem_compute_stress")
+        _check(_lib.load().fem_compute_stress(mesh.ctx, *_ptrs(mesh.u.contiguous(), mesh.F, mesh.stress)),
+               mesh.ctx, "fem_compute_stress")
 
     def compute_nodal_forces(self, mesh: FEMesh):
         """Negative internal force into ``mesh.f`` (deterministic gather, no atomics)."""
         self._ensure_bound(mesh)
         if mesh._bc_dirty:
             mesh._push_bc()
-        _check(_lib.load().fem_element_forces(mesh.ctx, _ptr(mesh.u.contiguous()), _ptr(mesh.f),
-                                              None, None), mesh.ctx, "fem_element_forces")
+        _check(_lib.load().fem_element_forces(mesh.ctx, *_ptrs(mesh.u.contiguous(), mesh.f), None, None),
+               mesh.ctx, "fem_element_forces")
 
     def get_elasticity_tensor(self) -> np.ndarray:
         raise NotImplementedError
