@@ -44,41 +44,49 @@ __device__ __forceinline__ float block_sum_f(float v, float* sh) {
 }  // namespace
 
 // ───────────────────────── coarse operator assembly ─────────────────────────
-// One CTA per lattice cell.  Chunks of kCellThreads elements: each thread
-// writes its element's 12x12 tangent (fixed rows and columns zeroed) and the
-// 4x8 trilinear weights to shared memory; then each thread owns up to five of
-// the cell's 24x24 block entries and adds w_a,c1 K_ab w_b,c2 over the chunk,
-// in element order (FP32 products, FP64 accumulation).
-constexpr int kCellThreads = 128;
-constexpr int kCellEntries = 576;  // (8 corners x 3)^2
-constexpr int kCellOwned = (kCellEntries + kCellThreads - 1) / kCellThreads;
+// kCellSlices CTAs per lattice cell, in chunks of kCellChunk elements.  First
+// three threads per element, one per direction d2 of the displaced vertex:
+// the 12 x 4 columns of its tangent (fixed rows and columns zeroed) in
+// registers, contracted with the trilinear weights of the column vertices,
+//   T(a d1, c2 d2) = sum_b K(a d1, b d2) w_b,c2,
+// into shared memory (FP32).  Then 72 threads per half of the chunk, one per
+// (d1, c2 d2), add sum_a w_a,c1 T(a d1, c2 d2) for the eight corners c1, in
+// element order (FP32 products, FP64 accumulation); the halves are added last.
+// The 24 x 24 entries straight from K took 20 multiplications and 32
+// shared-memory reads per entry and element; this form 4 + 2 and 1.5: 302 us
+// against 1,040 at 566,000 J2 elements and 4-voxel cells, 132 against 480 at
+// 236,000 elements in 1,900-element cells.
+constexpr int kCellChunk = 32;
+constexpr int kCellThreads = 160;
+constexpr int kCellEntries = 576;           // (8 corners x 3)^2
+constexpr int kCellT = 12 * 24 + 1;         // words of an element's T (odd: lanes are elements)
 // CTAs per cell: slice s takes chunks s, s + kCellSlices, ... of the cell's
 // elements; the dense kernel adds the slices in order
 constexpr int kCellSlices = 8;
 
 template <int MODEL>
 __global__ void __launch_bounds__(kCellThreads) coarse_cell_kernel(const __grid_constant__ CoarseArgs a) {
-  extern __shared__ __align__(16) float s_cell[];
-  float* sK = s_cell;                                // [kCellThreads][144]
-  float* sW = s_cell + kCellThreads * 144;           // [kCellThreads][32]
+  __shared__ __align__(16) float sT[kCellChunk * kCellT];
+  __shared__ __align__(16) float sW[kCellChunk][36];  // [4][8] (padded rows)
   const MeshDev& m = a.m;
   const CoarseDev& c = a.c;
   const int cell = blockIdx.x / kCellSlices, slice = blockIdx.x - cell * kCellSlices;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int3 ijk = c.cell_ijk[cell];
   const int e0 = c.cell_elem_ptr[cell], e1 = c.cell_elem_ptr[cell + 1];
-  double acc[kCellOwned];
+  // the sums' part: half of the chunk, direction d1, column 3 c2 + d2
+  const int half = tid / 72, item = tid - 72 * half, d1s = item / 24, col = item - 24 * d1s;
+  double acc[8];
 #pragma unroll
-  for (int k = 0; k < kCellOwned; ++k) acc[k] = 0.0;
-  for (int c0 = e0 + slice * kCellThreads; c0 < e1; c0 += kCellSlices * kCellThreads) {
-    const int idx = c0 + tid;
-    float* K = sK + tid * 144;
-    float* W = sW + tid * 32;
-    if (idx < e1) {
-      const int e = __ldg(c.cell_elems + idx);
+  for (int k = 0; k < 8; ++k) acc[k] = 0.0;
+  for (int c0 = e0 + slice * kCellChunk; c0 < e1; c0 += kCellSlices * kCellChunk) {
+    const int nvalid = min(kCellChunk, e1 - c0);
+    if (warp < 3 && lane < nvalid) {
+      const int d2 = warp;
+      const int e = __ldg(c.cell_elems + c0 + lane);
       const int4 cn = __ldg(m.conn + e);
       const int nid[4] = {cn.x, cn.y, cn.z, cn.w};
-      float xv[4][3];
+      float xv[4][3], W[4][8];
       int fx[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -90,7 +98,10 @@ __global__ void __launch_bounds__(kCellThreads) coarse_cell_kernel(const __grid_
         float t[3];
         cell_local(c, ijk, X.x, X.y, X.z, t);
 #pragma unroll
-        for (int q = 0; q < 8; ++q) W[k * 8 + q] = tri_weight(t[0], t[1], t[2], q);
+        for (int q = 0; q < 8; ++q) {
+          W[k][q] = tri_weight(t[0], t[1], t[2], q);
+          if (d2 == 0) sW[lane][k * 8 + q] = W[k][q];
+        }
       }
       TetGeom<float> g;
       tet_geom(xv[0], xv[1], xv[2], xv[3], g);
@@ -111,73 +122,84 @@ __global__ void __launch_bounds__(kCellThreads) coarse_cell_kernel(const __grid_
         w[3][j] = g.c[2][j];
         w[0][j] = -(g.c[0][j] + g.c[1][j] + g.c[2][j]);
       }
+      float K[4][12];
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
+        const bool col_fixed = (fx[b] >> d2) & 1;
+        float dF[9], dP[9];
 #pragma unroll
-        for (int d2 = 0; d2 < 3; ++d2) {
-          const bool col_fixed = (fx[b] >> d2) & 1;
-          float dF[9];
+        for (int i = 0; i < 3; ++i)
 #pragma unroll
-          for (int k = 0; k < 9; ++k) dF[k] = 0.f;
+          for (int j = 0; j < 3; ++j) dF[3 * i + j] = i == d2 ? w[b][j] * g.inv_det : 0.f;
+        dP_any<MODEL>(mat, scale, pay, dF, dP);
 #pragma unroll
-          for (int j = 0; j < 3; ++j) dF[3 * d2 + j] = w[b][j] * g.inv_det;
-          float dP[9];
-          dP_any<MODEL>(mat, scale, pay, dF, dP);
+        for (int aa = 0; aa < 4; ++aa)
 #pragma unroll
-          for (int aa = 0; aa < 4; ++aa)
-#pragma unroll
-            for (int d1 = 0; d1 < 3; ++d1) {
-              const float v = g.s6 * (dP[3 * d1] * w[aa][0] + dP[3 * d1 + 1] * w[aa][1] +
-                                      dP[3 * d1 + 2] * w[aa][2]);
-              const bool row_fixed = (fx[aa] >> d1) & 1;
-              K[(3 * aa + d1) * 12 + 3 * b + d2] = (col_fixed || row_fixed) ? 0.f : v;
-            }
-        }
-      }
-    }
-    __syncthreads();
-    const int nvalid = min(kCellThreads, e1 - c0);
-#pragma unroll
-    for (int k = 0; k < kCellOwned; ++k) {
-      const int q = tid + k * kCellThreads;
-      if (q < kCellEntries) {
-        const int r = q / 24, col = q - 24 * r;
-        const int c1 = r / 3, d1 = r - 3 * c1;
-        const int c2 = col / 3, d2 = col - 3 * c2;
-        for (int el = 0; el < nvalid; ++el) {
-          const float* K = sK + el * 144;
-          const float* W = sW + el * 32;
-          float s = 0.f;
-#pragma unroll
-          for (int aa = 0; aa < 4; ++aa) {
-            float t = 0.f;
-#pragma unroll
-            for (int b = 0; b < 4; ++b) t += K[(3 * aa + d1) * 12 + 3 * b + d2] * W[b * 8 + c2];
-            s += W[aa * 8 + c1] * t;
+          for (int d1 = 0; d1 < 3; ++d1) {
+            const float v = g.s6 * (dP[3 * d1] * w[aa][0] + dP[3 * d1 + 1] * w[aa][1] + dP[3 * d1 + 2] * w[aa][2]);
+            const bool row_fixed = (fx[aa] >> d1) & 1;
+            K[b][3 * aa + d1] = (col_fixed || row_fixed) ? 0.f : v;
           }
-          acc[k] += (double)s;
-        }
       }
+      float* T = sT + lane * kCellT + d2;
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+#pragma unroll
+        for (int r = 0; r < 12; ++r) {
+          float t = 0.f;
+#pragma unroll
+          for (int b = 0; b < 4; ++b) t += K[b][r] * W[b][q];
+          T[24 * r + 3 * q] = t;
+        }
     }
     __syncthreads();
-  }
+    if (half < 2)
+      for (int el = half * (kCellChunk / 2); el < min(nvalid, (half + 1) * (kCellChunk / 2)); ++el) {
+        const float* T = sT + el * kCellT + 24 * d1s + col;
+        float s[8];
 #pragma unroll
-  for (int k = 0; k < kCellOwned; ++k) {
-    const int q = tid + k * kCellThreads;
-    if (q < kCellEntries) c.blocks[(size_t)blockIdx.x * kCellEntries + q] = acc[k];
+        for (int q = 0; q < 8; ++q) s[q] = 0.f;
+#pragma unroll
+        for (int aa = 0; aa < 4; ++aa) {
+          const float t = T[72 * aa];
+          const float4 w0 = *reinterpret_cast<const float4*>(&sW[el][8 * aa]);
+          const float4 w1 = *reinterpret_cast<const float4*>(&sW[el][8 * aa + 4]);
+          s[0] += w0.x * t; s[1] += w0.y * t; s[2] += w0.z * t; s[3] += w0.w * t;
+          s[4] += w1.x * t; s[5] += w1.y * t; s[6] += w1.z * t; s[7] += w1.w * t;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc[q] += (double)s[q];
+      }
+    __syncthreads();
   }
+  // the second half's sums onto the first's
+  double* s_acc = reinterpret_cast<double*>(sT);
+  if (half == 1)
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s_acc[72 * q + item] = acc[q];
+  __syncthreads();
+  if (half == 0)
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      c.blocks[(size_t)blockIdx.x * kCellEntries + (3 * q + d1s) * 24 + col] = acc[q] + s_acc[72 * q + item];
 }
 
-// Dense Ac (column-major, symmetric) from the cell blocks: entry (I, J) adds
-// the blocks of the cells that hold both coarse nodes, in ascending cell
-// order.  A DOF no free mesh DOF reaches gets a unit diagonal.
-__global__ void coarse_dense_kernel(const __grid_constant__ CoarseDev c) {
+// Dense Ac (column-major, symmetric, zeroed before) from the cell blocks:
+// entry (I, J) adds the blocks of the cells that hold both coarse nodes, in
+// ascending cell order.  A DOF no free mesh DOF reaches gets a unit diagonal.
+// A thread per (node of I, its k-th cell, corner t, d_I, d_J), at work where
+// cell k is the first to hold both nodes: a thread per entry of the matrix
+// searched the cells of every pair, 1,350 us at 7,728 unknowns for some 80
+// columns a row; now 37 us and the zeroing of the matrix.
+__global__ void __launch_bounds__(256) coarse_dense_kernel(const __grid_constant__ CoarseDev c) {
   const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = c.n_dof;
-  if (q >= (int64_t)n * n) return;
-  const int I = (int)(q % n), J = (int)(q / n);
-  const int nI = I / 3, dI = I - 3 * nI;
-  const int nJ = J / 3, dJ = J - 3 * nJ;
+  if (q >= (int64_t)c.n_cn * 64 * 9) return;
+  const int dd = (int)(q % 9), dI = dd % 3, dJ = dd / 3;
+  const int64_t p = q / 9;
+  const int nI = (int)(p >> 6), k0 = (int)(p >> 3) & 7, t0 = (int)p & 7;
+  const int ent0 = c.cn_cells[nI * 8 + k0];
+  if (ent0 < 0) return;
+  const int nJ = c.cell_corner[(ent0 >> 3) * 8 + t0];
   double acc = 0.0;
   for (int k = 0; k < 8; ++k) {
     const int ent = c.cn_cells[nI * 8 + k];
@@ -187,14 +209,14 @@ __global__ void coarse_dense_kernel(const __grid_constant__ CoarseDev c) {
 #pragma unroll
     for (int t = 0; t < 8; ++t)
       if (c.cell_corner[cell * 8 + t] == nJ) cJ = t;
-    if (cJ >= 0) {
-      const size_t off = (size_t)(3 * cI + dI) * 24 + 3 * cJ + dJ;
-      for (int sl = 0; sl < c.cell_slices; ++sl)
-        acc += c.blocks[((size_t)cell * c.cell_slices + sl) * kCellEntries + off];
-    }
+    if (cJ < 0) continue;
+    if (k < k0 || (k == k0 && cJ != t0)) return;  // another thread's pair
+    const size_t off = (size_t)(3 * cI + dI) * 24 + 3 * cJ + dJ;
+    for (int sl = 0; sl < c.cell_slices; ++sl)
+      acc += c.blocks[((size_t)cell * c.cell_slices + sl) * kCellEntries + off];
   }
-  if (I == J && !(acc > 0.0)) acc = 1.0;
-  c.Ac[q] = acc;
+  if (nI == nJ && dI == dJ && !(acc > 0.0)) acc = 1.0;
+  c.Ac[(size_t)(3 * nJ + dJ) * c.n_dof + 3 * nI + dI] = acc;
 }
 
 // Symmetric FP32 copy of the inverse whose lower triangle the dense inverse wrote
@@ -842,7 +864,6 @@ __global__ void jacobi_apply_kernel(const float* __restrict__ r, const float* __
 
 static inline int nblk(int64_t n, int t) { return (int)((n + t - 1) / t); }
 
-size_t coarse_cell_smem() { return sizeof(float) * kCellThreads * (144 + 32); }
 int coarse_cell_slices(int npe) { return npe == 8 ? kCellSlices * 4 : kCellSlices; }
 int coarse_restrict_slices(int n_cells) {
   int dev = 0, sms = 0;
@@ -867,20 +888,19 @@ void prepare_coarse_kernels(int model, int n_dof) {
 }
 
 void launch_coarse_assemble(const CoarseArgs& a, int model, cudaStream_t s) {
-  const size_t smem = coarse_cell_smem();
   const int g = a.c.n_cells * kCellSlices;
   if (a.m.npe == 8) launch_coarse_cells_hex(a, model, s);
   else switch (model) {
-    case M_LE: coarse_cell_kernel<M_LE><<<g, kCellThreads, smem, s>>>(a); break;
-    case M_NH: coarse_cell_kernel<M_NH><<<g, kCellThreads, smem, s>>>(a); break;
-    case M_MR: coarse_cell_kernel<M_MR><<<g, kCellThreads, smem, s>>>(a); break;
-    case M_J2: coarse_cell_kernel<M_J2><<<g, kCellThreads, smem, s>>>(a); break;
-    case M_TI: coarse_cell_kernel<M_TI><<<g, kCellThreads, smem, s>>>(a); break;
-    case M_FMR: coarse_cell_kernel<M_FMR><<<g, kCellThreads, smem, s>>>(a); break;
-    default: coarse_cell_kernel<-1><<<g, kCellThreads, smem, s>>>(a); break;
+    case M_LE: coarse_cell_kernel<M_LE><<<g, kCellThreads, 0, s>>>(a); break;
+    case M_NH: coarse_cell_kernel<M_NH><<<g, kCellThreads, 0, s>>>(a); break;
+    case M_MR: coarse_cell_kernel<M_MR><<<g, kCellThreads, 0, s>>>(a); break;
+    case M_J2: coarse_cell_kernel<M_J2><<<g, kCellThreads, 0, s>>>(a); break;
+    case M_TI: coarse_cell_kernel<M_TI><<<g, kCellThreads, 0, s>>>(a); break;
+    case M_FMR: coarse_cell_kernel<M_FMR><<<g, kCellThreads, 0, s>>>(a); break;
+    default: coarse_cell_kernel<-1><<<g, kCellThreads, 0, s>>>(a); break;
   }
-  const int64_t nn = (int64_t)a.c.n_dof * a.c.n_dof;
-  coarse_dense_kernel<<<nblk(nn, 256), 256, 0, s>>>(a.c);
+  cudaMemsetAsync(a.c.Ac, 0, sizeof(double) * (size_t)a.c.n_dof * a.c.n_dof, s);
+  coarse_dense_kernel<<<nblk((int64_t)a.c.n_cn * 64 * 9, 256), 256, 0, s>>>(a.c);
 }
 
 void launch_coarse_symmetrize(const CoarseDev& c, cudaStream_t s) {

@@ -434,7 +434,6 @@ void launch_matvec(const MvArgs& a, int model, cudaStream_t s);
 void prepare_kernels(const MeshDev& m, int model);
 void launch_diag(const DiagArgs& a, int model, cudaStream_t s);
 // coarse lattice (fem_coarse.cu)
-size_t coarse_cell_smem();
 // Galerkin block slots per lattice cell (TET4: one per CTA; HEX8: one per warp)
 int coarse_cell_slices(int npe);
 int coarse_restrict_slices(int n_cells);  // node slices (restriction warps) per lattice cell
