@@ -1091,8 +1091,9 @@ int compute_dinv(FemCtx* c, int precond, bool block = false) {
     a.payload = c->payload;
     a.dinv = c->dinv;
     a.boff = block ? c->boff : nullptr;
-    a.stage = c->stage;
-    c->n_launches += c->npe == 8 ? 2 : 1;
+    // (TET4: the residual's staging has the 32 bytes a slot needs)
+    a.stage = c->npe == 8 ? c->stage : reinterpret_cast<float4*>(c->stage_d);
+    c->n_launches += 2;
     launch_diag(a, c->model_kind, c->stream);
     CKL();
   } else {

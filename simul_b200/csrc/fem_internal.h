@@ -254,7 +254,7 @@ struct DiagArgs {
   const float* payload;
   float* dinv;              // [Nn] float4: 1/diag(K) on free DOFs, 0 elsewhere
   float* boff;              // non-null: nodal 3x3 block inverse, dinv its diagonal, boff (01, 02, 12)
-  float4* stage;            // HEX8: [2 * 8 Ne] per slot the 6 block entries (or 3 diagonal entries)
+  float4* stage;            // [2 * npe Ne] per slot the 6 block entries (or 3 diagonal entries)
 };
 
 // Coarse lattice of the two-level preconditioner (fem_coarse.cu).  Cells

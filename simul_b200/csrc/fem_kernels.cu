@@ -58,23 +58,6 @@ __device__ __forceinline__ void gather_chunk(const uint32_t* s_slots, const T (*
   }
 }
 
-// gather_chunk for W values per slot: sf[W * slot + k][thread]
-template <int NB, int W>
-__device__ __forceinline__ void gather_chunk_w(const uint32_t* s_slots, const float (*sf)[NB], int base, int& cur,
-                                               int end, float (&acc)[W]) {
-  const int lim = base + NB;
-  while (cur < end) {
-    const uint32_t ent = s_slots[cur];
-    const int li = (int)(ent >> 2);
-    if (li >= lim) break;
-    const int t = li - base;
-    const int s = (int)(ent & 3u);
-#pragma unroll
-    for (int k = 0; k < W; ++k) acc[k] += sf[W * s + k][t];
-    ++cur;
-  }
-}
-
 // ───────────────────────── residual (FP64) ─────────────────────────
 
 // Element e's four slot forces (FP64, the negative internal force of its
@@ -803,89 +786,110 @@ __global__ void __launch_bounds__(256) res_gather_kernel(const __grid_constant__
 // fixed rows and columns are zero.  A block that is not positive definite
 // falls back to the scalar inverse of its diagonal.
 
-template <int NB, int MODEL, bool BLOCK>
-__global__ void __launch_bounds__(NB) diag_kernel(const __grid_constant__ DiagArgs a) {
+// Two passes: one thread per element stores its four slots' entries in
+// node-slot order (32-byte rows of the residual's staging, two float4: 00 01 02
+// 11 | 12 22, or the diagonal), then a thread per node adds its rows in that
+// order, eight in flight.  (Evaluated per node block, with the elements that
+// several blocks share in each of them, it took 45 us at 236,000 J2 elements, 28 now;
+// the passes' traffic is 64 + 64 bytes an element.)
+template <int MODEL, bool BLOCK>
+__global__ void __launch_bounds__(128) diag_elem_kernel(const __grid_constant__ DiagArgs a) {
   constexpr int W = BLOCK ? 6 : 3;
-  extern __shared__ __align__(16) unsigned char s_dyn[];
-  uint32_t* s_slots = reinterpret_cast<uint32_t*>(s_dyn);
-  __shared__ float sf[4 * W][NB];
   const MeshDev& m = a.m;
-  const int b = blockIdx.x;
-  const int tid = threadIdx.x;
-  const int node = b * NB + tid;
-  const bool has_node = node < m.n_nodes;
-  int cur, end;
-  load_block_slots<NB>(m, b, s_slots, cur, end);
+  const int e = blockIdx.x * 128 + threadIdx.x;
+  if (e >= m.n_elems) return;
+  const int4 cn = __ldg(m.conn + e);
+  const int nid[4] = {cn.x, cn.y, cn.z, cn.w};
+  float xv[4][3];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float4 X = __ldg(m.X32 + nid[k]);
+    xv[k][0] = X.x;
+    xv[k][1] = X.y;
+    xv[k][2] = X.z;
+  }
+  TetGeom<float> g;
+  tet_geom(xv[0], xv[1], xv[2], xv[3], g);
+  const DevMat<float>& mat = a.matF[__ldg(m.mat_id + e)];
+  const float scale = __ldg(m.scale + e);
+  float pay[kPay];
+  {
+    const int npay = model_pay_words(MODEL >= 0 ? MODEL : mat.model);
+#pragma unroll
+    for (int k = 0; k < kPay; ++k)
+      pay[k] = (k < npay) ? __ldg(a.payload + (size_t)k * m.n_elems + e) : 0.f;
+  }
+  float w[4][3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    w[1][j] = g.c[0][j];
+    w[2][j] = g.c[1][j];
+    w[3][j] = g.c[2][j];
+    w[0][j] = -(g.c[0][j] + g.c[1][j] + g.c[2][j]);
+  }
+  const int4 sp = __ldg(m.spos + e);
+  const int pos[4] = {sp.x, sp.y, sp.z, sp.w};
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    float v[W];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      float dF[9];
+#pragma unroll
+      for (int k = 0; k < 9; ++k) dF[k] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 3; ++j) dF[3 * i + j] = w[s][j] * g.inv_det;
+      float dP[9];
+      dP_any<MODEL>(mat, scale, pay, dF, dP);
+      if (BLOCK) {
+        // force component k at the slot's node for a unit displacement in
+        // direction i: entries (i, k), k >= i -> 00 01 02 | 11 12 | 22
+#pragma unroll
+        for (int k = i; k < 3; ++k) {
+          const int ent = (i == 0) ? k : (i == 1 ? 2 + k : 5);
+          v[ent] = g.s6 * (dP[3 * k] * w[s][0] + dP[3 * k + 1] * w[s][1] + dP[3 * k + 2] * w[s][2]);
+        }
+      } else {
+        v[i] = g.s6 * (dP[3 * i] * w[s][0] + dP[3 * i + 1] * w[s][1] + dP[3 * i + 2] * w[s][2]);
+      }
+    }
+    __stcg(a.stage + 2 * (size_t)pos[s], make_float4(v[0], v[1], v[2], BLOCK ? v[W - 3] : 0.f));
+    if (BLOCK) __stcg(a.stage + 2 * (size_t)pos[s] + 1, make_float4(v[W - 2], v[W - 1], 0.f, 0.f));
+  }
+}
+
+template <bool BLOCK>
+__global__ void __launch_bounds__(128) diag_gather_kernel(const __grid_constant__ DiagArgs a) {
+  constexpr int W = BLOCK ? 6 : 3, kBatch = BLOCK ? 4 : 8;
+  const MeshDev& m = a.m;
+  const int n = blockIdx.x * 128 + threadIdx.x;
+  if (n >= m.n_nodes) return;
   float acc[W];
 #pragma unroll
   for (int k = 0; k < W; ++k) acc[k] = 0.f;
-  const int e0 = m.blk_ptr[b], e1 = m.blk_ptr[b + 1];
-  for (int c0 = e0; c0 < e1; c0 += NB) {
-    const int idx = c0 + tid;
-    if (idx < e1) {
-      const int e = __ldg(m.blk_elems + idx);
-      const int4 cn = __ldg(m.conn + e);
-      const int nid[4] = {cn.x, cn.y, cn.z, cn.w};
-      float xv[4][3];
+  const int j0 = __ldg(m.node_row + n), j1 = __ldg(m.node_row + n + 1);
+  for (int j = j0; j < j1; j += kBatch) {
+    float4 v[kBatch], w[kBatch];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float4 X = __ldg(m.X32 + nid[k]);
-        xv[k][0] = X.x;
-        xv[k][1] = X.y;
-        xv[k][2] = X.z;
-      }
-      TetGeom<float> g;
-      tet_geom(xv[0], xv[1], xv[2], xv[3], g);
-      const DevMat<float>& mat = a.matF[__ldg(m.mat_id + e)];
-      const float scale = __ldg(m.scale + e);
-      float pay[kPay];
-      {
-        const int npay = model_pay_words(MODEL >= 0 ? MODEL : mat.model);
+    for (int u = 0; u < kBatch; ++u) {
+      const size_t q = 2 * (size_t)min(j + u, j1 - 1);
+      v[u] = __ldcg(a.stage + q);
+      if (BLOCK) w[u] = __ldcg(a.stage + q + 1);
+    }
 #pragma unroll
-        for (int k = 0; k < kPay; ++k)
-          pay[k] = (k < npay) ? __ldg(a.payload + (size_t)k * m.n_elems + e) : 0.f;
-      }
-      float w[4][3];
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        w[1][j] = g.c[0][j];
-        w[2][j] = g.c[1][j];
-        w[3][j] = g.c[2][j];
-        w[0][j] = -(g.c[0][j] + g.c[1][j] + g.c[2][j]);
-      }
-#pragma unroll
-      for (int s = 0; s < 4; ++s) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          float dF[9];
-#pragma unroll
-          for (int k = 0; k < 9; ++k) dF[k] = 0.f;
-#pragma unroll
-          for (int j = 0; j < 3; ++j) dF[3 * i + j] = w[s][j] * g.inv_det;
-          float dP[9];
-          dP_any<MODEL>(mat, scale, pay, dF, dP);
-          if (BLOCK) {
-            // force component k at the slot's node for a unit displacement in
-            // direction i: entries (i, k), k >= i -> 00 01 02 | 11 12 | 22
-#pragma unroll
-            for (int k = i; k < 3; ++k) {
-              const int ent = (i == 0) ? k : (i == 1 ? 2 + k : 5);
-              sf[W * s + ent][tid] =
-                  g.s6 * (dP[3 * k] * w[s][0] + dP[3 * k + 1] * w[s][1] + dP[3 * k + 2] * w[s][2]);
-            }
-          } else {
-            sf[W * s + i][tid] =
-                g.s6 * (dP[3 * i] * w[s][0] + dP[3 * i + 1] * w[s][1] + dP[3 * i + 2] * w[s][2]);
-          }
+    for (int u = 0; u < kBatch; ++u)
+      if (j + u < j1) {
+        acc[0] += v[u].x;
+        acc[1] += v[u].y;
+        acc[2] += v[u].z;
+        if (BLOCK) {
+          acc[W - 3] += v[u].w;
+          acc[W - 2] += w[u].x;
+          acc[W - 1] += w[u].y;
         }
       }
-    }
-    __syncthreads();
-    gather_chunk_w<NB, W>(s_slots, sf, c0 - e0, cur, end, acc);
-    __syncthreads();
   }
-  if (!has_node) return;
-  diag_store<BLOCK>(acc, m.fixed[node], node, a.dinv, a.boff);
+  diag_store<BLOCK>(acc, m.fixed[n], n, a.dinv, a.boff);
 }
 
 // ───────────────────────── PCG vector kernels ─────────────────────────
@@ -1581,28 +1585,15 @@ void prepare_kernels(const MeshDev& m, int model) {
   }
 }
 
-template <int NB, int MODEL>
+template <int MODEL>
 static void diag_go(const DiagArgs& a, cudaStream_t s) {
-  const size_t smem = slots_smem(a.m);
+  const int ge = nblk(a.m.n_elems, 128), gn = nblk(a.m.n_nodes, 128);
   if (a.boff) {
-    allow_smem(diag_kernel<NB, MODEL, true>, smem, s);
-    diag_kernel<NB, MODEL, true><<<a.m.n_blocks, NB, smem, s>>>(a);
-    return;
-  }
-  allow_smem(diag_kernel<NB, MODEL, false>, smem, s);
-  diag_kernel<NB, MODEL, false><<<a.m.n_blocks, NB, smem, s>>>(a);
-}
-
-template <int NB>
-static void diag_nb(const DiagArgs& a, int model, cudaStream_t s) {
-  switch (model) {
-    case M_LE: diag_go<NB, M_LE>(a, s); break;
-    case M_NH: diag_go<NB, M_NH>(a, s); break;
-    case M_MR: diag_go<NB, M_MR>(a, s); break;
-    case M_J2: diag_go<NB, M_J2>(a, s); break;
-    case M_TI: diag_go<NB, M_TI>(a, s); break;
-    case M_FMR: diag_go<NB, M_FMR>(a, s); break;
-    default: diag_go<NB, -1>(a, s); break;
+    diag_elem_kernel<MODEL, true><<<ge, 128, 0, s>>>(a);
+    diag_gather_kernel<true><<<gn, 128, 0, s>>>(a);
+  } else {
+    diag_elem_kernel<MODEL, false><<<ge, 128, 0, s>>>(a);
+    diag_gather_kernel<false><<<gn, 128, 0, s>>>(a);
   }
 }
 
@@ -1611,10 +1602,14 @@ void launch_diag(const DiagArgs& a, int model, cudaStream_t s) {
     launch_diag_hex(a, model, s);
     return;
   }
-  switch (a.m.nb) {
-    case 128: diag_nb<128>(a, model, s); break;
-    case 512: diag_nb<512>(a, model, s); break;
-    default: diag_nb<256>(a, model, s); break;
+  switch (model) {
+    case M_LE: diag_go<M_LE>(a, s); break;
+    case M_NH: diag_go<M_NH>(a, s); break;
+    case M_MR: diag_go<M_MR>(a, s); break;
+    case M_J2: diag_go<M_J2>(a, s); break;
+    case M_TI: diag_go<M_TI>(a, s); break;
+    case M_FMR: diag_go<M_FMR>(a, s); break;
+    default: diag_go<-1>(a, s); break;
   }
 }
 
