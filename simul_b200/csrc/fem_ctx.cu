@@ -1044,6 +1044,14 @@ int ensure_assembled(FemCtx* c) {
   return FEM_OK;
 }
 
+// The residual kernels have written the tangent payload: the assembled blocks
+// belong to the old one.  (Linear models have no payload: their blocks stay
+// those of the materials.)
+void new_payload(FemCtx* c) {
+  c->tangent_valid = true;
+  if (c->model_kind != M_LE && c->model_kind != M_TI) c->asm_valid = false;
+}
+
 // fneg_out: the negative internal force in caller order (may be null).
 // rnorm2: ||R||^2; null: neither read back nor waited for.
 int eval_residual(FemCtx* c, double* fneg_out, double* rnorm2) {
@@ -1071,9 +1079,7 @@ int eval_residual(FemCtx* c, double* fneg_out, double* rnorm2) {
     CK(cudaMemcpyAsync(c->h_scalars, c->scalars, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
   }
-  c->tangent_valid = true;
-  // linear models have no tangent payload: their blocks stay those of the materials
-  if (c->model_kind != M_LE && c->model_kind != M_TI) c->asm_valid = false;
+  new_payload(c);
   if (rnorm2) *rnorm2 = c->h_scalars[0];
   return FEM_OK;
 }
@@ -3400,7 +3406,7 @@ int fem_profile_kernels(void* ctx, int32_t reps, double* ms_out) {
     CK(cudaEventElapsedTime(&ms, e0, e1));
     ms_out[k] = ms / reps;
   }
-  c->tangent_valid = true;
+  new_payload(c);
   return FEM_OK;
 }
 
