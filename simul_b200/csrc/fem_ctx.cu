@@ -1086,8 +1086,11 @@ int eval_residual(FemCtx* c, double* fneg_out, double* rnorm2) {
 
 // Jacobi scaling for the PCG solve: 1 / diag(K_T), or with `block` the
 // nodal 3 x 3 block inverse (diagonal in dinv, off-diagonals in boff).
-int compute_dinv(FemCtx* c, int precond, bool block = false) {
-  if (precond == FEM_PRECOND_JACOBI && c->asm_valid && c->mv_variant == MV_ASSEMBLED) {
+// `assembled`: from the assembled blocks, for a solve that runs on them.  The
+// two forms differ in rounding, so what is returned to a caller (the network's
+// output) is always built on the element pass.
+int compute_dinv(FemCtx* c, int precond, bool block = false, bool assembled = false) {
+  if (precond == FEM_PRECOND_JACOBI && assembled) {
     ++c->n_launches; launch_asm_diag(asm_args(c), c->dinv, block ? c->boff : nullptr, c->stream);
     CKL();
   } else if (precond == FEM_PRECOND_JACOBI) {
@@ -2186,7 +2189,9 @@ int run_pcg(FemCtx* c, const double* b_int, int precond, double rtol, int maxit,
     return set_err(c, FEM_ERR_STATE, "learned preconditioner has no weights (fem_mpnn_set_weights)");
   if ((st = choose_matvec_variant(c, !learned))) return st;
   if (c->mv_variant == MV_ASSEMBLED && (st = ensure_assembled(c))) return st;
-  if ((st = compute_dinv(c, (tl || learned) ? FEM_PRECOND_JACOBI : precond, tl && c->block_jacobi))) return st;
+  if ((st = compute_dinv(c, (tl || learned) ? FEM_PRECOND_JACOBI : precond, tl && c->block_jacobi,
+                         c->mv_variant == MV_ASSEMBLED)))
+    return st;
   if (tl && (st = ensure_coarse(c))) {
     // no positive definite coarse operator on this lattice yet (e.g. cells
     // finer than the elements of an anisotropic mesh): this solve runs as
@@ -2916,7 +2921,9 @@ int fem_batch_solve(void** ctxs, int32_t n, const FemSolveParams* prm, int32_t l
     if (learned && !c->mpnn_has_weights) return set_err(c, FEM_ERR_STATE, "learned preconditioner has no weights");
     if ((st = choose_matvec_variant(c, !learned))) return st;
     if (c->mv_variant == MV_ASSEMBLED && (st = ensure_assembled(c))) return st;
-    if ((st = compute_dinv(c, (tl || learned) ? FEM_PRECOND_JACOBI : p.precond, tl && c->block_jacobi))) return st;
+    if ((st = compute_dinv(c, (tl || learned) ? FEM_PRECOND_JACOBI : p.precond, tl && c->block_jacobi,
+                           c->mv_variant == MV_ASSEMBLED)))
+      return st;
     if ((tl || (learned && c->learned_coarse)) && (st = ensure_coarse(c))) return st;
     if (learned && (st = ensure_mpnn(c))) return st;
     const int kind = learned ? GRAPH_LEARNED : (tl ? GRAPH_TWO_LEVEL : GRAPH_JACOBI);

@@ -57,3 +57,18 @@ def test_solve_after_profiling_uses_the_new_tangent(cuda, element):
     ms = (C.c_double * 4)()
     assert lib.fem_profile_kernels(mesh.ctx, 1, ms) == 0
     assert _residual(mesh, _solve(mesh, r), r) < 1e-4
+
+
+def test_network_output_does_not_depend_on_an_earlier_solve(cuda):
+    from simul_b200 import learned
+    mesh, _, r = _plastic_body(cuda, "tet4")
+    learned.set_weights(mesh, learned.init_weights(seed=2, out_scale=0.2))
+    x = r.to(torch.float32)
+    z = []
+    for solve_first in (False, True):
+        if solve_first:
+            _solve(mesh, r)
+            assert mesh.stats()["matvec_variant"] == "assembled"
+        z.append(torch.empty_like(x))
+        assert _lib.load().fem_mpnn_forward(mesh.ctx, B._ptr(x), B._ptr(z[-1])) == 0
+    assert torch.equal(z[0], z[1])
