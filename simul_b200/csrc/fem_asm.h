@@ -2,6 +2,8 @@
 #pragma once
 #include <algorithm>
 #include <cstdint>
+#include <exception>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -12,16 +14,33 @@ namespace femb200 {
 // A CTA of the persistent solve takes at least this many rows (two warps').
 constexpr int kAsmMinRows = 64;
 
-// f(begin, end) over [0, n) on up to 16 host threads, `grain` or more each
+// f(begin, end) over [0, n) on up to 16 host threads, `grain` or more each.  A
+// thread that cannot be had leaves its range to the caller's; an exception of
+// any range is thrown here once all have ended.
 template <typename F>
 void parallel_ranges(int n, F f, int grain = 1024) {
   const int hw = std::max(1, (int)std::thread::hardware_concurrency());
   const int nt = std::max(1, std::min(std::min(hw, 16), n / grain));
+  std::vector<std::exception_ptr> err(nt);
+  auto part = [&](int t) {
+    try {
+      f((int)((int64_t)n * t / nt), (int)((int64_t)n * (t + 1) / nt));
+    } catch (...) {
+      err[t] = std::current_exception();
+    }
+  };
   std::vector<std::thread> pool;
-  for (int t = 1; t < nt; ++t)
-    pool.emplace_back([=] { f((int)((int64_t)n * t / nt), (int)((int64_t)n * (t + 1) / nt)); });
-  f(0, (int)((int64_t)n / nt));
+  pool.reserve(nt);
+  int started = 1;
+  try {
+    for (; started < nt; ++started) pool.emplace_back(part, started);
+  } catch (const std::system_error&) {
+  }
+  part(0);
+  for (int t = started; t < nt; ++t) part(t);
   for (auto& th : pool) th.join();
+  for (auto& e : err)
+    if (e) std::rethrow_exception(e);
 }
 
 struct AsmHost {

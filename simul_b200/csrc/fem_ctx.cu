@@ -44,6 +44,9 @@ inline int step_chunks(int n_nodes) { return (n_nodes + kStepThreads - 1) / kSte
 
 constexpr int kMvRule = -2;
 
+// device buffers and their sizes
+using TableBufs = std::vector<std::pair<void*, size_t>>;
+
 struct FemCtx {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -225,11 +228,12 @@ struct FemCtx {
   // warp-aggregated two-phase matvec tables (TET4; built when selected or timed)
   WaggDev wadev{};
   std::vector<void*> wa_bufs;
-  // assembled tangent: tables built on the first PCG solve that uses it
+  // assembled tangent: tables built on the first PCG solve that uses it.  They
+  // are optional: without them the solves run as the kernel chain
   AsmDev asmdev{};
-  std::vector<void*> asm_bufs;
+  TableBufs asm_bufs;
   bool asm_built = false;
-  bool asm_refused = false;   // the mesh does not fit the format
+  bool asm_refused = false;   // the mesh does not fit the format, or the tables the memory
   bool asm_valid = false;     // the values belong to the current tangent state
   // persistent PCG kernel (fem_pcg.cu): tables per matrix and per coarse
   // lattice; chain_forced: an option of the kernel chain was set, so the
@@ -239,8 +243,9 @@ struct FemCtx {
   std::vector<int> asm_prefix;         // steps of the first slices (shared-memory plan)
   bool pcg_coarse_built = false;
   bool chain_forced = false;
-  bool pcg_ok = true;         // a refused plan or launch turns it off
-  std::vector<void*> pcg_coarse_bufs;
+  bool pcg_ok[2] = {true, true};  // Jacobi, two-level: a refused plan or launch turns it off
+  TableBufs pcg_coarse_bufs;
+  TableBufs pcg_inv_bufs;     // the coarse inverse in the kernel's forms
   double* pcg_part = nullptr;
   unsigned int* pcg_bar = nullptr;
   float* pcg_p2 = nullptr;    // second buffer of the direction
@@ -323,10 +328,73 @@ int set_err(FemCtx* c, int code, const char* fmt, ...) {
                      cudaGetErrorString(e__), __FILE__, __LINE__);                        \
   } while (0)
 
+void free_tables(FemCtx* c, TableBufs& bufs) {
+  for (auto& b : bufs) {
+    cudaFree(b.first);
+    c->bytes -= b.second;
+  }
+  bufs.clear();
+}
+
+// Gives the optional tables of the persistent solve back (cudaFree waits for
+// the kernels that read them).
+void release_pcg_coarse(FemCtx* c) {
+  free_tables(c, c->pcg_coarse_bufs);
+  c->pcg_coarse_built = false;
+  c->pcgdev = PcgDev{};
+}
+
+void release_inverse_forms(FemCtx* c) {
+  free_tables(c, c->pcg_inv_bufs);
+  c->cdev.full_ld = 0;
+  c->cdev.Afull16 = nullptr;
+  c->cdev.Afull32 = c->cdev.Ainv32t = nullptr;
+}
+
+void release_asm(FemCtx* c) {
+  release_pcg_coarse(c);
+  free_tables(c, c->asm_bufs);
+  c->asmdev = AsmDev{};
+  c->pcg_part = nullptr;
+  c->pcg_bar = nullptr;
+  c->pcg_p2 = nullptr;
+  c->asm_built = c->asm_valid = false;
+}
+
+// cudaMalloc of what a call cannot do without: where the memory is short, the
+// context's optional tables make room and its solves run as the kernel chain.
+cudaError_t malloc_required(FemCtx* c, void** ptr, size_t bytes) {
+  cudaError_t e = cudaMalloc(ptr, bytes);
+  if (e == cudaErrorMemoryAllocation && c->asm_built) {
+    cudaGetLastError();
+    release_asm(c);
+    release_inverse_forms(c);
+    c->asm_refused = true;
+    e = cudaMalloc(ptr, bytes);
+  }
+  if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // reported here, not by the next launch
+  return e;
+}
+
+// A buffer of optional tables, zeroed, or false (no error is left behind).
+template <typename T>
+bool table_alloc(FemCtx* c, TableBufs& bufs, T** ptr, size_t count) {
+  const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
+  void* p = nullptr;
+  if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  bufs.push_back({p, bytes});
+  c->bytes += bytes;
+  *ptr = static_cast<T*>(p);
+  return cudaMemsetAsync(p, 0, bytes, c->stream) == cudaSuccess;
+}
+
 template <typename T>
 int dalloc(FemCtx* c, T** ptr, size_t count) {
   size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
-  cudaError_t e = cudaMalloc(reinterpret_cast<void**>(ptr), bytes);
+  cudaError_t e = malloc_required(c, reinterpret_cast<void**>(ptr), bytes);
   if (e != cudaSuccess)
     return set_err(c, FEM_ERR_CUDA, "cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
   c->bytes += bytes;
@@ -373,10 +441,9 @@ void free_ctx(FemCtx* c) {
     if (p) cudaFree(p);
   for (void* p : c->wa_bufs)
     if (p) cudaFree(p);
-  for (void* p : c->asm_bufs)
-    if (p) cudaFree(p);
-  for (void* p : c->pcg_coarse_bufs)
-    if (p) cudaFree(p);
+  for (auto& b : c->asm_bufs) cudaFree(b.first);
+  for (auto& b : c->pcg_coarse_bufs) cudaFree(b.first);
+  for (auto& b : c->pcg_inv_bufs) cudaFree(b.first);
   if (c->h_err) cudaFreeHost(c->h_err);
   if (c->dense_work) cudaFree(c->dense_work);
   if (c->dense_info) cudaFree(c->dense_info);
@@ -930,18 +997,9 @@ AsmArgs asm_args(const FemCtx* c) {
   return a;
 }
 
-template <typename T>
-int asm_upload(FemCtx* c, T** dst, const T* src, size_t n) {
-  int st;
-  if ((st = dalloc(c, dst, n))) return st;
-  c->asm_bufs.push_back(*dst);
-  if (src && n) CK(cudaMemcpyAsync(*dst, src, n * sizeof(T), cudaMemcpyHostToDevice, c->stream));
-  return FEM_OK;
-}
-
-// Tables of the assembled tangent; asm_refused where the mesh does not fit.
-int ensure_asm_tables(FemCtx* c) {
-  if (c->asm_built || c->asm_refused) return FEM_OK;
+// Tables of the assembled tangent; asm_refused where the mesh does not fit the
+// format.  *room = false where the device memory does not hold them.
+int build_asm_tables(FemCtx* c, bool* room) {
   const size_t cw = (size_t)c->npe / 4;
   std::vector<int4> conn(cw * c->Ne);
   CK(cudaMemcpyAsync(conn.data(), c->conn, conn.size() * sizeof(int4), cudaMemcpyDeviceToHost, c->stream));
@@ -953,26 +1011,31 @@ int ensure_asm_tables(FemCtx* c) {
     c->asm_refused = true;
     return FEM_OK;
   }
-  int st;
   AsmDev& S = c->asmdev;
   uint32_t* words = nullptr;
-  auto up = [&](auto** dst, const auto& v) { return asm_upload(c, dst, v.data(), v.size()); };
+  *room = false;  // until all of them are there
+  auto up = [&](auto** dst, const auto& v) {
+    return table_alloc(c, c->asm_bufs, dst, v.size()) &&
+           (v.empty() || cudaMemcpyAsync(*dst, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, c->stream) ==
+                             cudaSuccess);
+  };
   int *cta_row = nullptr, *cta_slice = nullptr, *slice_step = nullptr, *slice_rows = nullptr, *halo_ptr = nullptr,
       *halo = nullptr;
   uint2* edges = nullptr;
   uint32_t *eptr = nullptr, *list = nullptr;
-  if ((st = up(&cta_row, h.cta_row)) || (st = up(&cta_slice, h.cta_slice)) || (st = up(&slice_step, h.slice_step)) ||
-      (st = up(&slice_rows, h.slice_rows)) || (st = up(&halo_ptr, h.halo_ptr)) || (st = up(&halo, h.halo)))
-    return st;
+  if (!up(&cta_row, h.cta_row) || !up(&cta_slice, h.cta_slice) || !up(&slice_step, h.slice_step) ||
+      !up(&slice_rows, h.slice_rows) || !up(&halo_ptr, h.halo_ptr) || !up(&halo, h.halo))
+    return FEM_OK;
   const size_t n_edges = h.erow.back(), n_list = h.lrow.back();
-  if ((st = asm_upload(c, &edges, (const uint2*)nullptr, n_edges)) ||
-      (st = asm_upload(c, &eptr, (const uint32_t*)nullptr, n_edges + 1)) ||
-      (st = asm_upload(c, &list, (const uint32_t*)nullptr, n_list)))
-    return st;
-  if ((st = asm_upload(c, &words, (const uint32_t*)nullptr, (size_t)h.slice_step.back() * kAsmStepWords))) return st;
-  if ((st = asm_upload(c, &c->pcg_part, (const double*)nullptr, 4 * (size_t)h.grid))) return st;
-  if ((st = asm_upload(c, &c->pcg_bar, (const unsigned int*)nullptr, (size_t)1))) return st;
-  if ((st = asm_upload(c, &c->pcg_p2, (const float*)nullptr, 4 * (size_t)c->Nn))) return st;
+  auto table = [&](auto** dst, size_t n) { return table_alloc(c, c->asm_bufs, dst, n); };
+  if (!table(&edges, n_edges) || !table(&eptr, n_edges + 1) || !table(&list, n_list) ||
+      !table(&words, (size_t)h.slice_step.back() * kAsmStepWords) || !table(&c->pcg_part, 4 * (size_t)h.grid) ||
+      !table(&c->pcg_bar, 1) || !table(&c->pcg_p2, 4 * (size_t)c->Nn))
+    return FEM_OK;
+  uint32_t* hpos = nullptr;
+  if (c->npe == 8 &&
+      (!table(&hpos, 32 * (size_t)c->Ne) || !table(&S.hblk4, 2 * n_list) || !table(&S.hblk1, n_list)))
+    return FEM_OK;
   S.grid = h.grid;
   S.n_slices = (int)h.slice_step.size() - 1;
   S.n_edges = (int)n_edges;
@@ -995,7 +1058,10 @@ int ensure_asm_tables(FemCtx* c) {
   // the lists the device derives the rest from, for that only
   uint32_t* tmp = nullptr;
   const size_t nr = h.row.size(), nc = h.cols.size(), nn = (size_t)c->Nn;
-  CK(cudaMalloc(reinterpret_cast<void**>(&tmp), (3 * nr + nc + nn) * sizeof(uint32_t)));
+  if (cudaMalloc(reinterpret_cast<void**>(&tmp), (3 * nr + nc + nn) * sizeof(uint32_t)) != cudaSuccess) {
+    cudaGetLastError();
+    return FEM_OK;
+  }
   cudaError_t e = cudaSuccess;
   size_t at = 0;
   auto put = [&](const void* src, size_t n) {
@@ -1019,19 +1085,31 @@ int ensure_asm_tables(FemCtx* c) {
   cudaFree(tmp);
   CK(e);
   if (c->npe == 8) {
-    uint32_t* hpos = nullptr;
-    if ((st = asm_upload(c, &hpos, (const uint32_t*)nullptr, 32 * (size_t)c->Ne)) ||
-        (st = asm_upload(c, &S.hblk4, (const float4*)nullptr, 2 * n_list)) ||
-        (st = asm_upload(c, &S.hblk1, (const float*)nullptr, n_list)))
-      return st;
     CK(cudaMemsetAsync(hpos, 0xff, 32 * sizeof(uint32_t) * (size_t)c->Ne, c->stream));  // kNoPlace
     launch_asm_hex_places(list, n_list, hpos, c->stream);
     CKL();
     S.hpos = hpos;
   }
-  c->asm_built = true;
+  c->asm_built = *room = true;
   c->asm_valid = false;
   return FEM_OK;
+}
+
+int ensure_asm_tables(FemCtx* c) {
+  if (c->asm_built || c->asm_refused) return FEM_OK;
+  bool room = true;
+  int st = FEM_OK;
+  try {
+    st = build_asm_tables(c, &room);
+  } catch (const std::exception&) {  // host memory or threads
+    room = false;
+  }
+  if (st || !room) {
+    cudaStreamSynchronize(c->stream);
+    release_asm(c);
+    c->asm_refused = true;
+  }
+  return st;
 }
 
 // The assembled blocks at the current tangent state.
@@ -1234,11 +1312,11 @@ CGState endless_cg() {
 // when fem_set_option set it; unless the option asks for timing, the
 // assembled product in the persistent PCG kernel for a plain solve (`plain`:
 // not the learned preconditioner, no option of the kernel chain set) of a
-// TET4 mesh that fits it, and the persistent element pass else; with timing,
-// the fastest of the element variants on this mesh, timed with CUDA events as
-// they run inside CG (3 warm-up + 10 timed launches each, p = 1 on free
-// DOFs).  The CG state is reset by cg_init afterwards.
-int choose_matvec_variant(FemCtx* c, bool plain) {
+// mesh that fits it, and the persistent element pass else (HEX8: its only
+// one); with timing, the fastest of the element variants on this mesh, timed
+// with CUDA events as they run inside CG (3 warm-up + 10 timed launches each,
+// p = 1 on free DOFs).  The CG state is reset by cg_init afterwards.
+int choose_matvec_variant(FemCtx* c, bool plain, bool two_level) {
   int st;
   if (c->npe == 8 && c->mv_forced != kMvRule) {
     // of the element passes HEX8 has the two-phase one only
@@ -1255,7 +1333,7 @@ int choose_matvec_variant(FemCtx* c, bool plain) {
   if (c->mv_forced == kMvRule) {
     // (a batch of several workers overlaps its contexts' chains: one
     // persistent kernel at a time took 196 ms where eight chains take 150)
-    plain = plain && !c->chain_forced && c->pcg_ok && !c->in_batch;
+    plain = plain && !c->chain_forced && c->pcg_ok[two_level] && !c->in_batch;
     if (plain && (st = ensure_asm_tables(c))) return st;
     c->mv_variant = plain && c->asm_built ? MV_ASSEMBLED : (c->npe == 8 ? MV_TWO_PHASE : MV_PERSIST);
     return FEM_OK;
@@ -1379,10 +1457,9 @@ int drop_coarse(FemCtx* c) {
   for (void* p : c->coarse_bufs)
     if (p) cudaFree(p);
   c->coarse_bufs.clear();
-  for (void* p : c->pcg_coarse_bufs)
-    if (p) cudaFree(p);
-  c->pcg_coarse_bufs.clear();
-  c->pcg_coarse_built = false;
+  release_pcg_coarse(c);
+  release_inverse_forms(c);
+  c->pcg_ok[1] = true;  // another lattice may fit
   c->cdev = CoarseDev{};
   c->coarse_have_inverse = false;
   c->tl_part = nullptr;
@@ -1407,7 +1484,7 @@ void invalidate_coarse(FemCtx* c) { c->coarse_valid = false; }
 
 int ensure_cg_graph(FemCtx* c, int kind) {
   int st;
-  if ((st = choose_matvec_variant(c, false))) return st;
+  if ((st = choose_matvec_variant(c, false, false))) return st;
   const bool fused = use_fused(c, kind);
   const bool pdl = use_pdl(c, kind);
   const int flags = (kind == GRAPH_LEARNED ? (c->learned_coarse ? 1 : 0) : 0) | (fused ? 2 : 0) | (pdl ? 4 : 0) |
@@ -1696,19 +1773,22 @@ int build_coarse(FemCtx* c) {
   } else {
     if ((st = coarse_alloc(c, &cd.Ainv, nd * nd))) return st;
   }
-  // the persistent solve reads full rows up to 16 MB: they come from L2 in
-  // about the time that adding up the packed tiles' two products takes
-  const size_t ld = (nd + 7) / 8 * 8, full = nd * ld * (c->coarse_bf16 ? 2 : 4);
-  cd.full_ld = full <= (16u << 20) ? (int)ld : 0;
-  if (cd.full_ld && c->coarse_bf16 && (st = coarse_alloc(c, &cd.Afull16, nd * ld))) return st;
-  if (cd.full_ld && !c->coarse_bf16 && (st = coarse_alloc(c, &cd.Afull32, nd * ld))) return st;
-  if (!cd.full_ld && !c->coarse_bf16 && (st = coarse_alloc(c, &cd.Ainv32t, nb * (nb + 1) / 2 * 4096))) return st;
   cd.r_slices = coarse_restrict_slices(n_cells);
   if ((st = coarse_alloc(c, &cd.cell_r, (size_t)n_cells * cd.r_slices * 24))) return st;
   if ((st = coarse_alloc(c, &cd.yc, nb * 64))) return st;
   if ((st = coarse_alloc(c, &cd.rc, nb * 64))) return st;
   // fused two-level step: per (cell, slice) restriction and ||r||^2 shares
   if ((st = coarse_alloc(c, &c->tl_part, (size_t)n_cells * cd.r_slices + step_chunks(Nn)))) return st;
+  // the persistent solve reads full rows up to 16 MB: they come from L2 in
+  // about the time that adding up the packed tiles' two products takes.
+  // Optional: without its form of the inverse it is refused (run_persistent)
+  const size_t ld = (nd + 7) / 8 * 8, full = nd * ld * (c->coarse_bf16 ? 2 : 4);
+  const bool rows = full <= (16u << 20);
+  bool have = true;
+  if (rows && c->coarse_bf16) have = table_alloc(c, c->pcg_inv_bufs, &cd.Afull16, nd * ld);
+  if (rows && !c->coarse_bf16) have = table_alloc(c, c->pcg_inv_bufs, &cd.Afull32, nd * ld);
+  if (!rows && !c->coarse_bf16) have = table_alloc(c, c->pcg_inv_bufs, &cd.Ainv32t, nb * (nb + 1) / 2 * 4096);
+  cd.full_ld = rows && have ? (int)ld : 0;
   CK(cudaStreamSynchronize(c->stream));
   c->coarse_H = H;
   c->coarse_built = true;
@@ -1765,7 +1845,7 @@ int ensure_coarse(FemCtx* c) {
     if (c->dense_work) cudaFree(c->dense_work);
     c->dense_work = nullptr;
     c->dense_bytes = 0;
-    CK(cudaMalloc(&c->dense_work, work));
+    CK(malloc_required(c, &c->dense_work, work));
     c->dense_bytes = work;
   }
   if (!c->dense_info) CK(cudaMalloc(reinterpret_cast<void**>(&c->dense_info), sizeof(int)));
@@ -2004,63 +2084,78 @@ void mpnn_sample(FemCtx* c, const float* R, const float* E, int k, bool coarse, 
 
 // ───────────────────────── persistent PCG ─────────────────────────
 
-template <typename T>
-int pcg_upload(FemCtx* c, std::vector<void*>& bufs, const T** dst, const std::vector<T>& v) {
-  T* d = nullptr;
-  int st;
-  if ((st = dalloc(c, &d, v.size()))) return st;
-  bufs.push_back(d);
-  if (!v.empty()) CK(cudaMemcpyAsync(d, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, c->stream));
-  *dst = d;
-  return FEM_OK;
-}
-
-int ensure_pcg_tables(FemCtx* c, bool two_level) {
-  int st;
+// Tables of the two-level phases; *fit = false where they do not fit the
+// format or the device memory.
+int build_pcg_coarse(FemCtx* c, bool* fit) {
   PcgDev& t = c->pcgdev;
-  if (!two_level || c->pcg_coarse_built) return FEM_OK;
+  *fit = false;
+  if (!c->cdev.full_ld && !c->cdev.Ainv16 && !c->cdev.Ainv32t) return FEM_OK;
   std::vector<int> node_cell(c->Nn), corner(8 * (size_t)c->cdev.n_cells);
   CK(cudaMemcpyAsync(node_cell.data(), c->cdev.node_cell, node_cell.size() * sizeof(int), cudaMemcpyDeviceToHost,
                      c->stream));
   CK(cudaMemcpyAsync(corner.data(), c->cdev.cell_corner, corner.size() * sizeof(int), cudaMemcpyDeviceToHost,
                      c->stream));
-  CK(cudaStreamSynchronize(c->stream));
   std::vector<int> halo_ptr(c->asm_cta_row.size());
-  CK(cudaMemcpy(halo_ptr.data(), c->asmdev.halo_ptr, halo_ptr.size() * sizeof(int), cudaMemcpyDeviceToHost));
+  CK(cudaMemcpyAsync(halo_ptr.data(), c->asmdev.halo_ptr, halo_ptr.size() * sizeof(int), cudaMemcpyDeviceToHost,
+                     c->stream));
+  CK(cudaStreamSynchronize(c->stream));
   std::vector<int> halo((size_t)halo_ptr.back());
   if (!halo.empty())
-    CK(cudaMemcpy(halo.data(), c->asmdev.halo, halo.size() * sizeof(int), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpyAsync(halo.data(), c->asmdev.halo, halo.size() * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
   PcgCoarseHost h;
   if (!pcg_coarse_tables(c->asm_cta_row, halo_ptr, halo, node_cell, corner, c->cdev.n_cn,
-                         c->cdev.full_ld ? 0 : (c->cdev.Ainv16 ? 2 : 4), &h)) {
-    c->pcg_ok = false;
+                         c->cdev.full_ld ? 0 : (c->cdev.Ainv16 ? 2 : 4), &h))
     return FEM_OK;
-  }
   auto& bufs = c->pcg_coarse_bufs;
+  auto up = [&](auto** dst, const auto& v) {
+    std::remove_const_t<std::remove_pointer_t<std::remove_reference_t<decltype(*dst)>>>* d = nullptr;
+    if (!table_alloc(c, bufs, &d, v.size())) return false;
+    *dst = d;
+    return v.empty() ||
+           cudaMemcpyAsync(d, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, c->stream) == cudaSuccess;
+  };
   const int* seg_rows = nullptr;
   float4* lat = nullptr;
-  if ((st = pcg_upload(c, bufs, &t.tab_ptr, h.tab_ptr))) return st;
-  if ((st = pcg_upload(c, bufs, &t.tab, h.tab))) return st;
-  if ((st = pcg_upload(c, bufs, &seg_rows, h.seg_rows))) return st;
-  if ((st = pcg_upload(c, bufs, &t.col_corners, h.col_corners))) return st;
-  if ((st = pcg_upload(c, bufs, &t.cn_ptr, h.cn_ptr))) return st;
-  t.merged = c->cdev.full_ld && 8 * h.n_seg <= kPcgMergedShares;
-  if ((st = dalloc(c, &lat, (size_t)c->Nn))) return st;
-  bufs.push_back(lat);
-  launch_pcg_seg_lat(seg_rows, c->cdev.node_lat, c->Nn, lat, c->stream);
-  CKL();
-  t.seg_lat = lat;
-  if ((st = dalloc(c, &t.seg_r, 8 * (size_t)h.n_seg))) return st;
-  bufs.push_back(t.seg_r);
-  if ((st = dalloc(c, &t.ypart, 64 * (size_t)h.n_parts))) return st;
-  bufs.push_back(t.ypart);
-  t.max_tab = h.max_tab;
-  t.max_lblk = h.max_lblk;
-  t.max_loc = h.max_loc;
-  t.max_tiles = h.max_tiles;
+  bool room = up(&t.tab_ptr, h.tab_ptr) && up(&t.tab, h.tab) && up(&seg_rows, h.seg_rows) &&
+              up(&t.col_corners, h.col_corners) && up(&t.cn_ptr, h.cn_ptr) &&
+              table_alloc(c, bufs, &lat, (size_t)c->Nn) && table_alloc(c, bufs, &t.seg_r, 8 * (size_t)h.n_seg) &&
+              table_alloc(c, bufs, &t.ypart, 64 * (size_t)h.n_parts);
+  if (room) {
+    t.merged = c->cdev.full_ld && 8 * h.n_seg <= kPcgMergedShares;
+    launch_pcg_seg_lat(seg_rows, c->cdev.node_lat, c->Nn, lat, c->stream);
+    t.seg_lat = lat;
+    t.max_tab = h.max_tab;
+    t.max_lblk = h.max_lblk;
+    t.max_loc = h.max_loc;
+    t.max_tiles = h.max_tiles;
+  }
   CK(cudaStreamSynchronize(c->stream));  // the host tables go out of scope
-  c->pcg_coarse_built = true;
+  CKL();
+  c->pcg_coarse_built = *fit = room;
   return FEM_OK;
+}
+
+// This kind of solve runs as the kernel chain from now on; the other kind
+// builds its tables again if it is asked for.
+void refuse_persistent(FemCtx* c, bool two_level) {
+  c->pcg_ok[two_level] = false;
+  release_asm(c);
+  if (two_level) release_inverse_forms(c);
+}
+
+int ensure_pcg_tables(FemCtx* c, bool two_level) {
+  if (!two_level || c->pcg_coarse_built) return FEM_OK;
+  bool fit = true;
+  int st = FEM_OK;
+  try {
+    st = build_pcg_coarse(c, &fit);
+  } catch (const std::exception&) {  // host memory or threads
+    cudaStreamSynchronize(c->stream);
+    fit = false;
+  }
+  if (st || !fit) refuse_persistent(c, two_level);
+  return st;
 }
 
 // One launch at a time on a device: the kernel fills the GPU and its CTAs
@@ -2075,8 +2170,9 @@ std::mutex& pcg_mutex(int device) {
 int run_persistent(FemCtx* c, const double* b_int, bool two_level, double rtol, int maxit, bool* ran) {
   int st;
   *ran = false;
+  if (!c->asm_built) return FEM_OK;  // another table of this solve took the memory
   if ((st = ensure_pcg_tables(c, two_level))) return st;
-  if (!c->pcg_ok) return FEM_OK;
+  if (!c->pcg_ok[two_level]) return FEM_OK;
   PcgArgs a;
   std::memset(&a, 0, sizeof(a));
   a.m = c->mesh();
@@ -2099,7 +2195,7 @@ int run_persistent(FemCtx* c, const double* b_int, bool two_level, double rtol, 
   a.max_iter = maxit;
   size_t smem = 0;
   if (!pcg_plan(a, two_level, c->asm_prefix, &smem)) {
-    c->pcg_ok = false;
+    refuse_persistent(c, two_level);
     return FEM_OK;
   }
   CK(cudaMemsetAsync(c->pcg_bar, 0, sizeof(unsigned int), c->stream));
@@ -2107,7 +2203,7 @@ int run_persistent(FemCtx* c, const double* b_int, bool two_level, double rtol, 
   const cudaError_t e = launch_pcg(a, two_level, smem, c->stream);
   if (e != cudaSuccess) {
     cudaGetLastError();
-    c->pcg_ok = false;
+    refuse_persistent(c, two_level);
     return FEM_OK;
   }
   ++c->n_launches;
@@ -2187,7 +2283,7 @@ int run_pcg(FemCtx* c, const double* b_int, int precond, double rtol, int maxit,
   const int kind = learned ? GRAPH_LEARNED : (tl ? GRAPH_TWO_LEVEL : GRAPH_JACOBI);
   if (learned && !c->mpnn_has_weights)
     return set_err(c, FEM_ERR_STATE, "learned preconditioner has no weights (fem_mpnn_set_weights)");
-  if ((st = choose_matvec_variant(c, !learned))) return st;
+  if ((st = choose_matvec_variant(c, !learned, tl))) return st;
   if (c->mv_variant == MV_ASSEMBLED && (st = ensure_assembled(c))) return st;
   if ((st = compute_dinv(c, (tl || learned) ? FEM_PRECOND_JACOBI : precond, tl && c->block_jacobi,
                          c->mv_variant == MV_ASSEMBLED)))
@@ -2919,7 +3015,7 @@ int fem_batch_solve(void** ctxs, int32_t n, const FemSolveParams* prm, int32_t l
     const bool tl = p.precond == FEM_PRECOND_TWO_LEVEL;
     const bool learned = p.precond == FEM_PRECOND_LEARNED;
     if (learned && !c->mpnn_has_weights) return set_err(c, FEM_ERR_STATE, "learned preconditioner has no weights");
-    if ((st = choose_matvec_variant(c, !learned))) return st;
+    if ((st = choose_matvec_variant(c, !learned, tl))) return st;
     if (c->mv_variant == MV_ASSEMBLED && (st = ensure_assembled(c))) return st;
     if ((st = compute_dinv(c, (tl || learned) ? FEM_PRECOND_JACOBI : p.precond, tl && c->block_jacobi,
                            c->mv_variant == MV_ASSEMBLED)))
@@ -2927,8 +3023,8 @@ int fem_batch_solve(void** ctxs, int32_t n, const FemSolveParams* prm, int32_t l
     if ((tl || (learned && c->learned_coarse)) && (st = ensure_coarse(c))) return st;
     if (learned && (st = ensure_mpnn(c))) return st;
     const int kind = learned ? GRAPH_LEARNED : (tl ? GRAPH_TWO_LEVEL : GRAPH_JACOBI);
-    if (c->mv_variant == MV_ASSEMBLED && (st = ensure_pcg_tables(c, tl))) return st;
-    if ((c->mv_variant != MV_ASSEMBLED || !c->pcg_ok) && (st = ensure_cg_graph(c, kind))) return st;
+    if (c->mv_variant == MV_ASSEMBLED && c->asm_built && (st = ensure_pcg_tables(c, tl))) return st;
+    if ((c->mv_variant != MV_ASSEMBLED || !c->asm_built) && (st = ensure_cg_graph(c, kind))) return st;
   }
   std::atomic<int> next{0};
   auto work = [&]() {
