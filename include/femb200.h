@@ -156,10 +156,12 @@ int fem_ctx_stats(void* ctx, int64_t* out18);
 /* Option keys of fem_set_option (no reference counterpart: the reference has
  * one matvec formulation, backend/fea/fem/material/nonlinear/base.py:110-145). */
 enum {
-  /* not set (default): plain TET4 solves run as one persistent kernel on the
-   * assembled tangent (stats variant 5) where the mesh fits it, everything
-   * else with variant 4; -1: time the element variants on the first PCG solve
-   * and keep the fastest; 0: fused node-block kernel; 1: element pass writing
+  /* -2 (default): Jacobi and two-level solves run as one persistent kernel on
+   * the assembled tangent (stats variant 5) where the mesh and the memory hold
+   * its tables and no option asks for the kernel chain, everything else with
+   * variant 4 (HEX8: 1); setting it also drops an earlier request for the
+   * chain and tries again what was refused; -1: time the element variants on
+   * the first PCG solve and keep the fastest; 0: fused node-block kernel; 1: element pass writing
    * slot vectors in node order plus a node gather; 2 (TET4): element-block
    * kernel that sums each block's slot vectors in shared memory, nodes
    * shared by blocks completed by a second kernel; 3 (TET4): the two-phase
@@ -189,22 +191,25 @@ enum {
   /* 1: the CG work after each matvec (update, restriction, coarse product,
    * preconditioner, direction) runs as one cooperative kernel with grid-wide
    * barriers, where the runtime accepts it in a graph; 0 (default): as a
-   * chain of kernels.  Jacobi and two-level; batched solves use the chain. */
+   * chain of kernels.  Jacobi and two-level; batched solves use the chain.
+   * Setting 1 asks for the kernel chain until FEM_OPT_MATVEC_VARIANT = -2. */
   FEM_OPT_FUSED_STEP = 6,
-  /* 1 (default): a PCG solve runs as one graph launch (a conditional WHILE
-   * node) where it does not run as the persistent kernel; 0: as launches of fixed 12- or 32-iteration graphs with a host
-   * check between them (kernel profilers cannot attribute kernels inside
-   * conditional graphs) */
+  /* 1 (default): a PCG solve of the kernel chain runs as one graph launch (a
+   * conditional WHILE node); 0, which selects the chain: as launches of fixed
+   * 12- or 32-iteration graphs with a host check between them (kernel
+   * profilers cannot attribute kernels inside conditional graphs) */
   FEM_OPT_WHOLE_SOLVE_GRAPH = 7,
   /* 1 (default): inside the captured CG graphs each kernel of the iteration
    * chain is launched as a programmatic dependent of the previous one (it is
    * scheduled while the previous one drains and waits for its results on the
-   * device), where the runtime accepts it; 0: plain stream order */
+   * device), where the runtime accepts it; 0: plain stream order.  Setting
+   * either value asks for the chain until FEM_OPT_MATVEC_VARIANT = -2. */
   FEM_OPT_PDL = 8,
   /* 1 (default): two-level PCG with the two-phase matvec applies the matvec
    * to z and forms the direction in its node gather by recurrence,
    * p = z + beta p and K p = K z + beta K p_old, saving the direction-update
-   * kernel; 0: p = z + beta p in its own kernel, then K p */
+   * kernel; 0, which selects the kernel chain: p = z + beta p in its own
+   * kernel, then K p */
   FEM_OPT_DIRECTION_RECURRENCE = 9,
   /* two-level preconditioner smoother: 1 (default) the inverse of each
    * node's 3 x 3 diagonal block of K_T (free DOFs), 0 the inverse of the

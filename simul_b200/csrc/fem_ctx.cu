@@ -235,14 +235,13 @@ struct FemCtx {
   bool asm_built = false;
   bool asm_refused = false;   // the mesh does not fit the format, or the tables the memory
   bool asm_valid = false;     // the values belong to the current tangent state
-  // persistent PCG kernel (fem_pcg.cu): tables per matrix and per coarse
-  // lattice; chain_forced: an option of the kernel chain was set, so the
-  // solves run as that chain
+  // persistent PCG kernel (fem_pcg.cu): tables per matrix and per coarse lattice
   PcgDev pcgdev{};
   std::vector<int> asm_cta_row;        // first row of each CTA
   std::vector<int> asm_prefix;         // steps of the first slices (shared-memory plan)
   bool pcg_coarse_built = false;
-  bool chain_forced = false;
+  bool chain_asked = false;      // by the fused step or programmatic launches; the rule's option value lifts it
+  bool loop_graph_off = false;   // whole-solve graphs switched off by option
   bool pcg_ok[2] = {true, true};  // Jacobi, two-level: a refused plan or launch turns it off
   TableBufs pcg_coarse_bufs;
   TableBufs pcg_inv_bufs;     // the coarse inverse in the kernel's forms
@@ -1308,6 +1307,12 @@ CGState endless_cg() {
   return hs;
 }
 
+// An option of the kernel chain stands at another value than its default, or
+// the chain was asked for: the solves run as that chain.
+bool chain_forced(const FemCtx* c) {
+  return c->chain_asked || c->fused_step || c->loop_graph_off || !c->direction_recurrence || !c->pdl;
+}
+
 // Picks the matvec variant for the current material tables: the forced one
 // when fem_set_option set it; unless the option asks for timing, the
 // assembled product in the persistent PCG kernel for a plain solve (`plain`:
@@ -1333,7 +1338,7 @@ int choose_matvec_variant(FemCtx* c, bool plain, bool two_level) {
   if (c->mv_forced == kMvRule) {
     // (a batch of several workers overlaps its contexts' chains: one
     // persistent kernel at a time took 196 ms where eight chains take 150)
-    plain = plain && !c->chain_forced && c->pcg_ok[two_level] && !c->in_batch;
+    plain = plain && !chain_forced(c) && c->pcg_ok[two_level] && !c->in_batch;
     if (plain && (st = ensure_asm_tables(c))) return st;
     c->mv_variant = plain && c->asm_built ? MV_ASSEMBLED : (c->npe == 8 ? MV_TWO_PHASE : MV_PERSIST);
     return FEM_OK;
@@ -2524,10 +2529,10 @@ int fem_set_option(void* ctx, int32_t key, int64_t value) {
   if ((st = check_ctx(c))) return st;
   switch (key) {
     case FEM_OPT_MATVEC_VARIANT:
-      if (value < -1 || value >= MV_N_VARIANTS)
+      if (value < kMvRule || value >= MV_N_VARIANTS)
         return set_err(c, FEM_ERR_INVALID,
-                       "matvec variant %lld not in {-1 (auto), 0 (fused), 1 (two-phase), 2 (element-block), "
-                       "3 (warp-aggregated), 4 (persistent two-phase)}",
+                       "matvec variant %lld not in {-2 (the default rule), -1 (timed), 0 (fused), 1 (two-phase), "
+                       "2 (element-block), 3 (warp-aggregated), 4 (persistent two-phase)}",
                        (long long)value);
       if (value == MV_ELEM_BLOCK && c->npe != 4)
         return set_err(c, FEM_ERR_INVALID, "the element-block matvec is TET4 only");
@@ -2539,8 +2544,12 @@ int fem_set_option(void* ctx, int32_t key, int64_t value) {
       if (value == MV_ELEM_BLOCK && (st = build_eb_tables(c, c->eb_forced > 0 ? c->eb_forced : 512))) return st;
       if (value == MV_WARP_AGG && (st = build_wagg_tables(c))) return st;
       c->mv_forced = (int)value;
-      c->mv_variant = value >= 0 ? (int)value : MV_FUSED;
+      c->mv_variant = value >= 0 ? (int)value : (value == kMvRule ? MV_PERSIST : MV_FUSED);
       c->mv_tuned = false;
+      if (value == kMvRule) {  // as in a new context: also what was refused is tried again
+        c->chain_asked = c->asm_refused = false;
+        c->pcg_ok[0] = c->pcg_ok[1] = true;
+      }
       return FEM_OK;
     case FEM_OPT_EXTRAPOLATE:
       if (value != 0 && value != 1) return set_err(c, FEM_ERR_INVALID, "extrapolation flag must be 0 or 1");
@@ -2592,7 +2601,7 @@ int fem_set_option(void* ctx, int32_t key, int64_t value) {
         }
         c->use_loop_graph = value != 0;
       }
-      if (value == 0) c->chain_forced = true;
+      c->loop_graph_off = value == 0;
       return FEM_OK;
     case FEM_OPT_COARSE_MAX_NODES:
       if (value < 8 || value > kMaxCoarseNodesLimit)
@@ -2614,17 +2623,16 @@ int fem_set_option(void* ctx, int32_t key, int64_t value) {
     case FEM_OPT_DIRECTION_RECURRENCE:
       if (value != 0 && value != 1) return set_err(c, FEM_ERR_INVALID, "direction recurrence flag must be 0 or 1");
       c->direction_recurrence = value != 0;
-      c->chain_forced = true;
       return FEM_OK;
     case FEM_OPT_PDL:
       if (value != 0 && value != 1) return set_err(c, FEM_ERR_INVALID, "programmatic launch flag must be 0 or 1");
       c->pdl = value != 0;
-      c->chain_forced = true;
+      c->chain_asked = true;
       return FEM_OK;
     case FEM_OPT_FUSED_STEP:
       if (value != 0 && value != 1) return set_err(c, FEM_ERR_INVALID, "fused step flag must be 0 or 1");
       c->fused_step = value != 0;
-      c->chain_forced = true;
+      if (value != 0) c->chain_asked = true;
       return FEM_OK;
     case FEM_OPT_COARSE_REUSE:
       if (value < -1 || value > (1 << 20))

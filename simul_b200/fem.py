@@ -219,26 +219,32 @@ class FEMesh:
             _check(lib.fem_set_option(self.ctx, _lib.FEM_OPT_COARSE_REUSE, int(reuse)), self.ctx, "fem_set_option")
 
     def set_fused_step(self, on: bool):
-        """Runs the CG work after each matvec as one cooperative kernel (True)
-        or as a chain of kernels (False, the default)."""
+        """Runs the CG work after each matvec of the kernel chain as one
+        cooperative kernel (True) or as single kernels (False, the default).
+        True asks for the chain in place of the persistent PCG kernel, until
+        ``set_matvec_variant("auto")``."""
         _check(_lib.load().fem_set_option(self.ctx, _lib.FEM_OPT_FUSED_STEP, 1 if on else 0), self.ctx,
                "fem_set_option")
 
     def set_whole_solve_graph(self, on: bool):
-        """One graph launch per PCG solve (True, the default) or fixed-size
-        iteration graphs with a host check between them (False; kernel
-        profilers cannot see inside the conditional graph)."""
+        """Solves of the kernel chain: one graph launch per PCG solve (True, the
+        default) or fixed-size iteration graphs with a host check between them
+        (False, which selects the chain; kernel profilers cannot see inside the
+        conditional graph)."""
         _check(_lib.load().fem_set_option(self.ctx, _lib.FEM_OPT_WHOLE_SOLVE_GRAPH, 1 if on else 0), self.ctx,
                "fem_set_option")
 
     def set_programmatic_launch(self, on: bool):
-        """Programmatic dependent launches between the CG iteration's kernels
-        inside the captured graphs (True, the default) or plain stream order."""
+        """Programmatic dependent launches between the kernels of the chain's
+        captured CG iterations (True, as the chain has them unless this is
+        called) or plain stream order.  Either value asks for the chain in
+        place of the persistent PCG kernel, until ``set_matvec_variant("auto")``."""
         _check(_lib.load().fem_set_option(self.ctx, _lib.FEM_OPT_PDL, 1 if on else 0), self.ctx, "fem_set_option")
 
     def set_direction_recurrence(self, on: bool):
-        """Two-level PCG: form the search direction by recurrence inside the
-        matvec's node gather (True, the default) or in its own kernel."""
+        """Two-level PCG as the kernel chain: form the search direction by
+        recurrence inside the matvec's node gather (True, the default) or in its
+        own kernel (False, which selects the chain)."""
         _check(_lib.load().fem_set_option(self.ctx, _lib.FEM_OPT_DIRECTION_RECURRENCE, 1 if on else 0), self.ctx,
                "fem_set_option")
 
@@ -258,12 +264,13 @@ class FEMesh:
     def set_matvec_variant(self, variant, block_size=None):
         """Forces the tangent-matvec variant ("fused", "two_phase",
         "element_block", "warp_agg", "persistent") or times them on the next
-        solve and keeps the fastest (None).  Where it is never called, plain
-        TET4 solves run as one persistent kernel on the assembled tangent and
-        all others with "persistent".  ``block_size``
+        solve and keeps the fastest (None).  "auto", the state of a new mesh:
+        Jacobi and two-level solves run as one persistent kernel on the
+        assembled tangent, all else with "persistent" (HEX8: "two_phase").
+        ``block_size``
         fixes the element-block variant's elements per block (256, 512, 768
         or 1024; 0: timed; None: unchanged)."""
-        code = {None: -1, "fused": 0, "two_phase": 1, "element_block": 2, "warp_agg": 3, "persistent": 4}[variant]
+        code = {"auto": -2, None: -1, "fused": 0, "two_phase": 1, "element_block": 2, "warp_agg": 3, "persistent": 4}[variant]
         lib = _lib.load()
         if block_size is not None:
             _check(lib.fem_set_option(self.ctx, _lib.FEM_OPT_EB_SIZE, int(block_size)), self.ctx, "fem_set_option")
