@@ -1307,6 +1307,25 @@ CGState endless_cg() {
   return hs;
 }
 
+// Solves under way on a device (fem_pcg, fem_newton_solve), of all contexts.
+std::atomic<int>& solves_under_way(int device) {
+  static std::atomic<int> n[64];
+  return n[device & 63];
+}
+
+struct SolveUnderWay {
+  std::atomic<int>& n;
+  explicit SolveUnderWay(const FemCtx* c) : n(solves_under_way(c->device)) { ++n; }
+  ~SolveUnderWay() { --n; }
+};
+
+// Above this many solves under way on a device (each from a thread of its own)
+// a solve runs as the kernel chain: chains of several contexts overlap, the
+// persistent kernel takes the whole GPU for one.  Five load steps of 32-voxel
+// bodies, one after another against overlapping: two 6.7 and 7.1 ms, three 8.9
+// and 7.6, eight 22.0 and 15.4.
+constexpr int kPersistSolves = 2;
+
 // An option of the kernel chain stands at another value than its default, or
 // the chain was asked for: the solves run as that chain.
 bool chain_forced(const FemCtx* c) {
@@ -1316,8 +1335,8 @@ bool chain_forced(const FemCtx* c) {
 // Picks the matvec variant for the current material tables: the forced one
 // when fem_set_option set it; unless the option asks for timing, the
 // assembled product in the persistent PCG kernel for a plain solve (`plain`:
-// not the learned preconditioner, no option of the kernel chain set) of a
-// mesh that fits it, and the persistent element pass else (HEX8: its only
+// not the learned preconditioner, no option of the kernel chain set, not one
+// of many at once) of a mesh that fits it, and the persistent element pass else (HEX8: its only
 // one); with timing, the fastest of the element variants on this mesh, timed
 // with CUDA events as they run inside CG (3 warm-up + 10 timed launches each,
 // p = 1 on free DOFs).  The CG state is reset by cg_init afterwards.
@@ -1338,7 +1357,8 @@ int choose_matvec_variant(FemCtx* c, bool plain, bool two_level) {
   if (c->mv_forced == kMvRule) {
     // (a batch of several workers overlaps its contexts' chains: one
     // persistent kernel at a time took 196 ms where eight chains take 150)
-    plain = plain && !chain_forced(c) && c->pcg_ok[two_level] && !c->in_batch;
+    plain = plain && !chain_forced(c) && c->pcg_ok[two_level] && !c->in_batch &&
+            solves_under_way(c->device) <= kPersistSolves;
     if (plain && (st = ensure_asm_tables(c))) return st;
     c->mv_variant = plain && c->asm_built ? MV_ASSEMBLED : (c->npe == 8 ? MV_TWO_PHASE : MV_PERSIST);
     return FEM_OK;
@@ -3220,6 +3240,7 @@ int fem_pcg(void* ctx, int32_t precond, const double* r, double* du, double rtol
   if (maxit <= 0 || !(rtol > 0)) return set_err(c, FEM_ERR_INVALID, "need max_iterations > 0 and rtol > 0");
   if (precond < FEM_PRECOND_NONE || precond > FEM_PRECOND_LEARNED)
     return set_err(c, FEM_ERR_INVALID, "unknown preconditioner %d", precond);
+  const SolveUnderWay under_way(c);
   // caller order -> internal order, fixed DOFs of the right-hand side zeroed
   ++c->n_launches; launch_gather_d_masked(r, c->tmpd, c->d_perm_node, c->fixed, c->Nn, c->stream);
   CKL();
@@ -3263,6 +3284,7 @@ int fem_newton_solve(void* ctx, const FemSolveParams* prm_in, FemSolveResult* re
     return set_err(c, FEM_ERR_INVALID, "need max_iterations > 0 and tol > 0");
   if (prm.precond < FEM_PRECOND_NONE || prm.precond > FEM_PRECOND_LEARNED)
     return set_err(c, FEM_ERR_INVALID, "unknown preconditioner %d", prm.precond);
+  const SolveUnderWay under_way(c);
   FemSolveResult out;
   std::memset(&out, 0, sizeof(out));
   // Load-step extrapolation (FEM_OPT_EXTRAPOLATE): when the last solve
