@@ -31,174 +31,203 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <mutex>
 
 #include "fem_asm.h"
 
 namespace femb200 {
 
-// ───────────────────────── tables (host) ─────────────────────────
+// ───────────────────────── tables ─────────────────────────
+//
+// The first solve of a context pays for them, so the neighbour lists, halos,
+// columns and edge lists are derived on the device and the host only deals out
+// the rows: 2.0 ms at 74,600 hexes, where the neighbours and halos on the host
+// took 16 ms with sixteen cores and 67 with one, more than a whole solve.
 
-bool build_asm_host(const int4* conn4, int Nn, int Ne, int npe, int sms, AsmHost* out) {
-  const int* conn = &conn4[0].x;
-  // node -> (element, vertex), elements ascending
-  std::vector<int> arow(Nn + 1, 0);
-  for (int64_t i = 0; i < (int64_t)npe * Ne; ++i) arow[conn[i] + 1]++;
-  for (int i = 0; i < Nn; ++i) arow[i + 1] += arow[i];
-  std::vector<uint32_t> acol(arow[Nn]);
-  {
-    std::vector<int> fill(arow.begin(), arow.end() - 1);
-    for (int e = 0; e < Ne; ++e)
-      for (int k = 0; k < npe; ++k) acol[fill[conn[(size_t)npe * e + k]]++] = (uint32_t)e * npe + k;
-  }
-  // neighbours of each node (ascending), edges to higher nodes and the
-  // (element, vertex pair) lists of those edges: count, then fill
-  std::vector<int64_t> nrow(Nn + 1, 0), erow(Nn + 1, 0), lrow(Nn + 1, 0);
-  struct Part {
-    int a0;
-    std::vector<int> cols;
-  };
-  std::vector<Part> found;  // the neighbours, by the threads' runs of nodes
-  std::mutex mu;
-  parallel_ranges(Nn, [&](int a0, int a1) {
-    Part p{a0, {}};
-    p.cols.reserve((size_t)(a1 - a0) * (npe == 8 ? 27 : 15));
-    // (rows are short: scanning the ones found so far beats sorting all repeats)
-    for (int a = a0; a < a1; ++a) {
-      const size_t base = p.cols.size();
-      int64_t l = 0;
-      for (int j = arow[a]; j < arow[a + 1]; ++j) {
-        const int* cn = conn + (size_t)npe * (acol[j] / npe);
-        for (int k = 0; k < npe; ++k) {
-          const int b = cn[k];
-          if (b == a) continue;
-          l += b > a;
-          size_t q = base;
-          while (q < p.cols.size() && p.cols[q] != b) ++q;
-          if (q == p.cols.size()) p.cols.push_back(b);
-        }
-      }
-      std::sort(p.cols.begin() + base, p.cols.end());
-      nrow[a + 1] = (int64_t)(p.cols.size() - base);
-      erow[a + 1] = p.cols.end() - std::upper_bound(p.cols.begin() + base, p.cols.end(), a);
-      lrow[a + 1] = l;
-    }
-    std::lock_guard<std::mutex> lock(mu);
-    found.push_back(std::move(p));
-  });
-  for (int a = 0; a < Nn; ++a) {
-    nrow[a + 1] += nrow[a];
-    erow[a + 1] += erow[a];
-    lrow[a + 1] += lrow[a];
-  }
-  const int64_t nnz = nrow[Nn];
-  if (nnz > 0x7fffffffLL || lrow[Nn] > 0x7fffffffLL || (uint64_t)Ne * npe * npe > 0xffffffffULL) return false;
-  out->cols.resize((size_t)nnz);
-  out->row.assign(nrow.begin(), nrow.end());
-  parallel_ranges((int)found.size(), [&](int p0, int p1) {
-    for (int p = p0; p < p1; ++p)
-      std::copy(found[p].cols.begin(), found[p].cols.end(), out->cols.begin() + nrow[found[p].a0]);
-  }, 1);
-  // runs of rows with equal entries (a row counts as 4 more) per CTA
-  const int G = std::max(1, std::min(sms, Nn / kAsmMinRows));
+void asm_cta_rows(const std::vector<int>& deg, int sms, AsmHost* out) {
+  const int Nn = (int)deg.size(), G = std::max(1, std::min(sms, Nn / kAsmMinRows));
   out->grid = G;
   out->cta_row.assign(G + 1, Nn);
   out->cta_row[0] = 0;
-  {
-    const int64_t total = nnz + 4 * (int64_t)Nn;
-    int g = 1;
-    for (int a = 0; a < Nn && g < G; ++a)
-      while (g < G && (nrow[a + 1] + 4 * (int64_t)(a + 1)) * G >= total * g) out->cta_row[g++] = a + 1;
-    // at least one row each
-    for (int k = 1; k < G; ++k) out->cta_row[k] = std::max(out->cta_row[k], out->cta_row[k - 1] + 1);
-    for (int k = G - 1; k > 0; --k) out->cta_row[k] = std::min(out->cta_row[k], out->cta_row[k + 1] - 1);
+  // runs of rows with equal entries (a row counts as 4 more) per CTA
+  int64_t total = 4 * (int64_t)Nn, at = 0;
+  for (int d : deg) total += d;
+  int g = 1;
+  for (int a = 0; a < Nn && g < G; ++a) {
+    at += deg[a] + 4;
+    while (g < G && at * G >= total * g) out->cta_row[g++] = a + 1;
   }
-  // slices; halos
-  std::vector<uint32_t>& slot0 = out->slot0;
-  slot0.assign(Nn, 0u);
-  std::vector<std::vector<int>> halo(G), order(G);
-  parallel_ranges(G, [&](int g0, int g1) {
-    for (int g = g0; g < g1; ++g) {
-      const int r0 = out->cta_row[g], r1 = out->cta_row[g + 1];
-      for (int64_t j = nrow[r0]; j < nrow[r1]; ++j)
-        if (out->cols[j] < r0 || out->cols[j] >= r1) halo[g].push_back(out->cols[j]);
-      std::sort(halo[g].begin(), halo[g].end());
-      halo[g].erase(std::unique(halo[g].begin(), halo[g].end()), halo[g].end());
-      for (int r = r0; r < r1; ++r) order[g].push_back(r);
-      std::stable_sort(order[g].begin(), order[g].end(),
-                       [&](int a, int b) { return nrow[a + 1] - nrow[a] > nrow[b + 1] - nrow[b]; });
-    }
-  }, 1);
+  // at least one row each
+  for (int k = 1; k < G; ++k) out->cta_row[k] = std::max(out->cta_row[k], out->cta_row[k - 1] + 1);
+  for (int k = G - 1; k > 0; --k) out->cta_row[k] = std::min(out->cta_row[k], out->cta_row[k + 1] - 1);
+}
+
+bool asm_slices(const std::vector<int>& deg, AsmHost* out) {
+  const int Nn = (int)deg.size(), G = out->grid;
+  constexpr int kWarps = kPcgThreads / 32;
+  out->slot0.assign(Nn, 0u);
   out->cta_slice.assign(1, 0);
   out->slice_step.assign(1, 0);
-  out->halo_ptr.assign(1, 0);
-  std::vector<std::vector<int>> csteps(G);
+  out->slice_rows.reserve((size_t)Nn + 32 * (size_t)G);
+  std::vector<int> order, first, prefix(1, 0);
   int64_t steps = 0;
   for (int g = 0; g < G; ++g) {
-    const int rows = (int)order[g].size();
-    csteps[g].push_back(0);
-    for (int i = 0; i < rows; i += 32) {
-      const int deg = (int)(nrow[order[g][i] + 1] - nrow[order[g][i]]);
+    const int r0 = out->cta_row[g], r1 = out->cta_row[g + 1], rows = r1 - r0;
+    // longest rows first, else in their order
+    int lo = deg[r0], hi = deg[r0];
+    for (int r = r0; r < r1; ++r) {
+      lo = std::min(lo, deg[r]);
+      hi = std::max(hi, deg[r]);
+    }
+    first.assign(hi - lo + 2, 0);
+    for (int r = r0; r < r1; ++r) ++first[hi - deg[r] + 1];
+    for (size_t k = 1; k < first.size(); ++k) first[k] += first[k - 1];
+    order.resize(rows);
+    for (int r = r0; r < r1; ++r) order[first[hi - deg[r]]++] = r;
+    const int64_t step0 = steps;
+    int pieces[kWarps] = {}, n = 0;
+    for (int i = 0; i < rows; i += 32, ++n) {
+      const int d = deg[order[i]];
       for (int l = 0; l < 32; ++l) {
-        const int r = i + l < rows ? order[g][i + l] : -1;
+        const int r = i + l < rows ? order[i + l] : -1;
         out->slice_rows.push_back(r);
-        if (r >= 0) slot0[r] = (uint32_t)(steps * 32 + l);
+        if (r >= 0) out->slot0[r] = (uint32_t)(steps * 32 + l);
       }
-      steps += deg;
+      steps += d;
       if (steps >= (1LL << 27)) return false;
       out->slice_step.push_back((int)steps);
-      csteps[g].push_back(csteps[g].back() + deg);
+      if ((int)prefix.size() == n + 1) prefix.push_back(prefix.back());
+      prefix[n + 1] = std::max(prefix[n + 1], (int)(steps - step0));
+      pieces[n % kWarps] += (d + kPcgPiece - 1) / kPcgPiece;
     }
     out->cta_slice.push_back((int)out->slice_step.size() - 1);
-    out->max_slices = std::max(out->max_slices, (int)csteps[g].size() - 1);
-    out->max_halo = std::max(out->max_halo, (int)halo[g].size());
-    out->max_cols = std::max(out->max_cols, rows + (int)halo[g].size());
-    out->halo.insert(out->halo.end(), halo[g].begin(), halo[g].end());
-    out->halo_ptr.push_back((int)out->halo.size());
+    out->max_slices = std::max(out->max_slices, n);
+    for (int w : pieces) out->max_pieces = std::max(out->max_pieces, w);
+    for (size_t k = n + 1; k < prefix.size(); ++k) prefix[k] = std::max(prefix[k], (int)(steps - step0));
   }
-  for (int g = 0; g < G; ++g) {
-    constexpr int kWarps = kPcgThreads / 32;
-    int n[kWarps] = {};
-    for (size_t k = 0; k + 1 < csteps[g].size(); ++k)
-      n[k % kWarps] += (csteps[g][k + 1] - csteps[g][k] + kPcgPiece - 1) / kPcgPiece;
-    for (int w : n) out->max_pieces = std::max(out->max_pieces, w);
-  }
-  if (out->max_cols > 65536) return false;
-  out->prefix.assign(out->max_slices + 1, 0);
-  for (int g = 0; g < G; ++g)
-    for (int k = 0; k <= out->max_slices; ++k)
-      out->prefix[k] = std::max(out->prefix[k], csteps[g][std::min(k, (int)csteps[g].size() - 1)]);
-  out->erow.assign(erow.begin(), erow.end());
-  out->lrow.assign(lrow.begin(), lrow.end());
+  out->prefix = prefix;
   return true;
 }
 
+// A warp per node: the other vertices of its elements, each at the place that
+// the smaller ones and the earlier equal ones leave it, then without repeats.
+template <int SH>
+__global__ void __launch_bounds__(128) asm_neighbours_kernel(const MeshDev m, int* cand, int* cols, int* counts) {
+  constexpr int kN = 1 << SH, kOther = kN - 1;
+  constexpr unsigned kFull = 0xffffffffu;
+  const int a = blockIdx.x * 4 + ((int)threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (a >= m.n_nodes) return;
+  const int s0 = m.node_row[a], ns = m.node_row[a + 1] - s0, n = ns * kOther;
+  const int base = m.blk_ptr[a / m.nb];
+  cand += (size_t)s0 * kOther;
+  cols += (size_t)s0 * kOther;
+  for (int j = lane; j < ns; j += 32) {
+    const uint32_t code = m.node_slots[s0 + j];
+    const int la = (int)(code & (uint32_t)kOther);
+    const int* cn = reinterpret_cast<const int*>(m.conn) + kN * (size_t)m.blk_elems[base + (int)(code >> SH)];
+#pragma unroll
+    for (int k = 0; k < kN; ++k)
+      if (k != la) cand[kOther * j + (k < la ? k : k - 1)] = cn[k];
+  }
+  __syncwarp();
+  for (int i = lane; i < n; i += 32) {
+    const int v = cand[i];
+    int at = 0;
+    for (int j = 0; j < n; ++j) {
+      const int w = cand[j];
+      at += w < v || (w == v && j < i);
+    }
+    cols[at] = v;
+  }
+  __syncwarp();
+  int deg = 0, up = 0, len = 0, carry = -1;
+  for (int c = 0; c < n; c += 32) {
+    const bool in = c + lane < n;
+    const int v = in ? cols[c + lane] : -1;
+    int prev = __shfl_up_sync(kFull, v, 1);
+    if (lane == 0) prev = carry;
+    carry = __shfl_sync(kFull, v, 31);
+    const bool first = in && v != prev;
+    const unsigned mask = __ballot_sync(kFull, first);
+    if (first) cols[deg + __popc(mask & ((1u << lane) - 1u))] = v;  // (below the next chunk)
+    deg += __popc(mask);
+    up += __popc(__ballot_sync(kFull, first && v > a));
+    len += __popc(__ballot_sync(kFull, in && v > a));
+    __syncwarp();
+  }
+  if (lane == 0) {
+    counts[a] = deg;
+    counts[m.n_nodes + a] = up;
+    counts[2 * (size_t)m.n_nodes + a] = len;
+  }
+}
+
+// The halo of one CTA of the solve: its rows' columns outside its run, marked.
+__global__ void __launch_bounds__(256) asm_halo_mark_kernel(const MeshDev m, const __grid_constant__ AsmLists t,
+                                                            const int* cta_row, uint32_t* bits0, uint32_t* bits1,
+                                                            int* count) {
+  __shared__ int s_n;
+  const int g = blockIdx.x, r0 = cta_row[g], r1 = cta_row[g + 1], words = (m.n_nodes + 31) / 32;
+  uint32_t* bits = (g & 1 ? bits1 : bits0) + (size_t)(g >> 1) * words;
+  if (threadIdx.x == 0) s_n = 0;
+  for (int r = r0 + (int)threadIdx.x; r < r1; r += 256) {
+    const int* c = t.cols + (size_t)m.node_row[r] * (m.npe - 1);
+    const int deg = t.deg[r];
+    for (int k = 0; k < deg; ++k) {
+      const int n = c[k];
+      if (n < r0 || n >= r1) atomicOr(bits + (n >> 5), 1u << (n & 31));
+    }
+  }
+  __syncthreads();
+  int n = 0;
+  for (int w = threadIdx.x; w < words; w += 256) n += __popc(__ldcg(bits + w));
+  atomicAdd(&s_n, n);
+  __syncthreads();
+  if (threadIdx.x == 0) count[g] = s_n;
+}
+
+// ... and listed: each thread a run of words, after the marks of the runs before it.
+__global__ void __launch_bounds__(256) asm_halo_list_kernel(int n_nodes, const uint32_t* bits0,
+                                                            const uint32_t* bits1, const int* halo_ptr, int* halo) {
+  __shared__ int s_n[256];
+  const int g = blockIdx.x, tid = threadIdx.x, words = (n_nodes + 31) / 32;
+  const uint32_t* bits = (g & 1 ? bits1 : bits0) + (size_t)(g >> 1) * words;
+  const int w0 = (int)((int64_t)words * tid / 256), w1 = (int)((int64_t)words * (tid + 1) / 256);
+  int n = 0;
+  for (int w = w0; w < w1; ++w) n += __popc(bits[w]);
+  s_n[tid] = n;
+  __syncthreads();
+  int at = halo_ptr[g];
+  for (int k = 0; k < tid; ++k) at += s_n[k];
+  for (int w = w0; w < w1; ++w)
+    for (uint32_t b = bits[w]; b; b &= b - 1u) halo[at++] = 32 * w + __ffs((int)b) - 1;
+}
+
 // Edges to higher nodes, their slots and their (element, vertex pair) lists,
-// a thread per node: the elements on the node in its slot order.  (On the host
-// this took a third of the tables' time, and its upload as long as the rest.)
+// a thread per node: the elements on the node in its slot order.
 template <int SH>
 __global__ void __launch_bounds__(128) asm_list_kernel(const MeshDev m, const __grid_constant__ AsmLists t, uint2* edges,
                                                        uint32_t* eptr, uint32_t* list) {
   const int a = blockIdx.x * 128 + threadIdx.x;
   if (a >= m.n_nodes) return;
   constexpr int kN = 1 << SH;
-  const int j0 = t.row[a], deg = t.row[a + 1] - j0;
+  const int s0 = m.node_row[a], s1 = m.node_row[a + 1], deg = t.deg[a];
+  const int* ca = t.cols + (size_t)s0 * (kN - 1);
   const uint32_t e0 = t.erow[a], ne = t.erow[a + 1] - e0;
   uint32_t l = t.lrow[a];
   const int up = deg - (int)ne;
-  const int base = m.blk_ptr[a / m.nb], s0 = m.node_row[a], s1 = m.node_row[a + 1];
+  const int base = m.blk_ptr[a / m.nb];
   for (uint32_t q = 0; q < ne; ++q) {
-    const int b = t.cols[j0 + up + (int)q];
-    int lo = t.row[b], hi = t.row[b + 1];
-    const int b0 = lo;
+    const int b = ca[up + (int)q];
+    const int* cb = t.cols + (size_t)m.node_row[b] * (kN - 1);
+    int lo = 0, hi = t.deg[b];
     while (lo < hi) {
       const int mid = (lo + hi) >> 1;
-      if (t.cols[mid] < a)
+      if (cb[mid] < a)
         lo = mid + 1;
       else
         hi = mid;
     }
-    edges[e0 + q] = make_uint2(t.slot0[a] + 32u * (uint32_t)(up + (int)q), t.slot0[b] + 32u * (uint32_t)(lo - b0));
+    edges[e0 + q] = make_uint2(t.slot0[a] + 32u * (uint32_t)(up + (int)q), t.slot0[b] + 32u * (uint32_t)lo);
     eptr[e0 + q] = l;
     for (int j = s0; j < s1; ++j) {
       const uint32_t code = m.node_slots[j];
@@ -213,16 +242,17 @@ __global__ void __launch_bounds__(128) asm_list_kernel(const MeshDev m, const __
 }
 
 // Local columns of the steps; one CTA per CTA of the solve, a warp per slice.
-__global__ void __launch_bounds__(512) asm_fill_kernel(const __grid_constant__ AsmDev S, const int* row, const int* cols) {
+__global__ void __launch_bounds__(512) asm_fill_kernel(const MeshDev m, const __grid_constant__ AsmDev S,
+                                                       const __grid_constant__ AsmLists t) {
   const int g = blockIdx.x, lane = threadIdx.x & 31, r0 = S.cta_row[g], r1 = S.cta_row[g + 1];
   const int* halo = S.halo + S.halo_ptr[g];
   const int nh = S.halo_ptr[g + 1] - S.halo_ptr[g];
   for (int s = S.cta_slice[g] + ((int)threadIdx.x >> 5); s < S.cta_slice[g + 1]; s += 16) {
-    const int r = S.slice_rows[32 * (size_t)s + lane];
-    const int j0 = r >= 0 ? row[r] : 0, deg = r >= 0 ? row[r + 1] - j0 : 0;
+    const int r = S.slice_rows[32 * (size_t)s + lane], deg = r >= 0 ? t.deg[r] : 0;
+    const int* c = t.cols + (r >= 0 ? (size_t)m.node_row[r] * (m.npe - 1) : 0);
     const int t0 = S.slice_step[s], t1 = S.slice_step[s + 1];
-    for (int t = t0; t < t1; ++t) {
-      const int n = t - t0 < deg ? cols[j0 + t - t0] : r;  // padding: the row itself
+    for (int k = t0; k < t1; ++k) {
+      const int n = k - t0 < deg ? c[k - t0] : r;  // padding: the row itself
       int l = n < 0 ? 0 : n - r0;
       if (n >= 0 && (n < r0 || n >= r1)) {
         int lo = 0, hi = nh;
@@ -235,7 +265,7 @@ __global__ void __launch_bounds__(512) asm_fill_kernel(const __grid_constant__ A
         }
         l = r1 - r0 + lo;
       }
-      reinterpret_cast<uint16_t*>(S.words + (size_t)t * kAsmStepWords)[lane] = (uint16_t)l;
+      reinterpret_cast<uint16_t*>(S.words + (size_t)k * kAsmStepWords)[lane] = (uint16_t)l;
     }
   }
 }
@@ -337,6 +367,24 @@ __global__ void __launch_bounds__(128) asm_diag_kernel(const __grid_constant__ A
 
 // ───────────────────────── launchers ─────────────────────────
 
+void launch_asm_neighbours(const MeshDev& m, int* cand, int* cols, int* counts, cudaStream_t s) {
+  const int g = (m.n_nodes + 3) / 4;
+  if (m.npe == 8)
+    asm_neighbours_kernel<3><<<g, 128, 0, s>>>(m, cand, cols, counts);
+  else
+    asm_neighbours_kernel<2><<<g, 128, 0, s>>>(m, cand, cols, counts);
+}
+
+void launch_asm_halo_mark(const MeshDev& m, const AsmLists& t, const int* cta_row, int grid, uint32_t* bits0,
+                          uint32_t* bits1, int* count, cudaStream_t s) {
+  asm_halo_mark_kernel<<<grid, 256, 0, s>>>(m, t, cta_row, bits0, bits1, count);
+}
+
+void launch_asm_halo_list(int n_nodes, const uint32_t* bits0, const uint32_t* bits1, const int* halo_ptr, int grid,
+                          int* halo, cudaStream_t s) {
+  asm_halo_list_kernel<<<grid, 256, 0, s>>>(n_nodes, bits0, bits1, halo_ptr, halo);
+}
+
 void launch_asm_lists(const MeshDev& m, const AsmLists& t, uint2* edges, uint32_t* eptr, uint32_t* list, cudaStream_t s) {
   const int g = (m.n_nodes + 127) / 128;
   if (m.npe == 8)
@@ -345,8 +393,8 @@ void launch_asm_lists(const MeshDev& m, const AsmLists& t, uint2* edges, uint32_
     asm_list_kernel<2><<<g, 128, 0, s>>>(m, t, edges, eptr, list);
 }
 
-void launch_asm_fill(const AsmDev& S, const int* row, const int* cols, cudaStream_t s) {
-  asm_fill_kernel<<<S.grid, 512, 0, s>>>(S, row, cols);
+void launch_asm_fill(const MeshDev& m, const AsmDev& S, const AsmLists& t, cudaStream_t s) {
+  asm_fill_kernel<<<S.grid, 512, 0, s>>>(m, S, t);
 }
 
 void launch_asm(const AsmArgs& a, int model, cudaStream_t s) {

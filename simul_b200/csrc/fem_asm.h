@@ -1,10 +1,6 @@
 // Tables and launchers of the assembled tangent (fem_asm.cu).
 #pragma once
-#include <algorithm>
 #include <cstdint>
-#include <exception>
-#include <system_error>
-#include <thread>
 #include <vector>
 
 #include "fem_internal.h"
@@ -14,54 +10,27 @@ namespace femb200 {
 // A CTA of the persistent solve takes at least this many rows (two warps').
 constexpr int kAsmMinRows = 64;
 
-// f(begin, end) over [0, n) on up to 16 host threads, `grain` or more each.  A
-// thread that cannot be had leaves its range to the caller's; an exception of
-// any range is thrown here once all have ended.
-template <typename F>
-void parallel_ranges(int n, F f, int grain = 1024) {
-  const int hw = std::max(1, (int)std::thread::hardware_concurrency());
-  const int nt = std::max(1, std::min(std::min(hw, 16), n / grain));
-  std::vector<std::exception_ptr> err(nt);
-  auto part = [&](int t) {
-    try {
-      f((int)((int64_t)n * t / nt), (int)((int64_t)n * (t + 1) / nt));
-    } catch (...) {
-      err[t] = std::current_exception();
-    }
-  };
-  std::vector<std::thread> pool;
-  pool.reserve(nt);
-  int started = 1;
-  try {
-    for (; started < nt; ++started) pool.emplace_back(part, started);
-  } catch (const std::system_error&) {
-  }
-  part(0);
-  for (int t = started; t < nt; ++t) part(t);
-  for (auto& th : pool) th.join();
-  for (auto& e : err)
-    if (e) std::rethrow_exception(e);
-}
+// A node's elements are sorted by one warp (asm_neighbours_kernel), in the
+// square of their number: above this many the mesh is refused.
+constexpr int kAsmMaxValence = 8192;
 
+// The rows dealt out to the CTAs and cut into slices, from the nodes' numbers
+// of neighbours.
 struct AsmHost {
-  std::vector<int> cols;           // neighbours of each node, ascending (CSR with row)
-  std::vector<int> row;
-  std::vector<uint32_t> erow;      // [Nn + 1] edges to higher nodes before each node
-  std::vector<uint32_t> lrow;      // [Nn + 1] (element, vertex pair) entries before each node's edges
-  std::vector<uint32_t> slot0;     // slot (step * 32 + lane) of each row's first entry (entry k: + 32 k)
   int grid = 0;
   std::vector<int> cta_row;        // [grid + 1] first row of each CTA
   std::vector<int> cta_slice;      // [grid + 1]
   std::vector<int> slice_step;     // [slices + 1] first step of each slice
   std::vector<int> slice_rows;     // [slices * 32] node of each lane, -1: none
-  std::vector<int> halo_ptr, halo;
+  std::vector<uint32_t> slot0;     // slot (step * 32 + lane) of each row's first entry (entry k: + 32 k)
   std::vector<int> prefix;         // prefix[k]: most steps that the first k slices of a CTA have
-  int max_slices = 0, max_halo = 0, max_cols = 0, max_pieces = 0;
+  int max_slices = 0, max_pieces = 0;
 };
 
-// Tables for a grid of at most `sms` CTAs.  False where the mesh does not fit
-// the format (2^27 steps, 65,536 columns of a CTA, 32-bit lists).
-bool build_asm_host(const int4* conn, int Nn, int Ne, int npe, int sms, AsmHost* out);
+// For a grid of at most `sms` CTAs.
+void asm_cta_rows(const std::vector<int>& deg, int sms, AsmHost* out);
+// False where the mesh does not fit the format (2^27 steps).
+bool asm_slices(const std::vector<int>& deg, AsmHost* out);
 
 struct AsmArgs {
   MeshDev m;
@@ -83,16 +52,30 @@ static __device__ __forceinline__ void asm_store(const AsmDev& S, uint32_t slot,
   reinterpret_cast<float*>(w + 272)[lane] = k22;
 }
 
-// AsmHost's lists on the device
+// Neighbour lists on the device, and where the edges go.
 struct AsmLists {
-  const int *row, *cols;
-  const uint32_t *erow, *lrow, *slot0;
+  const int* cols;       // node a's neighbours, ascending, from node_row[a] * (npe - 1) on
+  const int* deg;        // [Nn] their number
+  const uint32_t* erow;  // [Nn + 1] edges to higher nodes before each node
+  const uint32_t* lrow;  // [Nn + 1] (element, vertex pair) entries before each node's edges
+  const uint32_t* slot0;
 };
+// neighbours of every node; counts: [3][Nn] their number, those of higher
+// nodes, and the (element, vertex pair) entries of the edges to them.  cand and
+// cols: [node_row[Nn] * (npe - 1)]
+void launch_asm_neighbours(const MeshDev& m, int* cand, int* cols, int* counts, cudaStream_t s);
+// the columns of each CTA's rows outside its run, as one bit per node and their
+// number; then as ascending lists.  bits0 and bits1 take half the CTAs each:
+// [(grid + 1) / 2][(Nn + 31) / 32], zeroed
+void launch_asm_halo_mark(const MeshDev& m, const AsmLists& t, const int* cta_row, int grid, uint32_t* bits0,
+                          uint32_t* bits1, int* count, cudaStream_t s);
+void launch_asm_halo_list(int n_nodes, const uint32_t* bits0, const uint32_t* bits1, const int* halo_ptr, int grid,
+                          int* halo, cudaStream_t s);
 // the edges' slots, and per edge the elements on it as (element * npe +
 // vertex a) * npe + vertex b
 void launch_asm_lists(const MeshDev& m, const AsmLists& t, uint2* edges, uint32_t* eptr, uint32_t* list, cudaStream_t s);
 // local columns of every slot of the steps, from the neighbour lists
-void launch_asm_fill(const AsmDev& S, const int* row, const int* cols, cudaStream_t s);
+void launch_asm_fill(const MeshDev& m, const AsmDev& S, const AsmLists& t, cudaStream_t s);
 // values at the tangent state of `payload`
 void launch_asm(const AsmArgs& a, int model, cudaStream_t s);
 // HEX8: places of the elements' blocks in s.list (hpos, [32 Ne], preset to

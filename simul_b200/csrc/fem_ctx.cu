@@ -59,6 +59,7 @@ struct FemCtx {
   bool res_two_phase = true;   // TET4: two-phase FP64 residual (else the fused node-block kernel)
   int ndof = 0, ndof_pad = 0;
   int64_t blk_entries = 0;
+  int max_valence = 0;         // most elements on a node
   size_t bytes = 0;
   std::string err;
   std::vector<int> perm_node, perm_elem;  // internal -> caller
@@ -238,6 +239,7 @@ struct FemCtx {
   // persistent PCG kernel (fem_pcg.cu): tables per matrix and per coarse lattice
   PcgDev pcgdev{};
   std::vector<int> asm_cta_row;        // first row of each CTA
+  std::vector<int> asm_halo_ptr, asm_halo;  // its columns outside its rows
   std::vector<int> asm_prefix;         // steps of the first slices (shared-memory plan)
   bool pcg_coarse_built = false;
   bool chain_asked = false;      // by the fused step or programmatic launches; the rule's option value lifts it
@@ -401,6 +403,17 @@ int dalloc(FemCtx* c, T** ptr, size_t count) {
   if (e != cudaSuccess) return set_err(c, FEM_ERR_CUDA, "cudaMemset failed: %s", cudaGetErrorString(e));
   return FEM_OK;
 }
+
+// Places of several arrays in one allocation (base null: their total alone).
+struct Carve {
+  char* base;
+  size_t at = 0;
+  template <typename T>
+  void operator()(T** p, size_t n) {
+    *p = base ? reinterpret_cast<T*>(base + at) : nullptr;
+    at += (n * sizeof(T) + 255) & ~(size_t)255;
+  }
+};
 
 inline uint32_t spread10(uint32_t v) {
   v &= 0x3ffu;
@@ -591,6 +604,7 @@ int build_tables(FemCtx* c, const double* X, const int32_t* conn_user) {
       }
       std::sort(ents.begin(), ents.end());
       node_row[n + 1] = node_row[n] + (int)ents.size();
+      c->max_valence = std::max(c->max_valence, (int)ents.size());
       for (size_t k = 0; k < ents.size(); ++k) {
         const int pos = node_row[n] + (int)k;
         node_slots[pos] = ents[k].first;
@@ -999,96 +1013,144 @@ AsmArgs asm_args(const FemCtx* c) {
 // Tables of the assembled tangent; asm_refused where the mesh does not fit the
 // format.  *room = false where the device memory does not hold them.
 int build_asm_tables(FemCtx* c, bool* room) {
-  const size_t cw = (size_t)c->npe / 4;
-  std::vector<int4> conn(cw * c->Ne);
-  CK(cudaMemcpyAsync(conn.data(), c->conn, conn.size() * sizeof(int4), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
-  AsmHost h;
+  const size_t Nn = (size_t)c->Nn, Ne = (size_t)c->Ne, npe = (size_t)c->npe, words = (Nn + 31) / 32;
   int sms = 0;
   CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-  if (!build_asm_host(conn.data(), c->Nn, c->Ne, c->npe, sms, &h)) {
-    c->asm_refused = true;
+  c->asm_refused = true;
+  if (c->max_valence > kAsmMaxValence || Ne * npe * npe > 0xffffffffULL) return FEM_OK;
+  c->asm_refused = false;
+  *room = false;  // until all of them are there
+  const MeshDev m = c->mesh();
+  const cudaStream_t s = c->stream;
+  // All that the tables are derived through lies in buffers that hold nothing
+  // between calls: the slot stagings (npe (npe - 1) words an element of 4 npe
+  // and 8 npe, HEX8 8 npe both) and the solve's vectors (4 words a node; a
+  // CTA's marks take 1 / 32 word a node, so half the CTAs' fit one)
+  AsmHost h;
+  std::vector<int> counts(3 * Nn);
+  int* d_counts = reinterpret_cast<int*>(c->p);
+  uint32_t* d_erow = reinterpret_cast<uint32_t*>(c->y);
+  uint32_t *d_lrow = d_erow + Nn + 1, *d_slot0 = d_lrow + Nn + 1;
+  uint32_t* bits[2] = {reinterpret_cast<uint32_t*>(c->x), reinterpret_cast<uint32_t*>(c->r)};
+  int *cand = reinterpret_cast<int*>(c->stage), *cols = reinterpret_cast<int*>(c->stage_d);
+  launch_asm_neighbours(m, cand, cols, d_counts, s);
+  CKL();
+  CK(cudaMemcpyAsync(counts.data(), d_counts, counts.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
+  CK(cudaStreamSynchronize(s));
+  std::vector<int> deg(counts.begin(), counts.begin() + Nn);
+  asm_cta_rows(deg, sms, &h);
+  int *d_cta_row0 = reinterpret_cast<int*>(c->tmpf), *d_count = d_cta_row0 + h.grid + 1;
+  const size_t half = (size_t)((h.grid + 1) / 2) * words;
+  if (half > 4 * Nn) {  // (more than 250 CTAs)
+    c->asm_refused = *room = true;
     return FEM_OK;
   }
+  AsmLists t;
+  t.cols = cols;
+  t.deg = d_counts;
+  t.erow = d_erow;
+  t.lrow = d_lrow;
+  t.slot0 = d_slot0;
+  std::vector<int> halo_n(h.grid), halo_ptr(1, 0);
+  CK(cudaMemcpyAsync(d_cta_row0, h.cta_row.data(), h.cta_row.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+  for (uint32_t* b : bits) CK(cudaMemsetAsync(b, 0, half * sizeof(uint32_t), s));
+  launch_asm_halo_mark(m, t, d_cta_row0, h.grid, bits[0], bits[1], d_count, s);
+  CKL();
+  CK(cudaMemcpyAsync(halo_n.data(), d_count, halo_n.size() * sizeof(int), cudaMemcpyDeviceToHost, s));
+  std::vector<uint32_t> erow(Nn + 1, 0u), lrow(Nn + 1, 0u);
+  int64_t n_list = 0;
+  for (size_t a = 0; a < Nn; ++a) {
+    erow[a + 1] = erow[a] + (uint32_t)counts[Nn + a];
+    n_list += counts[2 * Nn + a];
+    lrow[a + 1] = (uint32_t)n_list;
+  }
+  const bool fits = n_list <= 0x7fffffffLL && asm_slices(deg, &h);
+  CK(cudaStreamSynchronize(s));
+  int max_halo = 0, max_cols = 0;
+  for (int g = 0; g < h.grid; ++g) {
+    halo_ptr.push_back(halo_ptr.back() + halo_n[g]);
+    max_halo = std::max(max_halo, halo_n[g]);
+    max_cols = std::max(max_cols, h.cta_row[g + 1] - h.cta_row[g] + halo_n[g]);
+  }
+  if (!fits || max_cols > 65536) {
+    c->asm_refused = *room = true;
+    return FEM_OK;
+  }
+  const size_t n_edges = erow[Nn], n_halo = (size_t)halo_ptr.back(), grid = (size_t)h.grid;
+  int *cta_row, *cta_slice, *slice_step, *slice_rows, *d_halo_ptr, *halo;
+  uint2* edges;
+  uint32_t *eptr, *list, *steps, *hpos = nullptr;
   AsmDev& S = c->asmdev;
-  uint32_t* words = nullptr;
-  *room = false;  // until all of them are there
-  auto up = [&](auto** dst, const auto& v) {
-    return table_alloc(c, c->asm_bufs, dst, v.size()) &&
-           (v.empty() || cudaMemcpyAsync(*dst, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, c->stream) ==
-                             cudaSuccess);
+  auto carve_tables = [&](char* base) {
+    Carve at{base};
+    at(&cta_row, grid + 1);
+    at(&cta_slice, grid + 1);
+    at(&slice_step, h.slice_step.size());
+    at(&slice_rows, h.slice_rows.size());
+    at(&d_halo_ptr, grid + 1);
+    at(&halo, n_halo);
+    at(&edges, n_edges);
+    at(&eptr, n_edges + 1);
+    at(&list, (size_t)n_list);
+    at(&steps, (size_t)h.slice_step.back() * kAsmStepWords);
+    at(&c->pcg_part, 4 * grid);
+    at(&c->pcg_bar, 1);
+    at(&c->pcg_p2, 4 * Nn);
+    if (npe == 8) {
+      at(&hpos, 32 * Ne);
+      at(&S.hblk4, 2 * (size_t)n_list);
+      at(&S.hblk1, (size_t)n_list);
+    }
+    return at.at;
   };
-  int *cta_row = nullptr, *cta_slice = nullptr, *slice_step = nullptr, *slice_rows = nullptr, *halo_ptr = nullptr,
-      *halo = nullptr;
-  uint2* edges = nullptr;
-  uint32_t *eptr = nullptr, *list = nullptr;
-  if (!up(&cta_row, h.cta_row) || !up(&cta_slice, h.cta_slice) || !up(&slice_step, h.slice_step) ||
-      !up(&slice_rows, h.slice_rows) || !up(&halo_ptr, h.halo_ptr) || !up(&halo, h.halo))
-    return FEM_OK;
-  const size_t n_edges = h.erow.back(), n_list = h.lrow.back();
-  auto table = [&](auto** dst, size_t n) { return table_alloc(c, c->asm_bufs, dst, n); };
-  if (!table(&edges, n_edges) || !table(&eptr, n_edges + 1) || !table(&list, n_list) ||
-      !table(&words, (size_t)h.slice_step.back() * kAsmStepWords) || !table(&c->pcg_part, 4 * (size_t)h.grid) ||
-      !table(&c->pcg_bar, 1) || !table(&c->pcg_p2, 4 * (size_t)c->Nn))
-    return FEM_OK;
-  uint32_t* hpos = nullptr;
-  if (c->npe == 8 &&
-      (!table(&hpos, 32 * (size_t)c->Ne) || !table(&S.hblk4, 2 * n_list) || !table(&S.hblk1, n_list)))
-    return FEM_OK;
+  char* tables = nullptr;
+  if (!table_alloc(c, c->asm_bufs, &tables, carve_tables(nullptr))) return FEM_OK;
+  carve_tables(tables);
   S.grid = h.grid;
   S.n_slices = (int)h.slice_step.size() - 1;
   S.n_edges = (int)n_edges;
   S.max_slices = h.max_slices;
-  S.max_halo = h.max_halo;
-  S.max_cols = (h.max_cols + 3) & ~3;  // (float4 arrays follow the planes)
+  S.max_halo = max_halo;
+  S.max_cols = (max_cols + 3) & ~3;  // (float4 arrays follow the planes)
   S.max_pieces = h.max_pieces;
   S.cta_row = cta_row;
   S.cta_slice = cta_slice;
   S.slice_step = slice_step;
   S.slice_rows = slice_rows;
-  S.words = words;
+  S.words = steps;
   S.edges = edges;
   S.eptr = eptr;
   S.list = list;
-  S.halo_ptr = halo_ptr;
+  S.halo_ptr = d_halo_ptr;
   S.halo = halo;
-  c->asm_cta_row = h.cta_row;
-  c->asm_prefix = h.prefix;
-  // the lists the device derives the rest from, for that only
-  uint32_t* tmp = nullptr;
-  const size_t nr = h.row.size(), nc = h.cols.size(), nn = (size_t)c->Nn;
-  if (cudaMalloc(reinterpret_cast<void**>(&tmp), (3 * nr + nc + nn) * sizeof(uint32_t)) != cudaSuccess) {
-    cudaGetLastError();
-    return FEM_OK;
-  }
+  S.hpos = hpos;
   cudaError_t e = cudaSuccess;
-  size_t at = 0;
-  auto put = [&](const void* src, size_t n) {
-    const uint32_t* d = tmp + at;
-    if (e == cudaSuccess && n) e = cudaMemcpyAsync(tmp + at, src, n * sizeof(uint32_t), cudaMemcpyHostToDevice, c->stream);
-    at += n;
-    return d;
+  auto up = [&](auto* dst, const auto& v) {
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, s);
   };
-  AsmLists t;
-  t.row = reinterpret_cast<const int*>(put(h.row.data(), nr));
-  t.erow = put(h.erow.data(), nr);
-  t.lrow = put(h.lrow.data(), nr);
-  t.slot0 = put(h.slot0.data(), nn);
-  t.cols = reinterpret_cast<const int*>(put(h.cols.data(), nc));
-  if (e == cudaSuccess) {
-    launch_asm_fill(S, t.row, t.cols, c->stream);
-    launch_asm_lists(c->mesh(), t, edges, eptr, list, c->stream);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);  // the host tables go out of scope
-  cudaFree(tmp);
+  up(cta_row, h.cta_row);
+  up(cta_slice, h.cta_slice);
+  up(slice_step, h.slice_step);
+  up(slice_rows, h.slice_rows);
+  up(d_halo_ptr, halo_ptr);
+  up(d_erow, erow);
+  up(d_lrow, lrow);
+  up(d_slot0, h.slot0);
   CK(e);
-  if (c->npe == 8) {
-    CK(cudaMemsetAsync(hpos, 0xff, 32 * sizeof(uint32_t) * (size_t)c->Ne, c->stream));  // kNoPlace
-    launch_asm_hex_places(list, n_list, hpos, c->stream);
-    CKL();
-    S.hpos = hpos;
+  launch_asm_halo_list(c->Nn, bits[0], bits[1], d_halo_ptr, h.grid, halo, s);
+  launch_asm_fill(m, S, t, s);
+  launch_asm_lists(m, t, edges, eptr, list, s);
+  if (hpos) {
+    CK(cudaMemsetAsync(hpos, 0xff, 32 * Ne * sizeof(uint32_t), s));  // kNoPlace
+    launch_asm_hex_places(list, (size_t)n_list, hpos, s);
   }
+  CKL();
+  c->asm_halo.resize(n_halo);
+  if (n_halo) CK(cudaMemcpyAsync(c->asm_halo.data(), halo, n_halo * sizeof(int), cudaMemcpyDeviceToHost, s));
+  CK(cudaStreamSynchronize(s));
+  c->asm_cta_row = h.cta_row;
+  c->asm_halo_ptr = halo_ptr;
+  c->asm_prefix = h.prefix;
   c->asm_built = *room = true;
   c->asm_valid = false;
   return FEM_OK;
@@ -1100,7 +1162,7 @@ int ensure_asm_tables(FemCtx* c) {
   int st = FEM_OK;
   try {
     st = build_asm_tables(c, &room);
-  } catch (const std::exception&) {  // host memory or threads
+  } catch (const std::bad_alloc&) {  // host memory
     room = false;
   }
   if (st || !room) {
@@ -1576,25 +1638,6 @@ int ensure_cg_graph(FemCtx* c, int kind) {
   return FEM_OK;
 }
 
-template <typename T>
-int coarse_upload(FemCtx* c, const T** dst, const std::vector<T>& v) {
-  T* d = nullptr;
-  int st;
-  if ((st = dalloc(c, &d, v.size()))) return st;
-  c->coarse_bufs.push_back(d);
-  if (!v.empty()) CK(cudaMemcpyAsync(d, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, c->stream));
-  *dst = d;
-  return FEM_OK;
-}
-
-template <typename T>
-int coarse_alloc(FemCtx* c, T** dst, size_t n) {
-  int st;
-  if ((st = dalloc(c, dst, n))) return st;
-  c->coarse_bufs.push_back(*dst);
-  return FEM_OK;
-}
-
 // Builds the coarse lattice: cell edge H = coarse_cell_voxels x the mesh
 // length (cube root of 5 x the mean element volume: the voxel edge on
 // 5-tet voxel meshes), grown by 25 % steps until at most coarse_max_nodes
@@ -1759,31 +1802,9 @@ int build_coarse(FemCtx* c) {
   cd.n_dof = 3 * n_cn;
   cd.inv_H = (float)(1.0 / H);
   cd.lo = make_float3((float)org[0], (float)org[1], (float)org[2]);
-  int st;
-  if ((st = coarse_upload(c, &cd.cell_ijk, cell_ijk))) return st;
-  if ((st = coarse_upload(c, &cd.cell_corner, cell_corner))) return st;
-  if ((st = coarse_upload(c, &cd.cell_node_ptr, cell_node_ptr))) return st;
-  if ((st = coarse_upload(c, &cd.cell_nodes, cell_nodes))) return st;
-  if ((st = coarse_upload(c, &cd.cell_elem_ptr, cell_elem_ptr))) return st;
-  if ((st = coarse_upload(c, &cd.cell_elems, cell_elems))) return st;
-  if ((st = coarse_upload(c, &cd.node_cell, node_cell))) return st;
-  if ((st = coarse_upload(c, &cd.cn_cells, cn_cells))) return st;
-  {
-    float4* lat = nullptr;
-    if ((st = coarse_alloc(c, &lat, (size_t)Nn))) return st;
-    cd.node_lat = lat;
-    launch_coarse_node_lat(c->mesh(), cd, lat, c->stream);
-    CKL();
-    uint4* corners = nullptr;
-    if ((st = coarse_alloc(c, &corners, (size_t)Nn))) return st;
-    cd.node_corners = corners;
-    launch_coarse_node_corners(c->mesh(), cd, corners, c->stream);
-    CKL();
-  }
-  const size_t nd = (size_t)cd.n_dof;
+  const size_t nd = (size_t)cd.n_dof, cells = (size_t)n_cells;
   cd.cell_slices = coarse_cell_slices(c->npe);
-  if ((st = coarse_alloc(c, &cd.blocks, (size_t)n_cells * cd.cell_slices * 576))) return st;
-  if ((st = coarse_alloc(c, &cd.Ac, nd * nd))) return st;
+  cd.r_slices = coarse_restrict_slices(n_cells);
   cd.nb16 = (cd.n_dof + 63) / 64;
   const size_t nb = (size_t)cd.nb16;
   cd.Ainv = nullptr;
@@ -1792,18 +1813,64 @@ int build_coarse(FemCtx* c) {
   cd.Afull32 = nullptr;
   cd.Ainv16 = nullptr;
   cd.yslots = nullptr;
-  if (c->coarse_bf16) {
-    if ((st = coarse_alloc(c, &cd.Ainv16, nb * (nb + 1) / 2 * 4096))) return st;
-    if ((st = coarse_alloc(c, &cd.yslots, nb * nb * 64))) return st;
-  } else {
-    if ((st = coarse_alloc(c, &cd.Ainv, nd * nd))) return st;
-  }
-  cd.r_slices = coarse_restrict_slices(n_cells);
-  if ((st = coarse_alloc(c, &cd.cell_r, (size_t)n_cells * cd.r_slices * 24))) return st;
-  if ((st = coarse_alloc(c, &cd.yc, nb * 64))) return st;
-  if ((st = coarse_alloc(c, &cd.rc, nb * 64))) return st;
-  // fused two-level step: per (cell, slice) restriction and ||r||^2 shares
-  if ((st = coarse_alloc(c, &c->tl_part, (size_t)n_cells * cd.r_slices + step_chunks(Nn)))) return st;
+  int3* d_ijk;
+  int *d_corner, *d_node_ptr, *d_nodes, *d_elem_ptr, *d_elems, *d_node_cell, *d_cn_cells;
+  float4* lat;
+  uint4* corners;
+  // (one allocation: a first solve pays for each)
+  auto carve = [&](char* base) {
+    Carve at{base};
+    at(&d_ijk, cell_ijk.size());
+    at(&d_corner, cell_corner.size());
+    at(&d_node_ptr, cell_node_ptr.size());
+    at(&d_nodes, cell_nodes.size());
+    at(&d_elem_ptr, cell_elem_ptr.size());
+    at(&d_elems, cell_elems.size());
+    at(&d_node_cell, node_cell.size());
+    at(&d_cn_cells, cn_cells.size());
+    at(&lat, (size_t)Nn);
+    at(&corners, (size_t)Nn);
+    at(&cd.blocks, cells * cd.cell_slices * 576);
+    at(&cd.Ac, nd * nd);
+    if (c->coarse_bf16) {
+      at(&cd.Ainv16, nb * (nb + 1) / 2 * 4096);
+      at(&cd.yslots, nb * nb * 64);
+    } else {
+      at(&cd.Ainv, nd * nd);
+    }
+    at(&cd.cell_r, cells * cd.r_slices * 24);
+    at(&cd.yc, nb * 64);
+    at(&cd.rc, nb * 64);
+    // fused two-level step: per (cell, slice) restriction and ||r||^2 shares
+    at(&c->tl_part, cells * cd.r_slices + step_chunks(Nn));
+    return at.at;
+  };
+  int st;
+  char* tables = nullptr;
+  if ((st = dalloc(c, &tables, carve(nullptr)))) return st;
+  c->coarse_bufs.push_back(tables);
+  carve(tables);
+  cudaError_t e = cudaSuccess;
+  auto up = [&](auto** field, auto* dst, const auto& v) {
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, c->stream);
+    *field = dst;
+  };
+  up(&cd.cell_ijk, d_ijk, cell_ijk);
+  up(&cd.cell_corner, d_corner, cell_corner);
+  up(&cd.cell_node_ptr, d_node_ptr, cell_node_ptr);
+  up(&cd.cell_nodes, d_nodes, cell_nodes);
+  up(&cd.cell_elem_ptr, d_elem_ptr, cell_elem_ptr);
+  up(&cd.cell_elems, d_elems, cell_elems);
+  up(&cd.node_cell, d_node_cell, node_cell);
+  up(&cd.cn_cells, d_cn_cells, cn_cells);
+  CK(e);
+  cd.node_lat = lat;
+  launch_coarse_node_lat(c->mesh(), cd, lat, c->stream);
+  CKL();
+  cd.node_corners = corners;
+  launch_coarse_node_corners(c->mesh(), cd, corners, c->stream);
+  CKL();
   // the persistent solve reads full rows up to 16 MB: they come from L2 in
   // about the time that adding up the packed tiles' two products takes.
   // Optional: without its form of the inverse it is refused (run_persistent)
@@ -2120,44 +2187,54 @@ int build_pcg_coarse(FemCtx* c, bool* fit) {
                      c->stream));
   CK(cudaMemcpyAsync(corner.data(), c->cdev.cell_corner, corner.size() * sizeof(int), cudaMemcpyDeviceToHost,
                      c->stream));
-  std::vector<int> halo_ptr(c->asm_cta_row.size());
-  CK(cudaMemcpyAsync(halo_ptr.data(), c->asmdev.halo_ptr, halo_ptr.size() * sizeof(int), cudaMemcpyDeviceToHost,
-                     c->stream));
-  CK(cudaStreamSynchronize(c->stream));
-  std::vector<int> halo((size_t)halo_ptr.back());
-  if (!halo.empty())
-    CK(cudaMemcpyAsync(halo.data(), c->asmdev.halo, halo.size() * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   PcgCoarseHost h;
-  if (!pcg_coarse_tables(c->asm_cta_row, halo_ptr, halo, node_cell, corner, c->cdev.n_cn,
+  if (!pcg_coarse_tables(c->asm_cta_row, c->asm_halo_ptr, c->asm_halo, node_cell, corner, c->cdev.n_cn,
                          c->cdev.full_ld ? 0 : (c->cdev.Ainv16 ? 2 : 4), &h))
     return FEM_OK;
-  auto& bufs = c->pcg_coarse_bufs;
-  auto up = [&](auto** dst, const auto& v) {
-    std::remove_const_t<std::remove_pointer_t<std::remove_reference_t<decltype(*dst)>>>* d = nullptr;
-    if (!table_alloc(c, bufs, &d, v.size())) return false;
-    *dst = d;
-    return v.empty() ||
-           cudaMemcpyAsync(d, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, c->stream) == cudaSuccess;
+  int *tab_ptr, *tab, *seg_rows, *cn_ptr;
+  uint4* col_corners;
+  float4* lat;
+  auto carve = [&](char* base) {
+    Carve at{base};
+    at(&tab_ptr, h.tab_ptr.size());
+    at(&tab, h.tab.size());
+    at(&seg_rows, h.seg_rows.size());
+    at(&col_corners, h.col_corners.size());
+    at(&cn_ptr, h.cn_ptr.size());
+    at(&lat, (size_t)c->Nn);
+    at(&t.seg_r, 8 * (size_t)h.n_seg);
+    at(&t.ypart, 64 * (size_t)h.n_parts);
+    return at.at;
   };
-  const int* seg_rows = nullptr;
-  float4* lat = nullptr;
-  bool room = up(&t.tab_ptr, h.tab_ptr) && up(&t.tab, h.tab) && up(&seg_rows, h.seg_rows) &&
-              up(&t.col_corners, h.col_corners) && up(&t.cn_ptr, h.cn_ptr) &&
-              table_alloc(c, bufs, &lat, (size_t)c->Nn) && table_alloc(c, bufs, &t.seg_r, 8 * (size_t)h.n_seg) &&
-              table_alloc(c, bufs, &t.ypart, 64 * (size_t)h.n_parts);
-  if (room) {
-    t.merged = c->cdev.full_ld && 8 * h.n_seg <= kPcgMergedShares;
-    launch_pcg_seg_lat(seg_rows, c->cdev.node_lat, c->Nn, lat, c->stream);
-    t.seg_lat = lat;
-    t.max_tab = h.max_tab;
-    t.max_lblk = h.max_lblk;
-    t.max_loc = h.max_loc;
-    t.max_tiles = h.max_tiles;
-  }
+  char* tables = nullptr;
+  if (!table_alloc(c, c->pcg_coarse_bufs, &tables, carve(nullptr))) return FEM_OK;
+  carve(tables);
+  cudaError_t e = cudaSuccess;
+  auto up = [&](auto* dst, const auto& v) {
+    if (e == cudaSuccess && !v.empty())
+      e = cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, c->stream);
+  };
+  up(tab_ptr, h.tab_ptr);
+  up(tab, h.tab);
+  up(seg_rows, h.seg_rows);
+  up(col_corners, h.col_corners);
+  up(cn_ptr, h.cn_ptr);
+  CK(e);
+  launch_pcg_seg_lat(seg_rows, c->cdev.node_lat, c->Nn, lat, c->stream);
+  t.tab_ptr = tab_ptr;
+  t.tab = tab;
+  t.col_corners = col_corners;
+  t.cn_ptr = cn_ptr;
+  t.seg_lat = lat;
+  t.merged = c->cdev.full_ld && 8 * h.n_seg <= kPcgMergedShares;
+  t.max_tab = h.max_tab;
+  t.max_lblk = h.max_lblk;
+  t.max_loc = h.max_loc;
+  t.max_tiles = h.max_tiles;
   CK(cudaStreamSynchronize(c->stream));  // the host tables go out of scope
   CKL();
-  c->pcg_coarse_built = *fit = room;
+  c->pcg_coarse_built = *fit = true;
   return FEM_OK;
 }
 
@@ -2175,7 +2252,7 @@ int ensure_pcg_tables(FemCtx* c, bool two_level) {
   int st = FEM_OK;
   try {
     st = build_pcg_coarse(c, &fit);
-  } catch (const std::exception&) {  // host memory or threads
+  } catch (const std::bad_alloc&) {  // host memory
     cudaStreamSynchronize(c->stream);
     fit = false;
   }

@@ -51,62 +51,77 @@ bool pcg_coarse_tables(const std::vector<int>& cta_row, const std::vector<int>& 
     tabs[g][word] = (int)tabs[g].size();
     tabs[g].insert(tabs[g].end(), v.begin(), v.end());
   };
-  // rows of each CTA by cell; the coarse nodes that its columns (its rows, then
-  // its halo) interpolate from
+  // Per CTA: its rows by cell (segments), and the coarse nodes that its columns
+  // (its rows, then its halo) interpolate from, ascending, so that neighbouring
+  // threads read neighbouring words of y_c.  By distinct cell, of which a CTA
+  // has few: sorting the rows and looking up every column's corners took 6 ms
+  // on one core at 51,000 rows, this 2.
+  const int n_cells = (int)(cell_corner.size() / 8);
   std::vector<std::vector<int>> shares(n_cn), loc(G);
-  o->seg_rows.reserve(Nn);
+  o->seg_rows.resize(Nn);
   o->col_corners.resize((size_t)Nn + halo.size());
-  std::vector<std::pair<int, int>> by_cell;
-  std::vector<int> sptr;
+  std::vector<int> cell_at(n_cells, -1), cell_rows(n_cells, 0), local(n_cn, -1), cells, lg, sptr;
+  std::vector<uint4> cell_cc(n_cells);
   for (int g = 0; g < G; ++g) {
-    by_cell.clear();
-    for (int r = cta_row[g]; r < cta_row[g + 1]; ++r) by_cell.push_back({node_cell[r], r});
-    std::sort(by_cell.begin(), by_cell.end());
+    const int r0 = cta_row[g], r1 = cta_row[g + 1], nh = halo_ptr[g + 1] - halo_ptr[g];
+    const int* hal = halo.data() + halo_ptr[g];
+    cells.clear();
+    for (int r = r0; r < r1; ++r) {
+      const int c = node_cell[r];
+      if (cell_at[c] != g) {
+        cell_at[c] = g;
+        cell_rows[c] = 0;
+        cells.push_back(c);
+      }
+      ++cell_rows[c];
+    }
+    std::sort(cells.begin(), cells.end());
+    const size_t row_cells = cells.size();
     sptr.assign(1, 0);
     tabs[g][TAB_SEG0] = o->n_seg;
-    tabs[g][TAB_SROW] = (int)o->seg_rows.size();
-    for (size_t j = 0; j < by_cell.size();) {
-      const int cell = by_cell[j].first;
-      size_t j1 = j;
-      while (j1 < by_cell.size() && by_cell[j1].first == cell) ++j1;
-      for (int q = 0; q < 8; ++q) shares[cell_corner[8 * (size_t)cell + q]].push_back(o->n_seg * 8 + q);
-      for (; j < j1; ++j) o->seg_rows.push_back(by_cell[j].second);
-      sptr.push_back((int)j1);
+    tabs[g][TAB_SROW] = r0;
+    for (int c : cells) {
+      for (int q = 0; q < 8; ++q) shares[cell_corner[8 * (size_t)c + q]].push_back(o->n_seg * 8 + q);
+      const int at = sptr.back();
+      sptr.push_back(at + cell_rows[c]);
+      cell_rows[c] = at;  // from here on the place of the cell's next row
       ++o->n_seg;
     }
-    tabs[g][TAB_NSEG] = (int)sptr.size() - 1;
+    for (int r = r0; r < r1; ++r) o->seg_rows[r0 + cell_rows[node_cell[r]]++] = r;
+    tabs[g][TAB_NSEG] = (int)row_cells;
     put(g, TAB_SPTR, sptr);
-  }
-  parallel_ranges(G, [&](int g0, int g1) {
-    std::vector<int> seen(n_cn, -1), local(n_cn, 0);
-    for (int g = g0; g < g1; ++g) {
-      const int nrow = cta_row[g + 1] - cta_row[g], nh = halo_ptr[g + 1] - halo_ptr[g];
-      // (ascending, so that neighbouring threads read neighbouring words of y_c)
-      auto cell_of = [&](int i) { return node_cell[i < nrow ? cta_row[g] + i : halo[halo_ptr[g] + i - nrow]]; };
-      std::vector<int>& lg = loc[g];
-      for (int i = 0; i < nrow + nh; ++i)
-        for (int q = 0; q < 8; ++q) {
-          const int cn = cell_corner[8 * (size_t)cell_of(i) + q];
-          if (seen[cn] != g) {
-            seen[cn] = g;
-            lg.push_back(cn);
-          }
-        }
-      std::sort(lg.begin(), lg.end());
-      for (size_t k = 0; k < lg.size(); ++k) local[lg[k]] = (int)k;
-      uint4* cc = o->col_corners.data() + cta_row[g] + halo_ptr[g];
-      for (int i = 0; i < nrow + nh; ++i) {
-        uint32_t idx[8];
-        for (int q = 0; q < 8; ++q) idx[q] = (uint32_t)local[cell_corner[8 * (size_t)cell_of(i) + q]];
-        cc[i] = make_uint4(idx[0] | idx[1] << 16, idx[2] | idx[3] << 16, idx[4] | idx[5] << 16, idx[6] | idx[7] << 16);
+    for (int k = 0; k < nh; ++k) {
+      const int c = node_cell[hal[k]];
+      if (cell_at[c] != g) {
+        cell_at[c] = g;
+        cells.push_back(c);
       }
     }
-  }, 1);
-  for (int g = 0; g < G; ++g) {
-    if (loc[g].size() > 65536) return false;
-    tabs[g][TAB_NLOC] = (int)loc[g].size();
-    put(g, TAB_LOC, loc[g]);
-    o->max_loc = std::max(o->max_loc, (int)loc[g].size());
+    lg.clear();
+    for (int c : cells)
+      for (int q = 0; q < 8; ++q) {
+        int& l = local[cell_corner[8 * (size_t)c + q]];
+        if (l < 0) {
+          l = 0;
+          lg.push_back(cell_corner[8 * (size_t)c + q]);
+        }
+      }
+    if (lg.size() > 65536) return false;
+    std::sort(lg.begin(), lg.end());
+    for (size_t k = 0; k < lg.size(); ++k) local[lg[k]] = (int)k;
+    for (int c : cells) {
+      uint32_t idx[8];
+      for (int q = 0; q < 8; ++q) idx[q] = (uint32_t)local[cell_corner[8 * (size_t)c + q]];
+      cell_cc[c] = make_uint4(idx[0] | idx[1] << 16, idx[2] | idx[3] << 16, idx[4] | idx[5] << 16, idx[6] | idx[7] << 16);
+    }
+    uint4* cc = o->col_corners.data() + r0 + halo_ptr[g];
+    for (int r = r0; r < r1; ++r) *cc++ = cell_cc[node_cell[r]];
+    for (int k = 0; k < nh; ++k) *cc++ = cell_cc[node_cell[hal[k]]];
+    for (int n : lg) local[n] = -1;
+    tabs[g][TAB_NLOC] = (int)lg.size();
+    put(g, TAB_LOC, lg);
+    o->max_loc = std::max(o->max_loc, (int)lg.size());
+    loc[g] = lg;
   }
   // the shares of a coarse node lie together: each share's place
   std::vector<int> place(8 * (size_t)o->n_seg);
