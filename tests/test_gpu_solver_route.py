@@ -65,3 +65,25 @@ def test_the_rule_can_be_restored(cuda, element):
     s.mesh.set_matvec_variant("auto")
     assert s.variant() == "assembled"
     assert _lib.load().fem_set_option(s.mesh.ctx, _lib.FEM_OPT_MATVEC_VARIANT, -3) == _lib.FEM_ERR_INVALID
+
+
+@pytest.mark.parametrize("grid,variant", [((7, 3, 3), "fused"), ((7, 3, 4), "persistent")])
+def test_single_product_by_size(cuda, grid, variant):
+    """128 nodes and 160: one launch, or the pair."""
+    X, conn = meshgen.structured_tets(*grid)
+    X = X + 0.02 / max(grid) * np.random.default_rng(0).standard_normal(X.shape)
+    assert (X.shape[0] <= 128) == (variant == "fused")
+    mesh = B.FEMesh(X.shape[0], conn.shape[0], device=cuda)
+    mesh.initialize_from_numpy(X, conn)
+    mat = B.NeoHookean(17e3, 0.3)
+    mesh.u.copy_(torch.from_numpy(0.01 * np.random.default_rng(1).standard_normal(X.shape)))
+    mat.compute_nodal_forces(mesh)
+    x = torch.randn(X.shape, device=cuda, generator=torch.Generator(cuda).manual_seed(0))
+    y = {}
+    for v in ("auto", "fused", "persistent"):
+        mesh.set_matvec_variant(v)
+        y[v] = torch.empty_like(x)
+        assert _lib.load().fem_tangent_matvec(mesh.ctx, B._ptr(x), B._ptr(y[v])) == 0
+    assert not torch.equal(y["fused"], y["persistent"])   # told apart by rounding
+    assert float((y["fused"] - y["persistent"]).norm() / y["fused"].norm()) < 1e-6
+    assert torch.equal(y["auto"], y[variant])
