@@ -289,8 +289,8 @@ def configure(mesh, args):
                             inverse=args.coarse_inverse, max_nodes=args.coarse_max_nodes)
     if args.matvec_variant != "auto":
         mesh.set_matvec_variant(args.matvec_variant)
-    # the options of the kernel chain only where they differ from the defaults:
-    # setting one makes the solves run as that chain
+    # the options of the kernel chain only where they differ from its defaults:
+    # most of them make the solves run as that chain
     if args.fused_step:
         mesh.set_fused_step(True)
     if not args.whole_solve_graph:
@@ -368,7 +368,7 @@ def roofline_point(args, n, dev):
     u[:, 2] = -0.004 * v.X[:, 2]
     mesh.u.copy_(torch.from_numpy(u))
     mat.compute_nodal_forces(mesh)
-    # the variant choice the solver makes (timed on a first PCG solve)
+    # a first PCG solve, as a program has made one
     rhs = torch.zeros(v.n_nodes, 3, dtype=torch.float64, device=dev)
     rhs[:, 2] = 1.0
     du = torch.zeros_like(rhs)
@@ -390,6 +390,41 @@ def roofline_point(args, n, dev):
     del mesh
     torch.cuda.empty_cache()
     return out
+
+
+def pcg_point(args, mesh, conn, dev):
+    """The persistent PCG kernel that the headline's solves run in: time per
+    iteration (two solves of 40 and 20 iterations, best of four) against the
+    bytes one streams, the assembled blocks (38 bytes an entry) and the coarse
+    inverse in the form the kernel reads."""
+    import ctypes as C
+    import torch
+    from simul_b200 import _lib
+    from simul_b200 import fem as B
+    rhs = torch.randn(mesh.n_nodes, 3, dtype=torch.float64, device=dev)
+    du = torch.zeros_like(rhs)
+    best = {}
+    for n_it in (40, 20) * 4:
+        it, rel = C.c_int32(), C.c_double()
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        _lib.load().fem_pcg(mesh.ctx, _lib.FEM_PRECOND_TWO_LEVEL, B._ptr(rhs), B._ptr(du), 1e-20, n_it, C.byref(it),
+                            C.byref(rel))
+        best[n_it] = min(best.get(n_it, 1e9), time.perf_counter() - t0)
+        if it.value != n_it or mesh.stats()["matvec_variant"] != "assembled":
+            return None
+    cn = torch.as_tensor(np.asarray(conn), dtype=torch.int64, device=dev)
+    a, b = torch.triu_indices(cn.shape[1], cn.shape[1], 1)
+    lo, hi = torch.minimum(cn[:, a], cn[:, b]), torch.maximum(cn[:, a], cn[:, b])
+    entries = 2 * int(torch.unique(lo * mesh.n_nodes + hi).numel())
+    info = mesh.coarse_info()
+    nd, word = info["coarse_dofs"], 2 if args.coarse_bf16 else 4
+    rows = nd * ((nd + 7) // 8 * 8) * word
+    nb = (nd + 63) // 64
+    inverse = rows if rows <= (16 << 20) else nb * (nb + 1) // 2 * 4096 * word
+    s = (best[40] - best[20]) / 20
+    return {"us_per_iteration": s * 1e6, "entries": entries, "matrix_bytes": 38 * entries, "inverse_bytes": inverse,
+            "achieved": (38 * entries + inverse) / s / 1e9, "unit": "GB/s"}
 
 
 def main():
@@ -556,7 +591,9 @@ def main():
                **learned_info(mesh, args)}
         del lsolver
 
-    # roofline of the dominant kernel (tangent matvec), CUDA events on the solver stream
+    # roofline of the single tangent product, CUDA events on the solver stream, and
+    # the persistent kernel that the solves run in
+    pcg = pcg_point(args, mesh, v.conn, dev) if args.precond == "two_level" else None
     kms = (C.c_double * 4)()
     rc = _lib.load().fem_profile_kernels(mesh.ctx, 200, kms)
     mv_ms = kms[0] if rc == 0 else None
@@ -566,8 +603,8 @@ def main():
     achieved = b_mv / (mv_ms * 1e-3) / 1e9 if mv_ms else None
     st = mesh.stats()
     variant = st["matvec_variant"]
-    # a solve in the persistent PCG kernel has no separate matvec launch: the
-    # profiled one is then the element pass of fem_tangent_matvec
+    # a solve in the persistent PCG kernel has no separate matvec launch
+    # ("pcg_kernel" below): the product here is then that of fem_tangent_matvec
     profiled = "persistent" if variant == "assembled" else variant
     traffic = load_traffic().get(f"matvec_{profiled}_j2_n{args.n}")
     traffic_warm = load_traffic().get(f"matvec_{profiled}_j2_n{args.n}_warm")
@@ -595,6 +632,8 @@ def main():
             "gpu_launches": int(launches // max(args.steps, 1)),
             "kernel_ms": {"matvec": kms[0], "residual": kms[1], "cg_update": kms[2], "cg_direction": kms[3]},
             "matvec_variant": {"chosen": variant, "ns_per_launch": st["matvec_ns"]},
+            "pcg_kernel": ({**pcg, "peak": peak, "frac": pcg["achieved"] / peak,
+                            "traffic": load_traffic().get(f"pcg_iteration_j2_n{args.n}")} if pcg else None),
             "fused_step": mesh.step_info(),
             "whole_solve_graphs": {"available": st["whole_solve_graph_available"],
                                    "pcg_solves_as_one_launch": st["whole_solve_graphs"]},

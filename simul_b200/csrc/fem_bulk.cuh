@@ -55,11 +55,6 @@ __device__ __forceinline__ void load_hint(void* dst, const void* src, uint32_t b
       : "memory");
 }
 
-__device__ __forceinline__ void load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  expect(bar, bytes);
-  copy(dst, src, bytes, bar);
-}
-
 // Waits for the barrier's phase of the given parity; false if it did not
 // complete within the limit (about a second).
 __device__ __forceinline__ bool wait(uint64_t* bar, uint32_t parity) {

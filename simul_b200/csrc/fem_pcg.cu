@@ -11,20 +11,23 @@
 //
 // (r.z = r.S r + r_c.y_c, so no phase of its own forms z before beta is known.
 // A small coarse space: every CTA adds up r_c itself, no barrier after C1.)
-// (Jacobi: A and B with z = D^-1 r.)  The recurrences, the
-// FP64 sums in a fixed order and the stopping tests are those of the kernel
-// chain.
+// (Jacobi: A and B with z = D^-1 r.)  The sums are FP64 in a fixed order and
+// the stopping tests those of the kernel chain; the scalars differ from the
+// chain's in rounding (its r.z is one sum over z, and its q comes by
+// recurrence).
 //
-// What bounds it: below about 50,000 rows the matrix stays in shared memory
-// for the whole solve and the phases' latencies are left: 2,700 cycles per
-// barrier and about 2,500 of dependent loads and sums per phase, 35,000 cycles
-// (18 us) an iteration at 16,000 rows against 30 us for the chain's seven
-// kernels (42,000 with z in a phase of its own, a barrier more, and one warp
-// per slice).  At 121,000 rows the matrix (55 MB) and the packed BF16 coarse
-// inverse (60 MB) stream once per iteration, 81,000 cycles (43 us) against
-// 70 us: the rings hold 20 MB of them, the rest comes at 7 TB/s.  All 128
-// registers are in use: loads held over a barrier beyond those of A spill and
-// cost more than they hide (the first row of C2: 92,000 cycles).
+// What bounds it: up to some 65,000 rows (a coarse space of full rows) the
+// matrix stays in shared memory for the whole solve and the phases' latencies
+// are left: 2,700 cycles per barrier and about 2,500 of dependent loads and sums
+// per phase, 35,000 cycles (18 us) an iteration at 16,000 rows against 30 us
+// for the chain's seven kernels (42,000 with z in a phase of its own, a barrier
+// more, and one warp per slice).  At 121,000 rows and 4-voxel cells the planes,
+// tables and rings take all of it: the matrix (55 MB) and the packed BF16
+// coarse inverse (61 MB) stream once per iteration, 72 MB of that from HBM
+// (half of the sectors hit L2), 81,000 cycles (42 us) against 70 us, HBM 21 %
+// and L2 17 % busy.  All 128 registers are in use: loads held over a barrier
+// beyond those of A spill and cost more than they hide (the first row of C2:
+// 92,000 cycles).
 //
 // The reference factorises the assembled tangent on the host
 // (backend/fea/fem/solver/static_solver.py:399-462).
@@ -528,8 +531,8 @@ __global__ void __launch_bounds__(kPcgThreads, 1) pcg_kernel(const __grid_consta
                                               : reinterpret_cast<const unsigned char*>(a.c.Ainv32t);
   unsigned char* ring = s_dyn + a.res_bytes + (size_t)warp * ns * a.stage_bytes;
   uint64_t* bar = bars + 3 * warp;
-  // the warp's list of streamed items: offset in units of 16 bytes (of the
-  // matrix, or with the top bit of the tiles) and bytes / 16 above bit 32
+  // the warp's list of streamed items: the first step and the bytes of a piece
+  // of the matrix, or the index of a 4 KB tile part and 0
   uint2* items = s_items + (size_t)warp * a.max_items;
   int n_items = 0, n_mat = 0;
   {

@@ -8,7 +8,6 @@
 
 namespace femb200 {
 
-
 // Static words of one CTA for the two-level phases, copied to shared memory
 // once per launch: a header of kTabWords, then the lists it points at.
 enum {

@@ -9,9 +9,10 @@ hot kernel ``--reps`` times through ``fem_profile_kernels``: the tangent matvec
 CG direction update; optionally the learned network's forward pass
 (``--learned weights.npz``) and one two-level PCG solve (``--two-level``,
 4-voxel cells with the packed BF16 coarse inverse by default, run as
-fixed-size iteration graphs so a kernel profiler sees every launch).  The
-per-launch CUDA-event times are printed as one JSON line.  With ``--reps 3`` and ``-k``/``-c`` filters an ncu capture of one kernel
-ends in seconds.
+fixed-size iteration graphs so a kernel profiler sees every launch), or a
+number of iterations of it in the persistent PCG kernel (``--persistent``).  The
+per-launch CUDA-event times are printed as one JSON line.  With ``--reps 3`` and
+``-k``/``-c`` filters an ncu capture of one kernel ends in seconds.
 
     python -m simul_b200.profile_case --n 64 --variant fused --reps 3
 """
@@ -20,6 +21,7 @@ from __future__ import annotations
 import argparse
 import ctypes as C
 import json
+import time
 
 import numpy as np
 
@@ -37,6 +39,8 @@ def main(argv=None):
                     help="TET4 FP64 residual variant")
     ap.add_argument("--learned", default="", help="weights file: also run the network forward --reps times")
     ap.add_argument("--two-level", action="store_true", help="also run one two-level PCG solve (rtol 1e-6)")
+    ap.add_argument("--persistent", type=int, default=0,
+                    help="also run this many iterations of a two-level solve in the persistent PCG kernel, and half as many")
     ap.add_argument("--coarse-cell", type=int, default=4, help="two-level: lattice cell edge in voxels")
     ap.add_argument("--coarse-bf16", type=int, default=1, help="two-level: BF16 packed coarse inverse")
     args = ap.parse_args(argv)
@@ -95,6 +99,25 @@ def main(argv=None):
             raise RuntimeError(_lib.last_error(mesh.ctx))
         extra["two_level_iterations"] = it.value
         extra["coarse"] = mesh.coarse_info()
+    if args.persistent:
+        mesh.set_coarse_options(cell=args.coarse_cell, bf16=bool(args.coarse_bf16), max_nodes=6144)
+        mesh.set_whole_solve_graph(True)
+        mesh.set_matvec_variant("auto")
+        rhs = torch.randn(v.n_nodes, 3, dtype=torch.float64, device=mesh.device)
+        du = torch.zeros_like(rhs)
+        it, rel = C.c_int32(), C.c_double()
+        ms_of = {}
+        for n_it in (args.persistent, args.persistent // 2) * 4:   # the first calls build the tables
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            rc = _lib.load().fem_pcg(mesh.ctx, _lib.FEM_PRECOND_TWO_LEVEL, B._ptr(rhs), B._ptr(du), 1e-20, n_it,
+                                     C.byref(it), C.byref(rel))
+            ms_of[it.value] = min(ms_of.get(it.value, 1e9), (time.perf_counter() - t0) * 1e3)
+            if rc not in (0, _lib.FEM_NOT_CONVERGED):
+                raise RuntimeError(_lib.last_error(mesh.ctx))
+        (n1, t1), (n0, t0) = sorted(ms_of.items(), reverse=True)[:2]
+        extra["persistent"] = {"iterations": n1, "variant": mesh.stats()["matvec_variant"],
+                               "us_per_iteration": 1e3 * (t1 - t0) / (n1 - n0), "coarse": mesh.coarse_info()}
     info = mesh.info()
     print(json.dumps({"n": args.n, "element": args.element, "elements": info["n_elements"],
                       "nodes": info["n_nodes"], "variant": "two_phase" if args.element == "hex8" else args.variant,
