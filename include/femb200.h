@@ -158,11 +158,13 @@ int fem_ctx_stats(void* ctx, int64_t* out18);
 enum {
   /* -2 (default): Jacobi and two-level solves run as one persistent kernel on
    * the assembled tangent (stats variant 5) where the mesh and the memory hold
-   * its tables and no option asks for the kernel chain, everything else with
-   * variant 4 (HEX8: 1); setting it also drops an earlier request for the
-   * chain and tries again what was refused; -1: time the element variants on
-   * the first PCG solve and keep the fastest; 0: fused node-block kernel; 1: element pass writing
-   * slot vectors in node order plus a node gather; 2 (TET4): element-block
+   * its tables, no option asks for the kernel chain and at most two solves are
+   * under way on the device, everything else with variant 4 (HEX8: 1; a single
+   * product of up to 128 TET4 nodes: 0); setting it also drops an earlier
+   * request for the chain and tries again what was refused; -1: time the
+   * element variants on the first PCG solve and keep the fastest; 0: fused
+   * node-block kernel; 1: element pass writing slot vectors in node order plus
+   * a node gather; 2 (TET4): element-block
    * kernel that sums each block's slot vectors in shared memory, nodes
    * shared by blocks completed by a second kernel; 3 (TET4): the two-phase
    * pass with each warp's slot vectors added per vertex in shared memory

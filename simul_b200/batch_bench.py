@@ -126,7 +126,7 @@ def run(instances=64, n_min=32, n_max=96, load_steps=10, threads=0, seed=0, prec
     out = {"instances": []}
     wall = 0.0
     if insts:   # a rank may hold no instance when there are more ranks than instances
-        # warm-up pass (graph capture, matvec-variant timing, coarse set-up), then reset
+        # warm-up pass (graph capture, coarse set-up), then reset
         batch.solve_batch(insts, load_steps=1, precond=precond, n_threads=threads)
         reset()
         t0 = time.perf_counter()
